@@ -3,8 +3,9 @@
 // own position (its key and value are already in the pages).
 //
 // This is the plain kernel of the family: one block per (token, query head),
-// 32-bit scores, running max and sum, 32-bit accumulator, IEEE expf.  It is the
-// kernel of the float32 path and the yardstick of the faster bfloat16 kernels.
+// 32-bit scores, running max and sum, 32-bit accumulator, IEEE expf.  It serves
+// the float32 path wherever attention_f32.cu declines (a bias, a sink, other head
+// sizes) and is the yardstick of the faster bfloat16 kernels.
 // The order of every reduction depends only on the token's own position, so
 // the result is the same whatever else is in the batch and however the prompt
 // was cut.
@@ -21,6 +22,7 @@
 // the scale): `bias` adds bias[h][min(p - j, n_dist - 1)] to the score of key j, a table by
 // distance and query head; `sink` adds exp(sink[h]) to the softmax denominator, a term without a
 // key or a value.
+#include "attention_f32.h"
 #include "common.cuh"
 
 constexpr int ATT_BLOCK = 128;
@@ -141,6 +143,12 @@ static int launch_generic(
     IMP_CHECK_ARG(page_size > 0 && num_pages > 0, "imp_paged_attention_generic: bad cache geometry");
     IMP_CHECK_ARG(Hq <= 65535, "imp_paged_attention_generic: more than 65535 query heads");
     cudaStream_t s = (cudaStream_t)stream;
+    if (dtype == IMP_F32 && !bias && !sink) {
+        const int rc = imp_attention_f32((float*)out, out_stride, (const float*)q, q_stride, (const float*)k_cache, (const float*)v_cache,
+                                         block_table, bt_stride, seq_of_token, positions, n_tokens, n_seqs, Hq, Hkv, Dh, page_size,
+                                         num_pages, scale, window, status, s);
+        if (rc != IMP_ERR_UNSUPPORTED) return rc;
+    }
     dim3 grid(n_tokens, Hq);
     if (dtype == IMP_F32)
         paged_attention_generic_kernel<float><<<grid, ATT_BLOCK, 0, s>>>(

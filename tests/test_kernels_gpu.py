@@ -156,6 +156,25 @@ def test_gemm_f32(K, M, N, K_):
     out2 = K.gemm_f32(torch.empty(M, N, device=DEV), wide[:, 3:3 + K_], w)
     assert torch.equal(out2, out)
 
+# Edges of both kernels: 1 ... 32 rows stream W (in groups of 1, 2, 4, 8 or 16 rows), more go to tiles of 64 x 64; 32 rows
+# of W a CTA; blocks of 32 k, stages of 4 blocks, 4 runs of blocks; clusters of 4, 2 and 1 CTAs by the number of tiles.
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 9, 17, 32, 33, 64, 65, 200])
+@pytest.mark.parametrize("N,K_", [(1, 1), (31, 32), (33, 33), (64, 127), (96, 516), (8192, 96), (12000, 40), (200, 2085)])
+def test_gemm_f32_edges(K, M, N, K_):
+    a, w = rnd(M, K_, seed=18).to(DEV), rnd(N, K_, seed=19).to(DEV)
+    out = K.gemm_f32(torch.empty(M, N, device=DEV), a, w)
+    a64, w64 = a.double(), w.double()
+    # an element passes through at most 16 multiply-adds, the pair's sum, a run's blocks and two sums of runs, each off by
+    # half a unit in the last place of what it holds
+    steps = 16 + 1 + (-(-K_ // 128) + 1) + 2
+    bound = steps * 2.0 ** -24 * (a64.abs() @ w64.abs().T) * 1.01 + 1e-30
+    assert ((out.double() - a64 @ w64.T).abs() <= bound).all()
+    for m in (0, M - 1):
+        assert torch.equal(K.gemm_f32(torch.empty(1, N, device=DEV), a[m:m + 1], w)[0], out[m])
+    wide = torch.full((M, K_ + 9), float("nan"), device=DEV)   # rows that do not start on 16 bytes; what lies beside them is not read
+    wide[:, 3:3 + K_] = a
+    assert torch.equal(K.gemm_f32(torch.empty(M, N, device=DEV), wide[:, 3:3 + K_], w), out)
+
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 7, 8, 9, 16])
 @pytest.mark.parametrize("N,K_", [(10, 64), (257, 200), (96, 4104), (50, 100)])
@@ -547,6 +566,35 @@ def test_attention_generic(K, dtype, Hq, Hkv, Dh, page, window):
                               seq, pos, 1 / math.sqrt(Dh), window, status)
     K.check_status(status)
     close(out.view(T, Hq, Dh), attention_reference(dense, toks, window), dtype)
+
+
+# The float32 kernel: a CTA a token (few tokens) and a warp a token (many) give the same bits, at the edges of 32-key chunks and of
+# rounds of eight chunks; groups of one, two, three (an odd head left over) and five query heads; windows and chunked masks.
+@pytest.mark.parametrize("Hq,Hkv,Dh,page,window", [(16, 8, 128, 16, 0), (5, 1, 64, 3, 0), (24, 8, 128, 32, 40), (4, 4, 256, 16, -48), (10, 2, 128, 1, 33)])
+def test_attention_f32_forms(K, Hq, Hkv, Dh, page, window):
+    lengths, q_counts = [300, 33, 1, 32, 290], [300, 33, 1, 2, 120]
+    bt, num_pages, kc, vc, dense, toks, q = attention_case(lengths, q_counts, Hq, Hkv, Dh, page, torch.float32)
+    T = len(toks)
+    seq = torch.tensor([s for s, _ in toks], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([p for _, p in toks], dtype=torch.int32, device=DEV)
+    q = q.reshape(T, Hq * Dh).to(DEV).repeat(8, 1)       # 8 x 456 tokens: well past the line between the two forms
+    kc, vc, bt = kc.to(DEV), vc.to(DEV), bt.to(DEV)
+    status = K.new_status(DEV)
+    out = torch.empty(8 * T, Hq * Dh, device=DEV)
+    K.paged_attention_generic(out, q, Hq, Hkv, Dh, kc, vc, bt, seq.repeat(8), pos.repeat(8), 1 / math.sqrt(Dh), window, status)
+    few = torch.empty(16, Hq * Dh, device=DEV)
+    for a in range(0, T - 15, 16):
+        K.paged_attention_generic(few, q[a:a + 16], Hq, Hkv, Dh, kc, vc, bt, seq[a:a + 16], pos[a:a + 16], 1 / math.sqrt(Dh), window, status)
+        assert torch.equal(few, out[a:a + 16])
+    K.check_status(status)
+    for r in range(8):
+        assert torch.equal(out[r * T:(r + 1) * T], out[:T])
+    if window >= 0:
+        want = attention_reference(dense, toks, window)
+    else:                                                 # the keys of the token's own chunk of -window positions
+        want = torch.stack([P.attention(dense[s][0].double()[p // -window * -window:p + 1], dense[s][1].double()[p // -window * -window:p + 1],
+                                        dense[s][2].double()[p // -window * -window:p + 1], 0)[-1] for s, p in toks])
+    close(out[:T].view(T, Hq, Dh), want, torch.float32)
 
 
 ALL_HEAD_DIMS = list(range(16, 257, 16))
