@@ -412,6 +412,24 @@ IMP_EXPORT ImpError imp_end(ImpContext ctx, int64_t id) {
     IMP_CATCH
 }
 
+IMP_EXPORT ImpError imp_host_alloc(size_t bytes, void** out) {
+    IMP_TRY
+    need_arg(out != nullptr && bytes > 0, "imp_host_alloc: out must not be null and bytes must be positive");
+    *out = nullptr;
+    const cudaError_t e = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
+    if (e != cudaSuccess) {
+        *out = nullptr;
+        (void)cudaGetLastError();
+        fail(e == cudaErrorMemoryAllocation ? IMP_ERROR_OUT_OF_MEMORY : IMP_ERROR_CUDA,
+             std::string("cannot allocate pinned host memory: ") + cudaGetErrorString(e));
+    }
+    IMP_CATCH
+}
+
+IMP_EXPORT void imp_host_free(void* p) {
+    if (p && cudaFreeHost(p) != cudaSuccess) (void)cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------- parts and architectures
 IMP_EXPORT ImpError imp_register_part(const char* category, const char* kind, const ImpPartVTable* vtable) {
     IMP_TRY

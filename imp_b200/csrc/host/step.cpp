@@ -330,9 +330,9 @@ Tensor Stepper::forward_decode_graph(Step& st) {
 }
 
 void Stepper::check_device_status(const std::string& what) {
-    int32_t code = 0;
-    IMP_CUDA(cudaMemcpyAsync(&code, rt_->status, 4, cudaMemcpyDeviceToHost, rt_->stream));
+    IMP_CUDA(cudaMemcpyAsync(status_host_.data(), rt_->status, 4, cudaMemcpyDeviceToHost, rt_->stream));
     IMP_CUDA(cudaStreamSynchronize(rt_->stream));
+    const int32_t code = *(const int32_t*)status_host_.data();
     if (code != 0) {
         IMP_CUDA(cudaMemsetAsync(rt_->status, 0, 4, rt_->stream));
         fail(IMP_ERROR_CUDA, what + ": device reported '" + imp_status_string(code) + "' (code " + std::to_string(code) + ")");

@@ -102,6 +102,7 @@ private:
     std::map<int, Graph> graphs_;
     std::map<int, int> graph_uses_;
     uint64_t arena_generation_ = 0;
+    PinnedBuffer status_host_{4};
 };
 
 }  // namespace imp

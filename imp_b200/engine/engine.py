@@ -22,6 +22,7 @@ from typing import Any, Dict, Hashable, List, Optional, Sequence
 from .. import capi
 from ..config.engine_config import EngineConfig
 from ..config.model_config import ModelConfig
+from .host_pool import HostPool
 
 
 class RequestStatus(enum.Enum):
@@ -218,6 +219,7 @@ class Engine:
         capi.check(capi.load().imp_context_create(model._h, ctypes.byref(c), ctypes.byref(ctx)))
         self._ctx = ctx
         self.vocab_size = model.vocab_size
+        self._host_pool = HostPool()            # step_tokens: where logits land
         self._outs = (capi.ImpStepOutput * max(self.config.max_batch_size * 2, 8))()
 
     # ------------------------------------------------------------ construction
@@ -234,6 +236,7 @@ class Engine:
         ctx, self._ctx = getattr(self, "_ctx", None), None
         if ctx:
             capi.load().imp_context_free(ctx)
+            self._host_pool.close()
 
     def __del__(self):
         try:
@@ -351,8 +354,8 @@ class Engine:
 
     def step_tokens(self, entries: Sequence[StepEntry]):
         """Run given tokens as one batch (no scheduling, no sampling).  Returns the logits of the wanted rows
-        as a float32 numpy array [wanted, vocab], in the order of the entries and of each `want`."""
-        import numpy as np
+        as a float32 numpy array [wanted, vocab], in the order of the entries and of each `want` (in page-locked memory
+        that serves a later call once nothing refers to the array any more)."""
         n = len(entries)
         arr = (capi.ImpStepEntry * max(n, 1))()
         keep = []
@@ -367,7 +370,7 @@ class Engine:
             arr[i].want = want
             arr[i].n_want = nw
             wanted += nw
-        out = np.empty((wanted, self.vocab_size), dtype=np.float32)
+        out = self._host_pool.array((wanted, self.vocab_size))
         capi.check(capi.load().imp_step_tokens(self._ctx, arr, n, out.ctypes.data_as(ctypes.c_void_p), out.size))
         return out
 

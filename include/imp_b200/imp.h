@@ -227,6 +227,11 @@ IMP_EXPORT ImpError imp_step_tokens(ImpContext ctx, const ImpStepEntry* entries,
                                     size_t capacity);
 IMP_EXPORT ImpError imp_end(ImpContext ctx, int64_t id);
 
+/* Page-locked host memory for `logits_out`: the device writes it directly at the bus's rate, ordinary memory is filled by
+ * the driver piece by piece.  Allocating costs about as much as one such fill: keep and reuse it.  Any thread; null may be freed. */
+IMP_EXPORT ImpError imp_host_alloc(size_t bytes, void** out);
+IMP_EXPORT void imp_host_free(void* p);
+
 #ifdef __cplusplus
 }
 #endif
