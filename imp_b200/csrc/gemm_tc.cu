@@ -20,6 +20,8 @@
 //
 // Reference counterpart: gemm() -> cublasLtMatmul with fp16 inputs and fp32 accumulation
 // (src/compute/gemm.cu:303-445); the reference has no tensor-memory kernel of its own.
+#include <algorithm>
+
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -611,12 +613,25 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
                  ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 
-template <int EPI>
+// A list of rows sorted by group, each group with a weight matrix of its own (routed experts): seg[g] ... seg[g + 1] are
+// group g's rows of A and C, and its matrix is rows g N ... (g + 1) N - 1 of W.  `seg` is device memory: a launch does not
+// depend on the routing.
+struct TcGroups {
+    const int* seg;
+    int count;
+};
+constexpr int TC2_MAX_GROUPS = 256;
+constexpr int TC2_GROUP_BYTES = (TC2_MAX_GROUPS + 1) * 4;
+static_assert(TC2_SMEM_BYTES + TC2_GROUP_BYTES <= 227 * 1024, "the pair kernel's shared memory with a table of groups");
+
+// GROUPED: the units are the groups' tiles, group after group (a group's row tiles fastest, then the columns: the tiles
+// that run together share a group's rows and weights in the L2), M is the most rows the list can have and splits is 1.
+template <int EPI, bool GROUPED = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
     gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                         void* __restrict__ Cv, int64_t ldc, int M, int N, int K, int* status,
                         const __grid_constant__ QkvRopeArgs qkv, int splits, int kb_per_split, int64_t split_stride,
-                        const __grid_constant__ CUtensorMap map_c, int tma_store, GateAct gate_act) {
+                        const __grid_constant__ CUtensorMap map_c, int tma_store, GateAct gate_act, TcGroups groups) {
     // tma_store (bfloat16 and SwiGLU epilogues): C goes out through shared memory and TMA stores described by map_c
     // (boxes of 128 rows x 64 columns, clipped at the matrix edges) instead of 16-byte stores from every thread.
     // splits > 1 (32-bit output only): the K range is cut into `splits` parts, each (tile, part) is a unit of work of its
@@ -634,7 +649,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
     const int k_blocks = (K + TC_BK - 1) / TC_BK;
     const int num_m = (M + TC2_BM - 1) / TC2_BM, num_n = (N + TC2_BN - 1) / TC2_BN;
     const int n_tiles = num_m * num_n;
-    const int total = n_tiles * splits;            // units: all tiles of part 0, then all of part 1, ...
+    int total = n_tiles * splits;                  // units: all tiles of part 0, then all of part 1, ...
+    int* first_unit = reinterpret_cast<int*>(tmem_slot + 1);   // GROUPED: of every group, and the number of units
+    // Where unit u lies: first row and column, part of K, first row of the group's weights, end of the rows.
+    struct Unit { int m0, n0, z, w0, rows; };
+    auto locate = [&](int u) -> Unit {
+        if constexpr (GROUPED) {
+            int g = 0;
+            for (int step = TC2_MAX_GROUPS / 2; step > 0; step >>= 1)
+                if (g + step < groups.count && first_unit[g + step] <= u) g += step;
+            const int a = groups.seg[g], b = groups.seg[g + 1], mt = (b - a + TC2_BM - 1) / TC2_BM, local = u - first_unit[g];
+            return Unit{a + local % mt * TC2_BM, local / mt * TC2_BN, 0, g * N, b};
+        } else {
+            const int t = u % n_tiles;
+            return Unit{(t % num_m) * TC2_BM, (t / num_m) * TC2_BN, u / n_tiles, 0, M};
+        }
+    };
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + TC2_STAGES);
     const uint32_t accf0 = smem_u32(bars + 2 * TC2_STAGES), acce0 = smem_u32(bars + 2 * TC2_STAGES + 2);
 
@@ -664,6 +694,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
     pdl_wait();
     IMP_TL_WAITED()
     pdl_launch_dependents();
+    if constexpr (GROUPED) {
+        if (warp == 0) {
+            int before = 0;
+            for (int g0 = 0; g0 < groups.count; g0 += 32) {
+                const int g = g0 + lane;
+                const int mine = g < groups.count ? (groups.seg[g + 1] - groups.seg[g] + TC2_BM - 1) / TC2_BM * num_n : 0;
+                int upto = mine;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                    if (lane >= o) upto += below;
+                }
+                if (g < groups.count) first_unit[g] = before + upto - mine;
+                before += __shfl_sync(0xffffffffu, upto, 31);
+            }
+            if (lane == 0) first_unit[groups.count] = before;
+        }
+        __syncthreads();
+        total = first_unit[groups.count];
+    }
 
     if (warp == 0) {
         if (lane == 0) {
@@ -671,9 +721,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             uint32_t it = 0;
             bool ok = true;
             for (int u = pair; u < total && ok; u += n_pairs) {
-                const int t = u % n_tiles, z = u / n_tiles;
-                const int kb_lo = z * kb_per_split, kb_hi = min(k_blocks, kb_lo + kb_per_split);
-                const int m0 = (t % num_m) * TC2_BM + (int)rank * 128, n0 = (t / num_m) * TC2_BN + (int)rank * 128;
+                const Unit at = locate(u);
+                const int kb_lo = at.z * kb_per_split, kb_hi = min(k_blocks, kb_lo + kb_per_split);
+                const int m0 = at.m0 + (int)rank * 128, n0 = at.w0 + at.n0 + (int)rank * 128;
                 for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
                     const uint32_t s = it % TC2_STAGES;
                     ok = mbar_wait(empty0 + 8 * s, ((it / TC2_STAGES) & 1u) ^ 1u, status);
@@ -697,7 +747,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             uint32_t it = 0, local = 0;
             bool ok = true;
             for (int u = pair; u < total && ok; u += n_pairs, ++local) {
-                const int z = u / n_tiles;
+                const int z = GROUPED ? 0 : u / n_tiles;
                 const int kb_lo = z * kb_per_split, kb_hi = min(k_blocks, kb_lo + kb_per_split);
                 const uint32_t buf = local & 1u;
                 ok = mbar_wait(acce0 + 8 * buf, ((local >> 1) & 1u) ^ 1u, status);   // both epilogues have drained it
@@ -727,7 +777,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
         uint32_t out_n = 0;                              // staging buffers used so far
         uint32_t local = 0;
         for (int u = pair; u < total; u += n_pairs, ++local) {
-            const int t = u % n_tiles, z = u / n_tiles;
+            const Unit at = locate(u);
             const uint32_t buf = local & 1u;
             bool ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * buf, (local >> 1) & 1u, status));
             if (EPI != TC_OUT_F32 && tma_store) {
@@ -747,17 +797,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             }
             if (!ok) break;
             tc_fence_after_sync();
-            const int m0 = (t % num_m) * TC2_BM + (int)rank * 128, n0 = (t / num_m) * TC2_BN;
-            void* Cz = EPI == TC_OUT_F32 ? (void*)(reinterpret_cast<float*>(Cv) + (int64_t)z * split_stride) : Cv;
+            const int m0 = at.m0 + (int)rank * 128, n0 = at.n0, rows = at.rows;
+            void* Cz = EPI == TC_OUT_F32 ? (void*)(reinterpret_cast<float*>(Cv) + (int64_t)at.z * split_stride) : Cv;
             const int row = m0 + quarter * 32 + lane;
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * TC2_BN;
             // TMA stores only for a CTA's 128 rows that all lie inside C (and whole 64-column pieces): a store that the
             // tensor map clips measured far slower than the threads' own stores (2048 x 24576 outputs cut at 320 rows:
             // 97 us against 78), so the last, partly filled row block of a matrix takes the plain path.
-            const bool whole = m0 + 128 <= M && n0 + TC2_BN <= N;
+            const bool whole = m0 + 128 <= rows && n0 + TC2_BN <= N;
             if (EPI == TC_OUT_QKV_ROPE) {
-                const QkvStage stg{tma_store && m0 + 128 <= M ? out_stage : nullptr, &map_c, storer, quarter * 32 + lane, m0};
-                qkv_rope_row(qkv, taddr, row, n0, N, row < M, status, stg);
+                const QkvStage stg{tma_store && m0 + 128 <= rows ? out_stage : nullptr, &map_c, storer, quarter * 32 + lane, m0};
+                qkv_rope_row(qkv, taddr, row, n0, N, row < rows, status, stg);
             } else if ((EPI == TC_OUT_BF16 || EPI == TC_OUT_SWIGLU_BF16) && tma_store && whole) {
                 constexpr int SUBS = EPI == TC_OUT_SWIGLU_BF16 ? 2 : 4;     // sub-tiles of 64 output columns
                 const int x0 = EPI == TC_OUT_SWIGLU_BF16 ? n0 >> 1 : n0;
@@ -812,7 +862,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                     float v[32];
                     tc_ld32(taddr + (uint32_t)(c * 32), v);
                     plain_act<EPI>(v, gate_act, n0 + c * 32, N);
-                    tc_store32<EPI == TC_OUT_QKV_ROPE ? TC_OUT_BF16 : EPI>(Cz, ldc, row, n0 + c * 32, M, N, v, gate_act);
+                    tc_store32<EPI == TC_OUT_QKV_ROPE ? TC_OUT_BF16 : EPI>(Cz, ldc, row, n0 + c * 32, rows, N, v, gate_act);
                 }
             }
             tc_fence_before_sync();
@@ -876,12 +926,13 @@ template <int BN, int WROWS> constexpr int tcs_rows_stages() {
 template <int BN, int WROWS> constexpr int tcs_rows_smem_bytes() { return tcs_rows_stages<BN, WROWS>() * tcs_rows_stage_bytes<BN, WROWS>() + 1024 + 256; }
 
 // EPI: 0 = bfloat16 C[M,N], 1 = float32 C[M,N] (also the split partials), 2 = SwiGLU bfloat16 C[M,N/2]
-template <int BN, int EPI, int WROWS = 128>
+// GROUPED (splits 1): blockIdx.y is a tile of up to BN rows of one group's part of the list; a CTA beyond the last tile leaves.
+template <int BN, int EPI, int WROWS = 128, bool GROUPED = false>
 __global__ void __launch_bounds__(128, 1) gemm_tc_swap_kernel(const __grid_constant__ CUtensorMap map_w,
                                                               const __grid_constant__ CUtensorMap map_x, void* __restrict__ Cv,
                                                               int64_t ldc, int64_t split_stride, int M, int N, int K,
                                                               int kb_per_split, int tile_rows, int* status,
-                                                              uint32_t wait_limit, int skip_kb, GateAct gate_act) {
+                                                              uint32_t wait_limit, int skip_kb, GateAct gate_act, TcGroups groups) {
     constexpr int TCS_STAGES = tcs_rows_stages<BN, WROWS>();
     static_assert(tcs_rows_stage_bytes<BN, WROWS>() >= TCS_W_BYTES && tcs_rows_stage_bytes<BN, WROWS>() % 1024 == 0, "a stage spans what the MMA reads");
     IMP_TL_BEGIN(10 + EPI)
@@ -895,6 +946,34 @@ __global__ void __launch_bounds__(128, 1) gemm_tc_swap_kernel(const __grid_const
     // A CTA owns tile_rows (<= 128, a multiple of 16) weight rows: map_w's box has that many rows, the MMA still
     // spans 128 and works on whatever the stage holds beyond them; those accumulator lanes are never stored.
     const int n0 = blockIdx.x * tile_rows;
+    int w0 = n0, row0 = 0;                          // the tile's first rows in W and in the list
+    if constexpr (GROUPED) {
+        pdl_wait();
+        int tile = blockIdx.y, g = -1, end = 0;
+        for (int base = 0; base < groups.count && g < 0; base += 32) {   // every warp for itself, 32 groups at a time
+            const int e = base + lane, a = e < groups.count ? groups.seg[e] : 0, b = e < groups.count ? groups.seg[e + 1] : 0;
+            const int mine = (b - a + BN - 1) / BN;
+            int upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += below;
+            }
+            const uint32_t past = __ballot_sync(0xffffffffu, tile < upto);
+            if (past) {
+                const int l = __ffs(past) - 1;
+                g = base + l;
+                row0 = __shfl_sync(0xffffffffu, a + (tile - (upto - mine)) * BN, l);
+                end = __shfl_sync(0xffffffffu, b, l);
+            } else {
+                tile -= __shfl_sync(0xffffffffu, upto, 31);
+            }
+        }
+        if (g < 0) return;
+        w0 = g * N + n0;
+        M = min(BN, end - row0);
+        Cv = reinterpret_cast<__nv_bfloat16*>(Cv) + (int64_t)row0 * ldc;   // 16-bit outputs only
+    }
     const uint32_t stage_tx = (uint32_t)(tile_rows + BN) * (TC_BK * 2);   // bytes the two boxes of a stage bring
     const int total_kb = (K + TC_BK - 1) / TC_BK;
     const int kb_lo = blockIdx.z * kb_per_split;
@@ -930,12 +1009,12 @@ __global__ void __launch_bounds__(128, 1) gemm_tc_swap_kernel(const __grid_const
         const int early = k_blocks < TCS_STAGES ? k_blocks : TCS_STAGES;
         for (int i = 0; i < early; ++i) {
             mbar_expect_tx(full0 + 8 * i, stage_tx);
-            tma_load_2d(smem_u32(tiles + i * STAGE), &map_w, (kb_lo + i) * TC_BK, n0, full0 + 8 * i);
+            tma_load_2d(smem_u32(tiles + i * STAGE), &map_w, (kb_lo + i) * TC_BK, w0, full0 + 8 * i);
         }
         pdl_wait();
         IMP_TL_WAITED()
         for (int i = 0; i < early; ++i)
-            tma_load_2d(smem_u32(tiles + i * STAGE) + W_BYTES, &map_x, (kb_lo + i) * TC_BK, 0, full0 + 8 * i);
+            tma_load_2d(smem_u32(tiles + i * STAGE) + W_BYTES, &map_x, (kb_lo + i) * TC_BK, row0, full0 + 8 * i);
         issued = early;
         for (int i = early; i < k_blocks; ++i) {
             const int s = i % TCS_STAGES;
@@ -944,8 +1023,8 @@ __global__ void __launch_bounds__(128, 1) gemm_tc_swap_kernel(const __grid_const
             if (i == skip_kb) { issued = i + 1; continue; }
             const uint32_t w_dst = smem_u32(tiles + s * STAGE), x_dst = w_dst + W_BYTES;
             mbar_expect_tx(full0 + 8 * s, stage_tx);
-            tma_load_2d(w_dst, &map_w, (kb_lo + i) * TC_BK, n0, full0 + 8 * s);
-            tma_load_2d(x_dst, &map_x, (kb_lo + i) * TC_BK, 0, full0 + 8 * s);
+            tma_load_2d(w_dst, &map_w, (kb_lo + i) * TC_BK, w0, full0 + 8 * s);
+            tma_load_2d(x_dst, &map_x, (kb_lo + i) * TC_BK, row0, full0 + 8 * s);
             issued = i + 1;
         }
         if (!ok)
@@ -1150,7 +1229,7 @@ static int launch_tc(void* C, int64_t ldc, const CUtensorMap& ma, const CUtensor
         if (EPI != TC_OUT_F32 && tma_out && ldc % 8 == 0)
             tma_store = make_map(&mc, C, M, EPI == TC_OUT_SWIGLU_BF16 ? N / 2 : N, ldc, 128) == 0 ? 1 : 0;
         cudaError_t e = imp_launch(gemm_tc_pair_kernel<EPI>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)TC2_SMEM_BYTES, s, ma, mw128,
-                                   C, ldc, M, N, K, status, QkvRopeArgs{}, 1, (K + TC_BK - 1) / TC_BK, (int64_t)0, mc, tma_store, gate_act);
+                                   C, ldc, M, N, K, status, QkvRopeArgs{}, 1, (K + TC_BK - 1) / TC_BK, (int64_t)0, mc, tma_store, gate_act, TcGroups{});
         if (e != cudaSuccess) { imp_set_error("gemm_tc: %s", cudaGetErrorString(e)); return (int)e; }
         return 0;
     }
@@ -1259,7 +1338,7 @@ IMP_API int imp_gemm_bf16_tc_partials(float* scratch, const void* A, int64_t lda
     const int pairs = units < sms / 2 ? units : sms / 2;
     cudaError_t e = imp_launch(gemm_tc_pair_kernel<TC_OUT_F32>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)TC2_SMEM_BYTES,
                                (cudaStream_t)stream, ma, mw128, (void*)scratch, (int64_t)N, M, N, K, status, QkvRopeArgs{}, splits,
-                               kb_per_split, (int64_t)M * N, CUtensorMap{}, 0, 0);
+                               kb_per_split, (int64_t)M * N, CUtensorMap{}, 0, 0, TcGroups{});
     if (e != cudaSuccess) { imp_set_error("imp_gemm_bf16_tc_partials: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;
 }
@@ -1324,7 +1403,7 @@ static int launch_tcs(void* C, int64_t ldc, int64_t split_stride, const CUtensor
     }
     dim3 grid((N + tile_rows - 1) / tile_rows, 1, splits);
     cudaError_t e = imp_launch(gemm_tc_swap_kernel<BN, EPI, WROWS>, grid, dim3(128), (size_t)tcs_rows_smem_bytes<BN, WROWS>(), s, mw, mx,
-                               C, ldc, split_stride, M, N, K, kb_per_split, tile_rows, status, g_tcs_wait_limit, g_tcs_skip_kb, gate_act);
+                               C, ldc, split_stride, M, N, K, kb_per_split, tile_rows, status, g_tcs_wait_limit, g_tcs_skip_kb, gate_act, TcGroups{});
     if (e != cudaSuccess) { imp_set_error("gemm_tc_swap: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;
 }
@@ -1465,6 +1544,73 @@ IMP_API int imp_gemm_bf16_tc_swap_sum(void* C, int64_t ldc, int epilogue, const 
     return 0;
 }
 
+// ---- rows in groups ---------------------------------------------------------------------------------
+// C[r, :] = A[r, :] W_g^T (or its gated or squared-relu form) for a list of at most M rows sorted by group: row r belongs to
+// the group g with seg[g] <= r < seg[g + 1] (device memory, G + 1 values), W_g is rows g N ... (g + 1) N - 1 of W [G N, K].
+// `epilogue` as for imp_gemm_bf16_tc_act, 16-bit outputs only.  IMP_ERR_UNSUPPORTED, with nothing launched, where the tensor
+// copies cannot take the operands or there are more than TC2_MAX_GROUPS groups.
+//
+// Few rows a group: the weights are what has to be read, and the few-rows kernel streams them with a tile of up to 32, 64 or
+// 128 of the list's rows beside them.  Many: CTA pairs walk 256 x 256 tiles of all groups in one launch.
+template <int EPI>
+static int launch_grouped_pair(void* C, int64_t ldc, const void* A, int64_t lda, const void* W, int M, int N, int K, TcGroups groups, int* status,
+                               cudaStream_t s, GateAct act) {
+    constexpr int smem = TC2_SMEM_BYTES + TC2_GROUP_BYTES;
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) { imp_set_error("gemm_tc_grouped: %s", cudaGetErrorString(e)); return (int)e; }
+    CUtensorMap ma, mw, mc{};
+    if (int rc = make_map(&ma, A, M, K, lda, TC_BM)) return rc;
+    if (int rc = make_map(&mw, W, N * groups.count, K, K, 128)) return rc;
+    const int tma_store = ldc % 8 == 0 && make_map(&mc, C, M, EPI == TC_OUT_SWIGLU_BF16 ? N / 2 : N, ldc, 128) == 0 ? 1 : 0;
+    const int64_t units = ((int64_t)M / TC2_BM + groups.count) * ((N + TC2_BN - 1) / TC2_BN);   // at most
+    const int pairs = (int)std::min<int64_t>(units, std::max(imp_sm_count() / 2, 1));
+    e = imp_launch(gemm_tc_pair_kernel<EPI, true>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)smem, s, ma, mw, C, ldc, M, N, K, status,
+                   QkvRopeArgs{}, 1, (K + TC_BK - 1) / TC_BK, (int64_t)0, mc, tma_store, act, groups);
+    if (e != cudaSuccess) { imp_set_error("gemm_tc_grouped: %s", cudaGetErrorString(e)); return (int)e; }
+    return 0;
+}
+
+template <int BN, int EPI>
+static int launch_grouped_swap(void* C, int64_t ldc, const void* A, int64_t lda, const void* W, int M, int N, int K, TcGroups groups, int* status,
+                               cudaStream_t s, GateAct act) {
+    constexpr int smem = tcs_rows_smem_bytes<BN, 128>();
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_swap_kernel<BN, EPI, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) { imp_set_error("gemm_tc_grouped: %s", cudaGetErrorString(e)); return (int)e; }
+    CUtensorMap mw, mx;
+    if (int rc = make_map(&mw, W, N * groups.count, K, K, 128)) return rc;
+    if (int rc = make_map(&mx, A, M, K, lda, BN)) return rc;
+    const int64_t tiles = std::min<int64_t>(M / BN + groups.count, M);   // at most: a full tile takes BN rows, a last one any
+    if (tiles > 65535) return IMP_ERR_UNSUPPORTED;
+    e = imp_launch(gemm_tc_swap_kernel<BN, EPI, 128, true>, dim3((N + 127) / 128, (unsigned)tiles), dim3(128), (size_t)smem, s, mw, mx, C, ldc,
+                   (int64_t)0, M, N, K, (K + TC_BK - 1) / TC_BK, 128, status, g_tcs_wait_limit, -1, act, groups);
+    if (e != cudaSuccess) { imp_set_error("gemm_tc_grouped: %s", cudaGetErrorString(e)); return (int)e; }
+    return 0;
+}
+
+// Average rows a group from which CTA pairs take a list (its last tiles of 256 rows are half empty on average).
+constexpr int TCG_PAIR_ROWS = 96;
+
+IMP_API int imp_gemm_bf16_tc_grouped(void* C, int64_t ldc, int epilogue, float limit, const void* A, int64_t lda, const void* W, const int* seg, int M,
+                                     int N, int K, int G, int* status, void* stream) {
+    if (M == 0 || N == 0 || G == 0) return 0;
+    IMP_CHECK_ARG(C && A && W && seg && M > 0 && N > 0 && K > 0 && G > 0, "imp_gemm_bf16_tc_grouped: bad argument");
+    const GateAct act = split_epilogue(&epilogue, limit);
+    IMP_CHECK_ARG(epilogue == TC_OUT_BF16 || epilogue == TC_OUT_SWIGLU_BF16, "imp_gemm_bf16_tc_grouped: unknown epilogue %d", epilogue);
+    const bool gated = epilogue == TC_OUT_SWIGLU_BF16;
+    if (gated) IMP_CHECK_ARG(N % 16 == 0, "imp_gemm_bf16_tc_grouped: %d interleaved rows are not a multiple of 16", N);
+    IMP_CHECK_ARG(lda >= K && ldc >= (gated ? N / 2 : N), "imp_gemm_bf16_tc_grouped: leading dimension too small");
+    if (K % 8 || lda % 8 || (uintptr_t)A % 16 || (uintptr_t)W % 16 || (uintptr_t)C % 16 || G > TC2_MAX_GROUPS || (int64_t)N * G > 0x7fffffff)
+        return IMP_ERR_UNSUPPORTED;
+    const TcGroups groups{seg, G};
+    cudaStream_t s = (cudaStream_t)stream;
+    const int avg = M / G;
+    auto run = [&](auto plain, auto glu) { return (gated ? glu : plain)(C, ldc, A, lda, W, M, N, K, groups, status, s, act); };
+    if (avg >= TCG_PAIR_ROWS) return run(launch_grouped_pair<TC_OUT_BF16>, launch_grouped_pair<TC_OUT_SWIGLU_BF16>);
+    if (avg > 48) return run(launch_grouped_swap<128, TC_OUT_BF16>, launch_grouped_swap<128, TC_OUT_SWIGLU_BF16>);
+    if (avg > 24) return run(launch_grouped_swap<64, TC_OUT_BF16>, launch_grouped_swap<64, TC_OUT_SWIGLU_BF16>);
+    return run(launch_grouped_swap<32, TC_OUT_BF16>, launch_grouped_swap<32, TC_OUT_SWIGLU_BF16>);
+}
+
 // q, k, v = A W^T with the per-head norm, the rotation and the cache write done in the product's epilogue
 // (see QkvRopeArgs): A [M, K], W [(Hq + 2 Hkv) * Dh, K] with q heads first, then k, then v.  Needs at least
 // 256 rows, head size 64 or 128 rotated over its whole width, CTA pairs enabled; returns IMP_ERR_UNSUPPORTED
@@ -1520,7 +1666,7 @@ IMP_API int imp_gemm_bf16_tc_qkv_rope(const void* A, int64_t lda, const void* W,
     }
     cudaError_t e = imp_launch(gemm_tc_pair_kernel<TC_OUT_QKV_ROPE>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)TC2_SMEM_BYTES,
                                (cudaStream_t)stream, ma, mw128, (void*)nullptr, (int64_t)0, M, N, K, status, a, 1,
-                               (K + TC_BK - 1) / TC_BK, (int64_t)0, mq, q_tma, 0);
+                               (K + TC_BK - 1) / TC_BK, (int64_t)0, mq, q_tma, 0, TcGroups{});
     if (e != cudaSuccess) { imp_set_error("imp_gemm_bf16_tc_qkv_rope: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;
 }

@@ -88,6 +88,8 @@ int imp_gemm_bf16_tc(void* C, int64_t ldc, int epilogue, const void* A, int64_t 
                      int N, int K, int* status, void* stream);
 int imp_gemm_bf16_tc_act(void* C, int64_t ldc, int epilogue, float limit, const float* bias, const void* A, int64_t lda, const void* W,
                          int64_t ldw, int M, int N, int K, int* status, void* stream);
+int imp_gemm_bf16_tc_grouped(void* C, int64_t ldc, int epilogue, float limit, const void* A, int64_t lda, const void* W, const int* seg, int M, int N,
+                             int K, int G, int* status, void* stream);
 int imp_gemm_bf16_tc_swap_act(void* C, int64_t ldc, int epilogue, float limit, const float* bias, const void* A, int64_t lda, const void* W,
                               int64_t ldw, int M, int N, int K, float* scratch, int* status, void* stream);
 int64_t imp_gemm_bf16_tc_swap_scratch_floats(int M, int N, int K, int epilogue);
@@ -227,13 +229,14 @@ int imp_moe_choose(const float* z, int64_t ldz, int n_splits, int64_t part_strid
                    int* idx, float* wts, float* gate, int score_mode, int n_groups, int keep, int group_top, float weight_scale,
                    const float* choice_bias, int renormalise, int* seg, int* row_token, int* pair_row, void* stream);
 int imp_moe_sort(const int* idx, int n_tokens, int top, int E, int* seg, int* row_token, int* pair_row, void* stream);
-int imp_gather_rows(void* dst, const void* src, int64_t ld, const int* idx, int n_rows, int d, int dtype, void* stream);
+int imp_gather_rows(void* dst, const void* src, int64_t ld, const int* idx, const int* n, int max_rows, int d, int dtype, void* stream);
 int imp_moe_combine(void* out, const void* y, const int* pair_row, const float* wts, int n_tokens, int top, const void* shared,
                     const float* gate, const void* input, int64_t input_ld, int d, int act_dtype, void* stream);
 }
 
 // Epilogues of the products over groups (imp_grouped_gemm_ex).
 enum { GROUPED_PLAIN = 0, GROUPED_RELU2 = 2, GROUPED_SIGMOID_GATE = 3 };
+constexpr int IMP_TC_GROUPS_MAX = 256;   // groups that imp_gemm_bf16_tc_grouped takes
 // Epilogues of the tcgen05 products.
 enum { TC_OUT_BF16 = 0, TC_OUT_F32 = 1, TC_OUT_SWIGLU = 2, TC_OUT_GEGLU = 4, TC_OUT_CLIPGLU = 5, TC_OUT_RELU2 = 6 };
 // 2 / 4: act(gate) * up, act silu / gelu (tanh form); 5: gate and up clipped to a limit; 6: max(., 0)^2, no gate

@@ -656,38 +656,26 @@ struct RoutedExperts : FeedForward {
         }
         Tensor hid = rt.empty(P, F);
         Tensor y = rt.empty(P, d);
-        // Portions of prompts with much work an expert (rows x F x d of 2^31 and more on average): the list's offsets come to
-        // the host, and every expert's rows go to the tensor-memory products as a dense matrix (the wait costs one round
-        // trip a layer; 2,048 tokens on 16 experts of 4096 x 4096: 1.2 against 2.0 ms a layer; with experts of 1024 x 1024
-        // the products' fixed cost loses: 5.9 against 4.0 ms for four layers).  All other steps, and every step that may
-        // be captured into a graph, run the two products over groups, whose launches do not depend on the routing.
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        IMP_CUDA(cudaStreamIsCapturing(rt.stream, &capturing));
-        static const double dense_work = [] { const std::string e = env_string("IMP_B200_MOE_DENSE_WORK", ""); return e.empty() ? 2147483648.0 : std::atof(e.c_str()); }();
-        const bool tensor_cores = interleaved || (!gated_expert && w_up.dtype == BF16 && w_down.dtype == BF16 && F % 8 == 0 && d % 8 == 0);
-        if (tensor_cores && !st.decode_only() && capturing == cudaStreamCaptureStatusNone && dense_work > 0 &&
-            (double)P / (double)R * (double)F * (double)d >= dense_work) {
-            std::vector<int> hseg((size_t)E + 1);
-            IMP_CUDA(cudaMemcpyAsync(hseg.data(), seg, hseg.size() * 4, cudaMemcpyDeviceToHost, rt.stream));
-            IMP_CUDA(cudaStreamSynchronize(rt.stream));
-            const int64_t listed = hseg[(size_t)E];   // choices that fell on identity experts are not in the list
+        // The tensor-memory products over groups; like those over lists they do not depend on the routing on the host, so a
+        // step may be captured.  (They want the rows side by side; where they take the first product they take the second.)
+        const bool tensor_cores = interleaved || (!gated_expert && w_up.dtype == BF16 && w_down.dtype == BF16);
+        bool done = false;
+        if (tensor_cores && F % 8 == 0 && d % 8 == 0 && E <= IMP_TC_GROUPS_MAX) {
             Tensor xs = rt.empty(P, d);
-            check_launch(imp_gather_rows(xs.data, x.data, x.stride0, row_token, (int)listed, (int)d, dt, rt.stream), "gather_rows");
-            const size_t el = elem_size(rt.dtype);
-            for (int64_t e = 0; e < E; ++e) {
-                const int64_t a0 = hseg[(size_t)e], n = hseg[(size_t)e + 1] - a0;
-                if (n <= 0) continue;
-                Tensor xe = tensor2d((char*)xs.data + (size_t)(a0 * d) * el, rt.dtype, n, d);
-                Tensor ae = tensor2d((char*)hid.data + (size_t)(a0 * F) * el, rt.dtype, n, F);
-                Tensor ye = tensor2d((char*)y.data + (size_t)(a0 * d) * el, rt.dtype, n, d);
-                Tensor wd = tensor2d((char*)w_down.data + (size_t)(e * d * F) * el, w_down.dtype, d, F);
-                if (gated_expert)
-                    linear_gated(rt, ae, xe, tensor2d((char*)w_gate.data + (size_t)(e * 2 * F * d) * el, w_gate.dtype, 2 * F, d), act);
-                else
-                    linear_relu2(rt, ae, xe, tensor2d((char*)w_up.data + (size_t)(e * F * d) * el, w_up.dtype, F, d));
-                linear(rt, ye, ae, wd);
+            ++rt.launches;
+            check_launch(imp_gather_rows(xs.data, x.data, x.stride0, row_token, seg + E, (int)P, (int)d, dt, rt.stream), "gather_rows");
+            const int up_epi = !gated_expert ? TC_OUT_RELU2 : act.kind == 0 ? TC_OUT_SWIGLU : act.kind == 1 ? TC_OUT_GEGLU : TC_OUT_CLIPGLU;
+            const int rc = imp_gemm_bf16_tc_grouped(hid.data, F, up_epi, act.limit, xs.data, d, gated_expert ? w_gate.data : w_up.data, seg, (int)P,
+                                                    (int)(gated_expert ? 2 * F : F), (int)d, (int)E, rt.status, rt.stream);
+            if (rc != -2) {
+                check_launch(rc, "gemm_tc_grouped (experts, up)");
+                check_launch(imp_gemm_bf16_tc_grouped(y.data, d, TC_OUT_BF16, 0.f, hid.data, F, w_down.data, seg, (int)P, (int)d, (int)F, (int)E,
+                                                      rt.status, rt.stream),
+                             "gemm_tc_grouped (experts, down)");
+                done = true;
             }
-        } else {
+        }
+        if (!done) {
             if (!gated_expert)
                 check_launch(imp_grouped_gemm_ex(hid.data, F, 0, x.data, x.stride0, 0, row_token, w_up.data, nullptr, F * d, d, seg, (int)P, (int)F, (int)d,
                                                  (int)E, 0, GROUPED_RELU2, nullptr, 0, 0, 0.f, dt, rt.stream),

@@ -372,12 +372,14 @@ __global__ void moe_combine_kernel(TA* __restrict__ out, const TA* __restrict__ 
     }
 }
 
-// dst[r] = src[idx[r]]: rows of d values, 16 bytes a thread where the rows allow it.
+// dst[r] = src[idx[r]] for r < *n: rows of d values, 16 bytes a thread where the rows allow it.
 template <typename TA>
-__global__ void gather_rows_kernel(TA* __restrict__ dst, const TA* __restrict__ src, int64_t ld, const int* __restrict__ idx, int d, int vec) {
+__global__ void gather_rows_kernel(TA* __restrict__ dst, const TA* __restrict__ src, int64_t ld, const int* __restrict__ idx, const int* __restrict__ n,
+                                   int d, int vec) {
     pdl_wait();
     pdl_launch_dependents();
     const int64_t r = blockIdx.x;
+    if (r >= *n) return;
     const TA* from = src + (int64_t)idx[r] * ld;
     TA* to = dst + r * d;
     if (vec) {
@@ -390,15 +392,16 @@ __global__ void gather_rows_kernel(TA* __restrict__ dst, const TA* __restrict__ 
 
 }  // namespace
 
-IMP_API int imp_gather_rows(void* dst, const void* src, int64_t ld, const int* idx, int n_rows, int d, int dtype, void* stream) {
-    if (n_rows == 0) return 0;
-    IMP_CHECK_ARG(dst && src && idx && d > 0, "imp_gather_rows: bad argument");
+// `n`: how many rows of the list there are (device memory; at most max_rows).
+IMP_API int imp_gather_rows(void* dst, const void* src, int64_t ld, const int* idx, const int* n, int max_rows, int d, int dtype, void* stream) {
+    if (max_rows == 0) return 0;
+    IMP_CHECK_ARG(dst && src && idx && n && d > 0, "imp_gather_rows: bad argument");
     const int el = dtype == IMP_F32 ? 4 : 2;
     const int vec = ((int64_t)d * el % 16 == 0 && ld * el % 16 == 0 && (uintptr_t)dst % 16 == 0 && (uintptr_t)src % 16 == 0) ? 1 : 0;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = dtype == IMP_F32 ? imp_launch(gather_rows_kernel<float>, dim3(n_rows), dim3(128), 0, s, (float*)dst, (const float*)src, ld, idx, d, vec)
-                                     : imp_launch(gather_rows_kernel<__nv_bfloat16>, dim3(n_rows), dim3(128), 0, s, (__nv_bfloat16*)dst,
-                                                  (const __nv_bfloat16*)src, ld, idx, d, vec);
+    cudaError_t e = dtype == IMP_F32 ? imp_launch(gather_rows_kernel<float>, dim3(max_rows), dim3(128), 0, s, (float*)dst, (const float*)src, ld, idx, n, d, vec)
+                                     : imp_launch(gather_rows_kernel<__nv_bfloat16>, dim3(max_rows), dim3(128), 0, s, (__nv_bfloat16*)dst,
+                                                  (const __nv_bfloat16*)src, ld, idx, n, d, vec);
     if (e != cudaSuccess) {
         imp_set_error("imp_gather_rows: %s", cudaGetErrorString(e));
         return (int)e;

@@ -351,6 +351,23 @@ def paged_attention_generic(out: torch.Tensor, q: torch.Tensor, n_q_heads: int, 
     return out
 
 
+GROUPED_PLAIN, GROUPED_SILU, GROUPED_GELU, GROUPED_CLIPPED, GROUPED_RELU2 = 0, 2, 4, 5, 6
+
+
+def gemm_bf16_tc_grouped(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, seg: torch.Tensor, status: torch.Tensor, epilogue: int = GROUPED_PLAIN,
+                         limit: float = 0.0) -> torch.Tensor:
+    """Rows seg[g] ... seg[g + 1] of out = the same rows of a[M, K] @ w[g].T for w[G, N, K] (gated epilogues: interleaved
+    in runs of 8, out N / 2 wide)."""
+    _need_cuda(out, a, w, seg)
+    G, N, K = w.shape
+    assert w.is_contiguous() and a.shape[1] == K and a.dtype == w.dtype == out.dtype == torch.bfloat16
+    assert seg.dtype == torch.int32 and seg.numel() == G + 1 and out.shape[0] == a.shape[0] and out.stride(1) == a.stride(1) == 1
+    assert out.shape[1] == (N // 2 if epilogue in (GROUPED_SILU, GROUPED_GELU, GROUPED_CLIPPED) else N)
+    L.check(L.load().imp_gemm_bf16_tc_grouped(out.data_ptr(), out.stride(0), int(epilogue), float(limit), a.data_ptr(), a.stride(0), w.data_ptr(),
+                                              seg.data_ptr(), a.shape[0], N, K, G, _ptr(status), _stream()), "gemm_bf16_tc_grouped")
+    return out
+
+
 def gemm_f32(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """out[M,N] = a[M,K] @ w[N,K]^T, true 32-bit."""
     _need_cuda(out, a, w)

@@ -45,6 +45,10 @@ _SIGNATURES = {
         c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,          # block_table, bt_stride, seq_of_token, positions, T, B
         c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int,   # Hq, Hkv, Dh, P, pages, scale, window, dtype
         c_void_p, c_void_p]),                                       # status, stream
+    "imp_gemm_bf16_tc_grouped": (c_int, [c_void_p, c_int64, c_int, c_float, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                                         c_void_p, c_void_p]),
+    "imp_grouped_gemm_ex": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p,
+                                    c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_int, c_float, c_int, c_void_p]),
     "imp_gemm_f32": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
     "imp_gemm_bf16_small_m": (c_int, [c_void_p, c_int64, c_int, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int,
                                       c_int, c_void_p]),

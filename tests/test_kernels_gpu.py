@@ -176,6 +176,47 @@ def test_gemm_f32_edges(K, M, N, K_):
     assert torch.equal(K.gemm_f32(torch.empty(M, N, device=DEV), wide[:, 3:3 + K_], w), out)
 
 
+# Routed rows on the tensor-memory products.  The average number of rows a group decides the kernel (tiles of 32, 64 and 128 of the
+# list's rows beside streamed weights; pairs of CTAs), so every kernel meets groups without rows, with one, with a whole tile, one more,
+# and many tiles; a list shorter than its buffer; matrices that are no multiple of a tile; every epilogue.
+GROUP_ROWS = [[1, 0, 2, 0], [0, 0, 7, 32, 33, 1, 0, 64, 30], [31, 65, 0, 40], [64, 1, 129, 0, 127], [0, 256, 257, 1, 0, 130, 300], [700], [0, 3] * 40 + [90]]
+
+
+@pytest.mark.parametrize("counts", GROUP_ROWS)
+@pytest.mark.parametrize("N,K_,spare", [(48, 40, 0), (272, 136, 5), (528, 200, 40)])
+@pytest.mark.parametrize("epi", [0, 2, 4, 5, 6])
+def test_gemm_bf16_tc_grouped(K, counts, N, K_, spare, epi):
+    G, total = len(counts), sum(counts)
+    M = total + spare
+    a = rnd(M, K_, dtype=torch.bfloat16, seed=3).to(DEV)
+    if spare:
+        a[total:] = float("nan")                       # rows that no group has
+    w = rnd(G, N, K_, dtype=torch.bfloat16, seed=4, scale=0.2).to(DEV)
+    seg = torch.tensor([sum(counts[:g]) for g in range(G + 1)], dtype=torch.int32, device=DEV)
+    cols = N // 2 if epi in (2, 4, 5) else N
+    out = torch.full((M, cols + 8), -7.0, dtype=torch.bfloat16, device=DEV)
+    status = K.new_status(DEV)
+    K.gemm_bf16_tc_grouped(out[:, :cols], a, w, seg, status, epi, 1.5)
+    K.check_status(status)
+    assert (out[:, cols:] == -7.0).all() and (out[total:] == -7.0).all()
+    for g, n in enumerate(counts):
+        lo = int(seg[g])
+        z = a[lo:lo + n].double() @ w[g].double().T
+        if epi == 6:
+            z = z.clamp(min=0) ** 2
+        elif epi:
+            z = z.view(n, N // 16, 2, 8)
+            gate, up = z[:, :, 0].reshape(n, cols), z[:, :, 1].reshape(n, cols)
+            if epi == 2:
+                z = gate * torch.sigmoid(gate) * up
+            elif epi == 4:
+                z = torch.nn.functional.gelu(gate, approximate="tanh") * up
+            else:
+                gate, up = gate.clamp(max=1.5), up.clamp(-1.5, 1.5)
+                z = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+        close(out[lo:lo + n, :cols], z, torch.bfloat16, max(float(z.abs().max()), 1.0) if n else 1.0)
+
+
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 7, 8, 9, 16])
 @pytest.mark.parametrize("N,K_", [(10, 64), (257, 200), (96, 4104), (50, 100)])
 @pytest.mark.parametrize("odtype", [torch.bfloat16, torch.float32])
