@@ -149,6 +149,30 @@ __device__ __forceinline__ void gs_cp_async4(void* dst, const void* src, bool va
                  "r"(valid ? 4 : 0) : "memory");
 }
 
+// Two neighbouring dimensions at a time (fma.rn.f32x2): half the instructions of the two sums and the update.
+__device__ __forceinline__ unsigned long long gs_pair(float lo, float hi) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ unsigned long long gs_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long gs_mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// (x.lo + y.lo) + (x.hi + y.hi)
+__device__ __forceinline__ float gs_sum4(unsigned long long x, unsigned long long y) {
+    float a, b, c, d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(c), "=f"(d) : "l"(y));
+    return __fadd_rn(__fadd_rn(a, c), __fadd_rn(b, d));
+}
+
 // DPL: key dimensions per lane (D <= 8 * DPL).  Lane r of a column holds dimensions [r * DPL, (r + 1) * DPL) of its
 // column of S in registers.  (Eight lanes a column: with four, a CTA's four warps had a scheduler each and every
 // dependent instruction waited out its latency, 730 cycles a token at D = 128; two warps a scheduler hide part of it.
@@ -163,38 +187,49 @@ __device__ __forceinline__ void gs_cp_async4(void* dst, const void* src, bool va
 // Per token, with a = S^T k, c = S^T q (both on the state before the token) and kq = k . q:
 //     u = beta (v - g a);   o = g c + u kq;   S <- g S + k u^T
 // which is the recurrence's read-out S_new^T q written so that both reductions over the key dimension start from
-// the old state at once: one round of shuffles per token on the critical path instead of two.
-template <int DPL, bool VEC>
-__global__ void __launch_bounds__(GS_BLOCK, 1) gdr_scan_kernel(
+// the old state at once.  Only a's round of shuffles is on the way from token to token: c's partial sums are kept for eight
+// tokens and then added over the lanes by one transposing tree (7 exchanges for eight tokens instead of 24), which leaves
+// token r's read-out in lane r; kq, the same for every column, is made once per chunk.
+//
+// What bounds it: that way from token to token, and the bytes of k and q that every thread takes from shared memory (128 a
+// token at DPL 16).  2,048 tokens of 16 heads of 128 x 128: 395 us, 562 with the sums and the update one dimension at a time, c's
+// shuffles beside a's and 32 columns a CTA.  COLS: columns
+// of a CTA, 32, or 16 (half a block of the layout) while that still leaves an SM a CTA or less, so that a scheduler serves one
+// warp instead of two.  SINGLE: every sequence brings one token (a decode step), where the state's way in and out is all there
+// is: without the eight tokens in flight three CTAs instead of one share an SM.  The same operations in the same order.
+template <int DPL, bool VEC, int COLS, bool SINGLE>
+__global__ void __launch_bounds__(COLS * GS_LANES, SINGLE ? 3 : 1) gdr_scan_kernel(
     const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc, const float* __restrict__ beta,
     const float* __restrict__ decay, float* __restrict__ state, float* __restrict__ out, const int* __restrict__ q_start,
     const int* __restrict__ slots, int G, int D, int H, int Dv) {
     pdl_wait();
     pdl_launch_dependents();
+    constexpr int THREADS = COLS * GS_LANES, PARTS = GS_COLS / COLS, P2 = DPL / 2;
     constexpr int ROW = DPL + 4;                          // padded so that the eight lanes' 16-byte reads miss each other's banks
-    constexpr int CH = DPL <= 16 ? 16 : 8;                // tokens per chunk
+    constexpr int CH = SINGLE ? 1 : DPL <= 16 ? 16 : 8;   // tokens per chunk
+    constexpr int GROUP = SINGLE ? 1 : 8;                              // tokens whose read-outs are added up together
     __shared__ __align__(16) float k_s[2][CH][GS_LANES * ROW];
     __shared__ __align__(16) float q_s[2][CH][GS_LANES * ROW];
-    __shared__ float v_s[2][CH][GS_COLS];
-    __shared__ float g_s[2][CH], b_s[2][CH];
-    __shared__ float o_s[CH][GS_COLS];
+    __shared__ float v_s[2][CH][COLS];
+    __shared__ float g_s[2][CH], b_s[2][CH], kq_s[CH];
+    __shared__ float o_s[CH][COLS];
     const int tid = threadIdx.x, r = tid & (GS_LANES - 1), ci = tid / GS_LANES;
-    const int col0 = blockIdx.x * GS_COLS;
+    const int col0 = blockIdx.x * COLS;
     const int h = blockIdx.y, seq = blockIdx.z;
     const int hk = h / (H / G);
     const int start = q_start[seq], n = q_start[seq + 1] - start;
-    if (n <= 0) return;
-    float* S = state + ((((int64_t)slots[seq] * H + h) * gridDim.x + blockIdx.x) * DPL) * GS_BLOCK + tid;
-    float s[DPL];
+    if (n <= 0 || (SINGLE && n != 1)) return;
+    float* S = state + ((((int64_t)slots[seq] * H + h) * (gridDim.x / PARTS) + blockIdx.x / PARTS) * DPL) * GS_BLOCK + blockIdx.x % PARTS * THREADS + tid;
+    unsigned long long s[P2];
 #pragma unroll
-    for (int i = 0; i < DPL; ++i) s[i] = S[i * GS_BLOCK];
+    for (int i = 0; i < P2; ++i) s[i] = gs_pair(S[2 * i * GS_BLOCK], S[(2 * i + 1) * GS_BLOCK]);
     const int nqk = G * D;
     const int64_t hv = (int64_t)H * Dv;
     auto load_chunk = [&](int t0, int buf) {
         const int nt = min(CH, n - t0);
         if (VEC) {
             constexpr int V4 = GS_LANES * DPL / 4;                      // 16-byte pieces of a (padded) row: 4 dimensions, all inside one lane's run
-            for (int e = tid; e < CH * V4; e += GS_BLOCK) {
+            for (int e = tid; e < CH * V4; e += THREADS) {
                 const int tt = e / V4, d = (e - tt * V4) * 4;
                 const bool ok = tt < nt && d < D;
                 const int64_t src = ok ? (int64_t)(start + t0 + tt) * nqk + hk * D + d : 0;
@@ -203,7 +238,7 @@ __global__ void __launch_bounds__(GS_BLOCK, 1) gdr_scan_kernel(
                 gs_cp_async16(&q_s[buf][tt][dst], qn + src, ok);
             }
         } else {
-            for (int e = tid; e < CH * GS_LANES * DPL; e += GS_BLOCK) {
+            for (int e = tid; e < CH * GS_LANES * DPL; e += THREADS) {
                 const int tt = e / (GS_LANES * DPL), d = e - tt * (GS_LANES * DPL);
                 const bool ok = tt < nt && d < D;
                 const int64_t src = ok ? (int64_t)(start + t0 + tt) * nqk + hk * D + d : 0;
@@ -212,8 +247,8 @@ __global__ void __launch_bounds__(GS_BLOCK, 1) gdr_scan_kernel(
                 gs_cp_async4(&q_s[buf][tt][dst], qn + src, ok);
             }
         }
-        for (int e = tid; e < CH * GS_COLS; e += GS_BLOCK) {
-            const int tt = e / GS_COLS, c = e - tt * GS_COLS;
+        for (int e = tid; e < CH * COLS; e += THREADS) {
+            const int tt = e / COLS, c = e - tt * COLS;
             const bool ok = tt < nt && col0 + c < Dv;
             gs_cp_async4(&v_s[buf][tt][c], vc + (ok ? (int64_t)(start + t0 + tt) * hv + (int64_t)h * Dv + col0 + c : 0), ok);
         }
@@ -236,50 +271,90 @@ __global__ void __launch_bounds__(GS_BLOCK, 1) gdr_scan_kernel(
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         }
         __syncthreads();
-        for (int tt = 0; tt < nt; ++tt) {
-            const float g = g_s[buf][tt], b = b_s[buf][tt], v = v_s[buf][tt][ci];
-            const float4* k4 = reinterpret_cast<const float4*>(&k_s[buf][tt][r * ROW]);
-            const float4* q4 = reinterpret_cast<const float4*>(&q_s[buf][tt][r * ROW]);
-            float a0 = 0.f, a1 = 0.f, c0 = 0.f, c1 = 0.f, e0 = 0.f, e1 = 0.f;
+        if (tid < (SINGLE ? 32 : CH * GS_LANES)) {   // k . q of the chunk's tokens: eight lanes a token, whole warps
+            const int kt = SINGLE ? 0 : tid / GS_LANES;
+            const ulonglong2* k2 = reinterpret_cast<const ulonglong2*>(&k_s[buf][kt][r * ROW]);
+            const ulonglong2* q2 = reinterpret_cast<const ulonglong2*>(&q_s[buf][kt][r * ROW]);
+            unsigned long long e0 = 0ull, e1 = 0ull;
 #pragma unroll
-            for (int i = 0; i < DPL / 4; ++i) {
-                const float4 kk = k4[i], qq = q4[i];
-                a0 = fmaf(s[4 * i], kk.x, a0);     a1 = fmaf(s[4 * i + 1], kk.y, a1);
-                a0 = fmaf(s[4 * i + 2], kk.z, a0); a1 = fmaf(s[4 * i + 3], kk.w, a1);
-                c0 = fmaf(s[4 * i], qq.x, c0);     c1 = fmaf(s[4 * i + 1], qq.y, c1);
-                c0 = fmaf(s[4 * i + 2], qq.z, c0); c1 = fmaf(s[4 * i + 3], qq.w, c1);
-                e0 = fmaf(kk.x, qq.x, e0);         e1 = fmaf(kk.y, qq.y, e1);
-                e0 = fmaf(kk.z, qq.z, e0);         e1 = fmaf(kk.w, qq.w, e1);
+            for (int i = 0; i < P2 / 2; ++i) {
+                e0 = gs_fma2(k2[i].x, q2[i].x, e0);
+                e1 = gs_fma2(k2[i].y, q2[i].y, e1);
             }
-            float a = a0 + a1, c = c0 + c1, kq = e0 + e1;
-            a += __shfl_xor_sync(0xffffffffu, a, 1);
-            c += __shfl_xor_sync(0xffffffffu, c, 1);
+            float kq = gs_sum4(e0, e1);
             kq += __shfl_xor_sync(0xffffffffu, kq, 1);
-            a += __shfl_xor_sync(0xffffffffu, a, 2);
-            c += __shfl_xor_sync(0xffffffffu, c, 2);
             kq += __shfl_xor_sync(0xffffffffu, kq, 2);
-            a += __shfl_xor_sync(0xffffffffu, a, 4);
-            c += __shfl_xor_sync(0xffffffffu, c, 4);
             kq += __shfl_xor_sync(0xffffffffu, kq, 4);
-            const float u = b * (v - g * a);
-#pragma unroll
-            for (int i = 0; i < DPL / 4; ++i) {
-                const float4 kk = k4[i];
-                s[4 * i] = fmaf(kk.x, u, g * s[4 * i]);
-                s[4 * i + 1] = fmaf(kk.y, u, g * s[4 * i + 1]);
-                s[4 * i + 2] = fmaf(kk.z, u, g * s[4 * i + 2]);
-                s[4 * i + 3] = fmaf(kk.w, u, g * s[4 * i + 3]);
-            }
-            if (r == 0) o_s[tt][ci] = fmaf(u, kq, g * c);
+            if (r == 0) kq_s[kt] = kq;
         }
         __syncthreads();
-        for (int e = tid; e < nt * GS_COLS; e += GS_BLOCK) {
-            const int tt = e / GS_COLS, c = e - tt * GS_COLS;
+        for (int tt0 = 0; tt0 < nt; tt0 += GROUP) {
+            const int m = min(GROUP, nt - tt0);
+            float c[GROUP], own_u = 0.f;
+            auto token = [&](int j) {
+                const int tt = tt0 + j;
+                const float g = g_s[buf][tt], b = b_s[buf][tt], v = v_s[buf][tt][ci];
+                const ulonglong2* k2 = reinterpret_cast<const ulonglong2*>(&k_s[buf][tt][r * ROW]);
+                const ulonglong2* q2 = reinterpret_cast<const ulonglong2*>(&q_s[buf][tt][r * ROW]);
+                unsigned long long k[P2], a0 = 0ull, a1 = 0ull, c0 = 0ull, c1 = 0ull;
+#pragma unroll
+                for (int i = 0; i < P2 / 2; ++i) {
+                    const ulonglong2 kk = k2[i], qq = q2[i];
+                    k[2 * i] = kk.x, k[2 * i + 1] = kk.y;
+                    a0 = gs_fma2(s[2 * i], kk.x, a0);
+                    a1 = gs_fma2(s[2 * i + 1], kk.y, a1);
+                    c0 = gs_fma2(s[2 * i], qq.x, c0);
+                    c1 = gs_fma2(s[2 * i + 1], qq.y, c1);
+                }
+                float a = gs_sum4(a0, a1);
+                c[j] = gs_sum4(c0, c1);
+                a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 1));
+                a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 2));
+                a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 4));
+                const float u = __fmul_rn(b, __fmaf_rn(-g, a, v));
+                if (SINGLE || r == j) own_u = u;
+                const unsigned long long u2 = gs_pair(u, u), g2 = gs_pair(g, g);
+#pragma unroll
+                for (int i = 0; i < P2; ++i) s[i] = gs_fma2(k[i], u2, gs_mul2(g2, s[i]));
+            };
+            if (m == GROUP) {
+#pragma unroll
+                for (int j = 0; j < GROUP; ++j) token(j);
+            } else {
+#pragma unroll
+                for (int j = 0; j < GROUP; ++j) {
+                    c[j] = 0.f;
+                    if (j < m) token(j);
+                }
+            }
+#pragma unroll
+            for (int o = GROUP / 2; o > 0; o >>= 1) {
+                const bool up = r & o;
+#pragma unroll
+                for (int j = 0; j < o; ++j) {
+                    const float keep = up ? c[j + o] : c[j], give = up ? c[j] : c[j + o];
+                    c[j] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, o));
+                }
+            }
+            if constexpr (SINGLE) {   // the tree's sums without its transposition
+#pragma unroll
+                for (int o = GS_LANES / 2; o > 0; o >>= 1) c[0] = __fadd_rn(c[0], __shfl_xor_sync(0xffffffffu, c[0], o));
+            }
+            if (r < m) o_s[tt0 + r][ci] = __fmaf_rn(own_u, kq_s[tt0 + r], __fmul_rn(g_s[buf][tt0 + r], c[0]));
+        }
+        __syncthreads();
+        for (int e = tid; e < nt * COLS; e += THREADS) {
+            const int tt = e / COLS, c = e - tt * COLS;
             if (col0 + c < Dv) out[(int64_t)(start + t0 + tt) * hv + (int64_t)h * Dv + col0 + c] = o_s[tt][c];
         }
     }
 #pragma unroll
-    for (int i = 0; i < DPL; ++i) S[i * GS_BLOCK] = s[i];
+    for (int i = 0; i < P2; ++i) {
+        float lo, hi;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(s[i]));
+        S[2 * i * GS_BLOCK] = lo;
+        S[(2 * i + 1) * GS_BLOCK] = hi;
+    }
 }
 
 // -------------------------------------------------------------------------------------- output
@@ -370,8 +445,9 @@ IMP_API int64_t imp_gdr_state_floats(int H, int D, int Dv) {
 
 // state: [slots, imp_gdr_state_floats(H, D, Dv)] float32 in the kernel's own layout, zero at a request's start, updated in
 // place; out: [n_tokens, H * Dv] float32.
-IMP_API int imp_gdr_scan(const float* qn, const float* kn, const float* vc, const float* beta, const float* decay, float* state,
-                         float* out, const int* q_start, const int* slots, int n_seqs, int G, int D, int H, int Dv, void* stream) {
+// single: every sequence has one token.
+IMP_API int imp_gdr_scan_ex(const float* qn, const float* kn, const float* vc, const float* beta, const float* decay, float* state,
+                            float* out, const int* q_start, const int* slots, int n_seqs, int G, int D, int H, int Dv, int single, void* stream) {
     if (n_seqs == 0) return 0;
     IMP_CHECK_ARG(qn && kn && vc && beta && decay && state && out && q_start && slots, "imp_gdr_scan: null pointer");
     IMP_CHECK_ARG(G > 0 && H % G == 0 && D > 0 && Dv > 0 && H <= 65535 && n_seqs <= 65535, "imp_gdr_scan: bad sizes");
@@ -380,16 +456,24 @@ IMP_API int imp_gdr_scan(const float* qn, const float* kn, const float* vc, cons
         return IMP_ERR_UNSUPPORTED;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    dim3 grid((Dv + GS_COLS - 1) / GS_COLS, H, n_seqs);
+    const int blocks = (Dv + GS_COLS - 1) / GS_COLS;
+    const bool halves = (int64_t)blocks * 2 * H * n_seqs <= imp_sm_count();
+    const dim3 grid(halves ? 2 * blocks : blocks, H, n_seqs);
     // 16-byte copies of q and k rows need rows that start on 16 bytes: D a multiple of 4 and aligned buffers
     const bool vec = D % 4 == 0 && (uintptr_t)qn % 16 == 0 && (uintptr_t)kn % 16 == 0;
     // Launched as an ordinary dependent, without the programmatic attribute: its CTAs hold three quarters of an SM's
     // registers, and resident early (waiting for the kernels before them) they starved those kernels: a 2,048-token
     // prompt of four layers took 8.1 instead of 6.7 ms.
-#define GDR_SCAN(DPL)                                                                                                          \
-    do {                                                                                                                       \
-        if (vec) gdr_scan_kernel<DPL, true><<<grid, GS_BLOCK, 0, s>>>(qn, kn, vc, beta, decay, state, out, q_start, slots, G, D, H, Dv); \
-        else gdr_scan_kernel<DPL, false><<<grid, GS_BLOCK, 0, s>>>(qn, kn, vc, beta, decay, state, out, q_start, slots, G, D, H, Dv);    \
+    // (The step of single tokens holds a third of that and is launched ahead.)
+#define GDR_SCAN_AS(DPL, VEC, COLS)                                                                                                   \
+    do {                                                                                                                              \
+        if (single) imp_launch(gdr_scan_kernel<DPL, VEC, COLS, true>, grid, dim3(COLS * GS_LANES), 0, s, qn, kn, vc, beta, decay, state, out, q_start, slots, G, D, H, Dv); \
+        else gdr_scan_kernel<DPL, VEC, COLS, false><<<grid, COLS * GS_LANES, 0, s>>>(qn, kn, vc, beta, decay, state, out, q_start, slots, G, D, H, Dv); \
+    } while (0)
+#define GDR_SCAN(DPL)                                                                                              \
+    do {                                                                                                           \
+        if (vec) { if (halves) GDR_SCAN_AS(DPL, true, GS_COLS / 2); else GDR_SCAN_AS(DPL, true, GS_COLS); }        \
+        else { if (halves) GDR_SCAN_AS(DPL, false, GS_COLS / 2); else GDR_SCAN_AS(DPL, false, GS_COLS); }          \
     } while (0)
     switch (gdr_dims_per_lane(D)) {
         case 4: GDR_SCAN(4); break;
@@ -398,7 +482,13 @@ IMP_API int imp_gdr_scan(const float* qn, const float* kn, const float* vc, cons
         default: GDR_SCAN(32); break;
     }
 #undef GDR_SCAN
+#undef GDR_SCAN_AS
     IMP_RETURN_LAUNCH();
+}
+
+IMP_API int imp_gdr_scan(const float* qn, const float* kn, const float* vc, const float* beta, const float* decay, float* state,
+                         float* out, const int* q_start, const int* slots, int n_seqs, int G, int D, int H, int Dv, void* stream) {
+    return imp_gdr_scan_ex(qn, kn, vc, beta, decay, state, out, q_start, slots, n_seqs, G, D, H, Dv, 0, stream);
 }
 
 
