@@ -6,20 +6,23 @@
 // and then merged, chunks ascending.  So the result is the same bits whatever else is in the batch, however the prompt was
 // cut, and whichever of the two forms computed it:
 //   a warp a token   (many tokens): eight neighbouring tokens a CTA, which mostly walk the same keys and meet them in L1.
-//   a CTA a token    (few tokens): its eight warps take a chunk each, the merge follows in order through shared memory.
-// A warp serves up to two query heads of a kv head, so a key and a value are read once for both.  A lane holds Dh / 32
+//   a CTA a token    (few tokens): its warps take a chunk each, the merge follows in order through shared memory.
+// A warp serves one or two query heads of a kv head; with two, a key and a value are read once for both.  A lane holds Dh / 32
 // neighbouring entries: rows of K and V are read whole (512 bytes an instruction at head size 128), and the 32 dot products
 // of a chunk are summed over the lanes by one transposing tree of 31 exchanges that leaves key i's score in lane i.
 //
-// What bounds it: latency at one row a sequence, the instructions' issue at many.  16 query heads over 8 kv heads of 128, four
-// sequences: 28 layers' launches of eight single-token steps and a step of 580 tokens 7 ms, with the plain kernel (a thread a row of
-// K, the values of 128 keys in one chain) 24.
+// What bounds it: latency at one row a sequence, the instructions' issue at many.  16 query heads over 8 kv heads of 128:
+//   four sequences of 60 to 260 keys, a token each     8.1 us with 16 warps of one head, 11.3 with 8 of two, 10.3 with 8 of one
+//   sixteen of 300                                     16.0, 13.1, 22.5
+//   four prompts of 60 to 260 tokens (a warp a token)  82 us with two heads and two CTAs an SM, 101 with one CTA, 89 with one head
+// hence the lines in af_launch.  The plain kernel (a thread a row of K, the values of 128 keys in one chain) took 24 ms where
+// this one takes 4.5: 28 layers, eight steps of four single tokens and a step of 580 tokens.
 #include "common.cuh"
 #include "attention_f32.h"
 
 namespace {
 
-constexpr int AF_WARPS = 8, AF_KEYS = 32;
+constexpr int AF_KEYS = 32;
 
 struct AfArgs {
     float* out;
@@ -135,8 +138,8 @@ __device__ __forceinline__ float af_over(float acc, float l, bool own) {
 }
 
 // Grid (tokens / 8 or tokens, kv heads x groups of GH query heads).
-template <int DV, int GH, bool CTA_A_TOKEN>
-__global__ void __launch_bounds__(AF_WARPS * 32) attention_f32_kernel(const AfArgs a) {
+template <int DV, int GH, int AF_WARPS, int MIN_CTAS, bool CTA_A_TOKEN>
+__global__ void __launch_bounds__(AF_WARPS * 32, MIN_CTAS) attention_f32_kernel(const AfArgs a) {
     pdl_wait();
     pdl_launch_dependents();
     constexpr int DH = 32 * DV;
@@ -233,14 +236,19 @@ __global__ void __launch_bounds__(AF_WARPS * 32) attention_f32_kernel(const AfAr
     }
 }
 
-template <int DV, int GH>
-cudaError_t af_launch(const AfArgs& a, cudaStream_t stream) {
+template <int DV, int GH, int WARPS, int MIN_CTAS, bool CTA_A_TOKEN>
+cudaError_t af_run(const AfArgs& a, cudaStream_t stream) {
     const int sets = (a.Hq / a.Hkv + GH - 1) / GH;
-    // A CTA a token while that leaves the device with no more than about eight CTAs an SM to run; from there on the
-    // tokens themselves fill it and the barriers of a CTA's merge only cost.
-    if ((int64_t)a.n_tokens * a.Hkv * sets <= 8ll * imp_sm_count())
-        return imp_launch(attention_f32_kernel<DV, GH, true>, dim3(a.n_tokens, a.Hkv * sets), AF_WARPS * 32, 0, stream, a);
-    return imp_launch(attention_f32_kernel<DV, GH, false>, dim3((a.n_tokens + AF_WARPS - 1) / AF_WARPS, a.Hkv * sets), AF_WARPS * 32, 0, stream, a);
+    return imp_launch(attention_f32_kernel<DV, GH, WARPS, MIN_CTAS, CTA_A_TOKEN>, dim3(CTA_A_TOKEN ? a.n_tokens : (a.n_tokens + WARPS - 1) / WARPS, a.Hkv * sets),
+                      WARPS * 32, 0, stream, a);
+}
+
+template <int DV>
+cudaError_t af_launch(const AfArgs& a, cudaStream_t stream) {
+    const int64_t heads = (int64_t)a.n_tokens * a.Hq;
+    if (heads <= imp_sm_count()) return af_run<DV, 1, 16, 1, true>(a, stream);
+    if (a.Hq == a.Hkv) return heads <= 8ll * imp_sm_count() ? af_run<DV, 1, 8, 1, true>(a, stream) : af_run<DV, 1, 8, 3, false>(a, stream);
+    return heads <= 8ll * imp_sm_count() ? af_run<DV, 2, 8, 1, true>(a, stream) : af_run<DV, 2, 8, 2, false>(a, stream);
 }
 
 }  // namespace
@@ -252,11 +260,7 @@ int imp_attention_f32(float* out, int64_t out_stride, const float* q, int64_t q_
     if ((Dh != 64 && Dh != 128 && Dh != 256) || ptrs % 16 || out_stride % 4 || q_stride % 4 || Hq > 65535) return IMP_ERR_UNSUPPORTED;
     const AfArgs a{out, q, k_cache, v_cache, block_table, seq_of_token, positions, status, out_stride, q_stride,
                    bt_stride, n_tokens, n_seqs, Hq, Hkv, page_size, num_pages, window, scale};
-    const bool pairs = Hq > Hkv;
-    cudaError_t e;
-    if (Dh == 64) e = pairs ? af_launch<2, 2>(a, stream) : af_launch<2, 1>(a, stream);
-    else if (Dh == 128) e = pairs ? af_launch<4, 2>(a, stream) : af_launch<4, 1>(a, stream);
-    else e = pairs ? af_launch<8, 2>(a, stream) : af_launch<8, 1>(a, stream);
+    const cudaError_t e = Dh == 64 ? af_launch<2>(a, stream) : Dh == 128 ? af_launch<4>(a, stream) : af_launch<8>(a, stream);
     if (e != cudaSuccess) {
         imp_set_error("imp_attention_f32: %s", cudaGetErrorString(e));
         return (int)e;
