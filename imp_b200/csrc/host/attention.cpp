@@ -441,6 +441,12 @@ bool linear_qkv_rope(Step& st, Tensor q_out, const Tensor& x, const Tensor& w, c
     if (lib || x.dtype != BF16 || w.dtype != BF16) return false;
     const int T = (int)rows(x);
     if (T < 256 || (g.dh != 64 && g.dh != 128) || rot.rot_dim != g.dh) return false;
+    // The fused epilogue takes about 10 us a tile, twice the plain one and more, which the next tiles' multiply-adds hide only where
+    // a pair of CTAs has several tiles of a long K; elsewhere the plain product and the kernel behind it are faster.  Fused against
+    // plain and rotary kernel, q,k,v of 6144 x 4096: 512 tokens 37.1 / 31.3 us, 576 36.5 / 34.8, 1,024 56.8 / 54.7, 2,048 81.4 / 87.6;
+    // 7168 x 5120: 512 42.3 / 39.6, 576 56.7 / 66.1, 2,048 116 / 129; 4096 x 1024: 512 20.2 / 15.4, 2,048 34.2 / 29.7.  The same bits.
+    const int64_t tiles = (int64_t)((T + 255) / 256) * ((rows(w) + 255) / 256), pairs = std::max(rt.sm_count / 2, 1);
+    if (tiles <= pairs || cols(x) < 4096) return false;
     check_cache(cache, g);
     const ImpCacheView& c = cache.view;
     need(rows(w) == (int64_t)(g.hq + 2 * g.hkv) * g.dh && cols(w) == cols(x) && q_out.dtype == BF16 && rows(q_out) == T &&

@@ -1086,6 +1086,47 @@ def test_sampler_mirostat_state_typical_and_dry_through_the_class(K):
     assert got == alone
 
 
+# Behind a plain product of 256 tokens and more stands a kernel that gives the fused epilogue's bits: head counts below, at and
+# beyond what a warp takes (8 heads of 128, 16 of 64), ones that leave part of a round empty; bad places are reported.
+@pytest.mark.parametrize("Hq,Hkv,Dh,page,with_norm", [(32, 8, 128, 16, True), (3, 1, 64, 8, True), (5, 2, 128, 32, False), (17, 1, 64, 5, True), (6, 1, 128, 64, True)])
+def test_plain_projection_and_rotary_kernel_give_the_fused_epilogues_bits(K, Hq, Hkv, Dh, page, with_norm):
+    T, Kd = 300, 192
+    lengths, starts = [210, 177], [40, 47]
+    bt, num_pages = paged_layout(lengths, page, seed=4)
+    toks = [(s, p) for s, (st, n) in enumerate(zip(starts, lengths)) for p in range(st, n)]
+    seq = torch.tensor([s for s, _ in toks], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([p for _, p in toks], dtype=torch.int32, device=DEV)
+    bt = bt.to(DEV)
+    N = (Hq + 2 * Hkv) * Dh
+    x, w = rnd(T, Kd, dtype=torch.bfloat16, seed=41).to(DEV), rnd(N, Kd, dtype=torch.bfloat16, seed=42, scale=0.1).to(DEV)
+    qw, kw = ((1 + 0.2 * rnd(Dh, seed=43)).to(DEV), (1 + 0.2 * rnd(Dh, seed=44)).to(DEV)) if with_norm else (None, None)
+    i = torch.arange(Dh // 2, dtype=torch.float64)
+    ang = torch.arange(256, dtype=torch.float64)[:, None] * (1e4 ** (-2.0 * i / Dh))[None, :]
+    cos, sin = ang.cos().float().to(DEV), ang.sin().float().to(DEV)
+    status = K.new_status(DEV)
+    cache = [torch.zeros(num_pages, Hkv, page, Dh, dtype=torch.bfloat16, device=DEV) for _ in range(4)]
+    q = torch.empty(T, Hq * Dh, dtype=torch.bfloat16, device=DEV)
+    assert K.linear_qkv_rope(q, x, w, Hq, Hkv, Dh, qw, kw, 1e-6, cos, sin, pos, seq, bt, cache[0], cache[1], status)
+    qkv = torch.empty(T, N, dtype=torch.bfloat16, device=DEV)
+    assert K.gemm_bf16_tc(qkv, x, w, status=status)
+    raw = qkv.clone()
+    K.qk_norm_rope_kv_write(qkv, Hq, Hkv, Dh, qw, kw, 1e-6, cos, sin, Dh, pos, seq, bt, cache[2], cache[3], status)
+    K.check_status(status)
+    assert torch.equal(qkv[:, :Hq * Dh], q) and torch.equal(cache[2], cache[0]) and torch.equal(cache[3], cache[1])
+    assert torch.equal(qkv[:, (Hq + Hkv) * Dh:], raw[:, (Hq + Hkv) * Dh:])
+    # without a cache k turns in place; the same bits
+    alone = raw.clone()
+    K.qk_norm_rope_kv_write(alone, Hq, Hkv, Dh, qw, kw, 1e-6, cos, sin, Dh, pos, seq, bt, None, None, status)
+    s0, p0 = toks[0]
+    assert torch.equal(alone[0, Hq * Dh:(Hq + Hkv) * Dh].view(Hkv, Dh), cache[2][int(bt[s0, p0 // page]), :, p0 % page])
+    for bad, match in ((dict(pos=torch.full_like(pos, -1)), "position"), (dict(bt=bt.clone().fill_(num_pages)), "page")):
+        before = cache[2].clone()
+        K.qk_norm_rope_kv_write(raw.clone(), Hq, Hkv, Dh, qw, kw, 1e-6, cos, sin, Dh, bad.get("pos", pos), seq, bad.get("bt", bt), cache[2], cache[3], status)
+        with pytest.raises(Exception, match=match):
+            K.check_status(status)
+        assert torch.equal(cache[2], before)
+
+
 @pytest.mark.parametrize("Hq,Hkv,Dh,page,with_norm", [(32, 8, 128, 16, True), (3, 1, 64, 8, True), (5, 2, 128, 32, False),
                                                       (8, 4, 64, 16, True)])
 def test_fused_qkv_projection_matches_projection_then_rotary_kernel(K, Hq, Hkv, Dh, page, with_norm):
