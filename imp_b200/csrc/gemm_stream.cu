@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
                     up += gate_act.bias[n0 + (l >> 2) + 8];
                 }
                 if (n0 + (l >> 2) + 8 < N && tok < M)
-                    C[(int64_t)tok * ldc + col] = from_float<TO>(gated_f(gate, up, gate_act));
+                    C[(int64_t)tok * ldc + col] = from_float<TO>(sizeof(TO) == 2 ? gated_fast_f(gate, up, gate_act) : gated_f(gate, up, gate_act));
             }
         } else {
             // 16 rows x 8*NT tokens = NT*128 sums; thread i takes register slot i / 32 of lane i % 32.

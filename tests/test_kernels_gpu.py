@@ -1127,6 +1127,26 @@ def test_plain_projection_and_rotary_kernel_give_the_fused_epilogues_bits(K, Hq,
         assert torch.equal(cache[2], before)
 
 
+# The gated epilogues divide by fused multiply-adds: the same bits as the division, over gates from far below to far above
+# where the exponential leaves the range; few rows (weights on the M side), and pairs of CTAs.
+@pytest.mark.parametrize("M", [3, 40, 70, 128, 300])
+def test_gated_epilogues_divide_exactly(K, M):
+    F, Kd = 1000, 64
+    x = rnd(M, Kd, dtype=torch.bfloat16, seed=51).to(DEV)
+    w = rnd(2 * F, Kd, dtype=torch.bfloat16, seed=52)
+    w *= torch.logspace(-4, 1, 2 * F)[torch.randperm(2 * F, generator=torch.Generator().manual_seed(1))][:, None].bfloat16()
+    w = w.to(DEV)
+    status = K.new_status(DEV)
+    z, out = torch.empty(M, 2 * F, device=DEV), torch.empty(M, F, dtype=torch.bfloat16, device=DEV)
+    run = K.gemm_bf16_tc if M > 128 else K.gemm_bf16_tc_swap
+    assert run(z, x, w, K.TC_OUT_F32, status) and run(out, x, w, K.TC_OUT_SWIGLU, status)
+    K.check_status(status)
+    want = K.swiglu(torch.empty(M, F, device=DEV), z, 8)
+    # (beyond e^87 the fused forms hold the divisor: what is left is below 1e-30 either way)
+    tiny = want.abs() < 1e-30
+    assert float(z.abs().max()) > 100 and torch.equal(out[~tiny], want.bfloat16()[~tiny]) and (out[tiny].abs() < 1e-30).all()
+
+
 @pytest.mark.parametrize("Hq,Hkv,Dh,page,with_norm", [(32, 8, 128, 16, True), (3, 1, 64, 8, True), (5, 2, 128, 32, False),
                                                       (8, 4, 64, 16, True)])
 def test_fused_qkv_projection_matches_projection_then_rotary_kernel(K, Hq, Hkv, Dh, page, with_norm):
