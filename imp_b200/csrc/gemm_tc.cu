@@ -632,8 +632,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                         void* __restrict__ Cv, int64_t ldc, int M, int N, int K, int* status,
                         const __grid_constant__ QkvRopeArgs qkv, int splits, int kb_per_split, int64_t split_stride,
                         const __grid_constant__ CUtensorMap map_c, int tma_store, GateAct gate_act, TcGroups groups) {
-    // tma_store (bfloat16 and SwiGLU epilogues): C goes out through shared memory and TMA stores described by map_c
-    // (boxes of 128 rows x 64 columns, clipped at the matrix edges) instead of 16-byte stores from every thread.
+    // tma_store: C goes out through shared memory and TMA stores described by map_c (boxes of 128 rows x 64 columns, 32 of
+    // 32-bit values, the parts of a cut K range one below the other) instead of 16-byte stores from every thread.
     // splits > 1 (32-bit output only): the K range is cut into `splits` parts, each (tile, part) is a unit of work of its
     // own and writes its partial product split_stride elements after the part before; the caller adds the parts in order.
     IMP_TL_BEGIN(20 + EPI)
@@ -780,7 +780,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             const Unit at = locate(u);
             const uint32_t buf = local & 1u;
             bool ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * buf, (local >> 1) & 1u, status));
-            if (EPI != TC_OUT_F32 && tma_store) {
+            if (tma_store) {
                 // the four warps meet at barriers below: they go on, or give up, together
                 uint32_t all;
                 asm volatile(
@@ -808,8 +808,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             if (EPI == TC_OUT_QKV_ROPE) {
                 const QkvStage stg{tma_store && m0 + 128 <= rows ? out_stage : nullptr, &map_c, storer, quarter * 32 + lane, m0};
                 qkv_rope_row(qkv, taddr, row, n0, N, row < rows, status, stg);
-            } else if ((EPI == TC_OUT_BF16 || EPI == TC_OUT_SWIGLU_BF16) && tma_store && whole) {
-                constexpr int SUBS = EPI == TC_OUT_SWIGLU_BF16 ? 2 : 4;     // sub-tiles of 64 output columns
+            } else if (EPI != TC_OUT_QKV_ROPE && tma_store && whole) {
+                constexpr int COLS = EPI == TC_OUT_F32 ? 32 : 64;           // of a sub-tile: rows of 128 bytes
+                constexpr int SUBS = (EPI == TC_OUT_SWIGLU_BF16 ? 128 : 256) / COLS;
                 const int x0 = EPI == TC_OUT_SWIGLU_BF16 ? n0 >> 1 : n0;
                 const int r = quarter * 32 + lane;                          // row in the CTA's half of the tile
 #pragma unroll 1
@@ -819,7 +820,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                     if (storer) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     uint4 q[8];
-                    if (EPI == TC_OUT_BF16) {
+                    if constexpr (EPI == TC_OUT_F32) {
+                        float v[32];
+                        tc_ld32(taddr + (uint32_t)(j * 32), v);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            q[i] = make_uint4(__float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]), __float_as_uint(v[4 * i + 2]), __float_as_uint(v[4 * i + 3]));
+                    } else if (EPI == TC_OUT_BF16) {
 #pragma unroll
                         for (int cc = 0; cc < 2; ++cc) {
                             float v[32];
@@ -852,7 +859,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (storer) {
-                        tma_store_2d(&map_c, smem_u32(buf), x0 + j * 64, m0);
+                        tma_store_2d(&map_c, smem_u32(buf), x0 + j * COLS, EPI == TC_OUT_F32 ? at.z * M + m0 : m0);
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
                 }
@@ -1172,18 +1179,18 @@ __global__ void gemm_tc_reduce4_kernel(TO* __restrict__ out, int64_t ldc, const 
 }
 
 // ------------------------------------------------------------------------------------- host
-// A [rows, K] bfloat16 matrix with row stride ld elements, fetched in boxes of box_rows x 64 elements.
-static int make_map(CUtensorMap* map, const void* base, int rows, int K, int64_t ld, int box_rows) {
+// A [rows, K] bfloat16 (or 32-bit) matrix with row stride ld elements, in boxes of box_rows x 64 (32) elements.
+static int make_map(CUtensorMap* map, const void* base, int rows, int K, int64_t ld, int box_rows, bool f32 = false) {
     EncodeTiledFn fn = get_encode_fn();
     if (!fn) {
         imp_set_error("gemm_tc: the driver does not provide cuTensorMapEncodeTiled");
         return IMP_ERR_UNSUPPORTED;
     }
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
+    const cuuint32_t box[2] = {(cuuint32_t)(f32 ? TC_BK / 2 : TC_BK), (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+    const CUresult r = fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
@@ -1230,8 +1237,8 @@ static int launch_tc(void* C, int64_t ldc, const CUtensorMap& ma, const CUtensor
         if (tma_out < 0) { const char* e = getenv("IMP_B200_TC_TMA_STORE"); tma_out = e ? atoi(e) : 1; }
         CUtensorMap mc{};
         int tma_store = 0;
-        if (EPI != TC_OUT_F32 && tma_out && ldc % 8 == 0)
-            tma_store = make_map(&mc, C, M, EPI == TC_OUT_SWIGLU_BF16 ? N / 2 : N, ldc, 128) == 0 ? 1 : 0;
+        if (tma_out && ldc % 8 == 0)
+            tma_store = make_map(&mc, C, M, EPI == TC_OUT_SWIGLU_BF16 ? N / 2 : N, ldc, 128, EPI == TC_OUT_F32) == 0 ? 1 : 0;
         cudaError_t e = imp_launch(gemm_tc_pair_kernel<EPI>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)TC2_SMEM_BYTES, s, ma, mw128,
                                    C, ldc, M, N, K, status, QkvRopeArgs{}, 1, (K + TC_BK - 1) / TC_BK, (int64_t)0, mc, tma_store, gate_act, TcGroups{});
         if (e != cudaSuccess) { imp_set_error("gemm_tc: %s", cudaGetErrorString(e)); return (int)e; }
@@ -1284,39 +1291,35 @@ IMP_API int imp_gemm_bf16_tc(void* C, int64_t ldc, int epilogue, const void* A, 
 }
 
 // ---- many rows, few tiles: the K range in parts ------------------------------------------------------
-// A portion of a prompt (256 to about a thousand rows) times a weight of a few thousand rows makes fewer 256 x 256
-// tiles than the device has CTA pairs (512 x 4096: 32 tiles on 74 pairs).  Then the K range is cut so that
-// tiles x parts fills the pairs, each part leaves a 32-bit partial product, and gemm_tc_reduce_kernel adds them in order.
-#ifndef TC2_MIN_KB_PER_SPLIT
-#define TC2_MIN_KB_PER_SPLIT 48    // blocks of K (3072 elements) a part has at least: a launch of the pair kernel costs about
-#endif                             // 12 us before and after its MMAs, so parts of a short K gain less than their sum costs
-#ifndef TC2_MAX_SPLITS
-#define TC2_MAX_SPLITS 4
-#endif
-#ifndef TC2_SPLIT_MIN_ROWS
-#define TC2_SPLIT_MIN_ROWS 129     // from where CTA pairs take the product (decode at 160 sequences: 12.87 -> 11.76 ms a step
-#endif                             // once the down projection's 16 tiles are cut in four)
+// A portion of a prompt (129 to about two thousand rows) times a weight of a few thousand rows makes fewer 256 x 256
+// tiles than the device has CTA pairs (512 x 4096: 32 tiles on 74 pairs).  Then the K range is cut into as many parts as cost the
+// least: a pair takes 0.32 us a block of K (64), so rounds x blocks x 0.32, and with more than one part 3 us for the launch
+// that adds them plus what it reads, at 4 TB/s.  Whole, and cut with the sum: 256 x 4096 x 4096 23.9 / 15.8 us, 512 x 4096 x 4096
+// 24.6 / 20.0, 256 x 4096 x 12288 60.4 / 29.8, 512 x 4096 x 12288 61.5 / 45.0.  (While every thread stored its row of the 32-bit
+// parts, a part cost 4.5 us more.)  Parts shorter than 32 blocks would still gain (512 x 1024 x 2048 13.4 / 10.0, 512 x 1024 x 3072
+// 18.0 / 12.0) and are left out so that products of a short K add in one order at every number of rows, whichever
+// portions a prompt came in.
+constexpr double TC2_BLOCK_US = 0.32, TC2_SUM_US = 3.0, TC2_SUM_BYTES_PER_US = 4e6;
+constexpr int TC2_MIN_KB_PER_SPLIT = 32, TC2_MIN_KB_COLUMN = 8;   // blocks of K of a part; the latter for one column of tiles
+constexpr int TC2_MAX_SPLITS = 8, TC2_MAX_SPLITS_COLUMN = 16;   // the latter for one column of tiles (a router, a low-rank product)
+constexpr int TC2_SPLIT_MIN_ROWS = 129;     // from where CTA pairs take the product
 IMP_API int imp_gemm_bf16_tc_splits(int M, int N, int K) {
     static int enabled = -1;       // IMP_B200_TC_SPLIT=0: never
     if (enabled < 0) { const char* e = getenv("IMP_B200_TC_SPLIT"); enabled = e ? atoi(e) : 1; }
     const char* pair_env = getenv("IMP_B200_TC_PAIR");
     if (!enabled || M < TC2_SPLIT_MIN_ROWS || getenv("IMP_B200_TC_SIMPLE") || (pair_env && atoi(pair_env) == 0)) return 1;
-    const int tiles2 = ((M + TC2_BM - 1) / TC2_BM) * ((N + TC2_BN - 1) / TC2_BN);
-    const int pairs = imp_sm_count() / 2;
-    const int k_blocks = (K + TC_BK - 1) / TC_BK;
-    int splits = pairs / (tiles2 > 0 ? tiles2 : 1);
-    // one column of tiles (a router, a low-rank product): the parts are small, so a part may be short
-    const int min_kb = N <= TC2_BN ? 8 : TC2_MIN_KB_PER_SPLIT, max_splits = N <= TC2_BN ? 16 : TC2_MAX_SPLITS;
-    if (splits > k_blocks / min_kb) splits = k_blocks / min_kb;
-    if (splits > max_splits) splits = max_splits;
-    if (splits < 1) return 1;
-    // no part is empty: as many as parts of equal length (the last one shorter) make
-    for (int before = 0; before != splits;) {
-        before = splits;
-        const int kb = (k_blocks + splits - 1) / splits;
-        splits = (k_blocks + kb - 1) / kb;
+    const int64_t tiles = (int64_t)((M + TC2_BM - 1) / TC2_BM) * ((N + TC2_BN - 1) / TC2_BN);
+    const int pairs = imp_sm_count() / 2 > 0 ? imp_sm_count() / 2 : 1, k_blocks = (K + TC_BK - 1) / TC_BK;
+    if (tiles > pairs) return 1;
+    int best = 1;
+    double least = k_blocks * TC2_BLOCK_US;      // tiles <= pairs: one round
+    for (int want = 2; want <= (N <= TC2_BN ? TC2_MAX_SPLITS_COLUMN : TC2_MAX_SPLITS); ++want) {
+        const int kb = (k_blocks + want - 1) / want, splits = (k_blocks + kb - 1) / kb;   // parts of equal length, none empty
+        if (kb < (N <= TC2_BN ? TC2_MIN_KB_COLUMN : TC2_MIN_KB_PER_SPLIT) || splits != want) continue;
+        const double us = (double)((tiles * splits + pairs - 1) / pairs) * kb * TC2_BLOCK_US + TC2_SUM_US + (double)splits * M * N * 4 / TC2_SUM_BYTES_PER_US;
+        if (us < least) least = us, best = splits;
     }
-    return splits;
+    return best;
 }
 
 // scratch[s][M, N] (32-bit, M * N floats apart) for s < imp_gemm_bf16_tc_splits(M, N, K): the parts of A W^T.
@@ -1335,6 +1338,8 @@ IMP_API int imp_gemm_bf16_tc_partials(float* scratch, const void* A, int64_t lda
     CUtensorMap ma, mw128;
     if (int rc = make_map(&ma, A, M, K, lda, TC_BM)) return rc;
     if (int rc = make_map(&mw128, W, N, K, ldw, 128)) return rc;
+    CUtensorMap mc{};
+    const int tma_store = (int64_t)splits * M <= 0x7fffffff && make_map(&mc, scratch, splits * M, N, N, 128, true) == 0 ? 1 : 0;
     const int k_blocks = (K + TC_BK - 1) / TC_BK;
     const int kb_per_split = (k_blocks + splits - 1) / splits;
     const int units = ((M + TC2_BM - 1) / TC2_BM) * ((N + TC2_BN - 1) / TC2_BN) * splits;
@@ -1342,7 +1347,7 @@ IMP_API int imp_gemm_bf16_tc_partials(float* scratch, const void* A, int64_t lda
     const int pairs = units < sms / 2 ? units : sms / 2;
     cudaError_t e = imp_launch(gemm_tc_pair_kernel<TC_OUT_F32>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)TC2_SMEM_BYTES,
                                (cudaStream_t)stream, ma, mw128, (void*)scratch, (int64_t)N, M, N, K, status, QkvRopeArgs{}, splits,
-                               kb_per_split, (int64_t)M * N, CUtensorMap{}, 0, 0, TcGroups{});
+                               kb_per_split, (int64_t)M * N, mc, tma_store, 0, TcGroups{});
     if (e != cudaSuccess) { imp_set_error("imp_gemm_bf16_tc_partials: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;
 }

@@ -166,6 +166,26 @@ static bool gemm_tc_swap_partials(Runtime& rt, Tensor out, const Tensor& a, cons
     return true;
 }
 
+// The same for more rows, where the product of a portion leaves its K range in parts.
+static bool gemm_tc_partials(Runtime& rt, Tensor out, const Tensor& a, const Tensor& w, Branch* result) {
+    const int M = (int)rows(a), N = (int)rows(w), K = (int)cols(a);
+    const int n_splits = imp_gemm_bf16_tc_splits(M, N, K);
+    if (n_splits < 2) return false;
+    const Arena::Mark mark = rt.arena->mark();
+    float* parts = (float*)rt.arena->alloc((size_t)n_splits * M * N * 4);
+    const int rc = imp_gemm_bf16_tc_partials(parts, a.data, a.stride0, w.data, w.stride0, M, N, K, rt.status, rt.stream);
+    if (rc == -2) {
+        rt.arena->restore(mark);
+        return false;
+    }
+    ++rt.launches;
+    check_launch(rc, "gemm_bf16_tc_partials");
+    result->t = out;
+    result->parts = parts;
+    result->n_splits = n_splits;
+    return true;
+}
+
 // A summand's tensor, its unsummed parts or its routed rows added up into it.
 static void sum_term(Runtime& rt, const Tensor& t, const float* parts, int n_splits, const RoutedRows& r) {
     if (parts) {
@@ -256,6 +276,7 @@ Branch linear(Runtime& rt, Tensor out, const Tensor& x, const Tensor& w, bool ma
             if (defer && gemm_tc_swap_partials(rt, out, x, w, &b)) return b;
             if (gemm_tc_swap(rt, out, x, w)) return Branch::of(out);
         }
+        if (M > TC_SWAP_MAX_M && defer && gemm_tc_partials(rt, out, x, w, &b)) return b;
         if (gemm_tc(rt, out, x, w)) return Branch::of(out);
     } else if (library_gemm_bf16(rt, out, x, w)) {
         return Branch::of(out);
