@@ -26,12 +26,41 @@ __global__ void embedding_kernel(float* __restrict__ out, const TW* __restrict__
     for (int i = threadIdx.x; i < d; i += blockDim.x) o[i] = to_float(row[i]) * scale;
 }
 
+// The same for rows that start on 16 bytes: 16 bytes of the table a thread, a CTA per token and 128 of its pieces, so that a row is
+// asked for at once and a few tokens spread over the device.  Bound by two trips to the memory, one behind the other.
+constexpr int EMB_THREADS = 128;
+template <typename TW>
+__global__ void __launch_bounds__(EMB_THREADS) embedding_vec_kernel(float* __restrict__ out, const TW* __restrict__ table, const int* __restrict__ ids,
+                                                                    int d, int vocab, float scale, int* status) {
+    pdl_wait();
+    pdl_launch_dependents();
+    constexpr int PER = 16 / (int)sizeof(TW);
+    const int t = blockIdx.x, c = (blockIdx.y * EMB_THREADS + threadIdx.x) * PER, id = ids[t];
+    const bool there = id >= 0 && id < vocab;
+    if (!there && threadIdx.x == 0 && blockIdx.y == 0) imp_report(status, IMP_BAD_TOKEN_ID);
+    if (c >= d) return;
+    uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+    if (there) raw = *reinterpret_cast<const uint4*>(table + (int64_t)id * d + c);
+    const TW* v = reinterpret_cast<const TW*>(&raw);
+    float* o = out + (int64_t)t * d + c;
+#pragma unroll
+    for (int e = 0; e < PER; e += 4)
+        *reinterpret_cast<float4*>(o + e) = make_float4(to_float(v[e]) * scale, to_float(v[e + 1]) * scale, to_float(v[e + 2]) * scale, to_float(v[e + 3]) * scale);
+}
+
 // out[t, :] = table[ids[t], :] * scale, as 32-bit floats.
 IMP_API int imp_embedding(float* out, const void* table, const int* ids, int n_tokens, int d, int vocab,
                           int table_dtype, float scale, int* status, void* stream) {
     if (n_tokens == 0) return 0;
     IMP_CHECK_ARG(out && table && ids && d > 0 && vocab > 0, "imp_embedding: bad argument");
     cudaStream_t s = (cudaStream_t)stream;
+    const int per = table_dtype == IMP_F32 ? 4 : 8, pieces = d / per;
+    if (d % per == 0 && (uintptr_t)table % 16 == 0 && (uintptr_t)out % 16 == 0 && (pieces + EMB_THREADS - 1) / EMB_THREADS <= 65535) {
+        const dim3 grid(n_tokens, (pieces + EMB_THREADS - 1) / EMB_THREADS);
+        if (table_dtype == IMP_F32) embedding_vec_kernel<float><<<grid, EMB_THREADS, 0, s>>>(out, (const float*)table, ids, d, vocab, scale, status);
+        else embedding_vec_kernel<__nv_bfloat16><<<grid, EMB_THREADS, 0, s>>>(out, (const __nv_bfloat16*)table, ids, d, vocab, scale, status);
+        IMP_RETURN_LAUNCH();
+    }
     const int block = d >= 1024 ? 256 : 128;
     if (table_dtype == IMP_F32)
         embedding_kernel<float><<<n_tokens, block, 0, s>>>(out, (const float*)table, ids, d, vocab, scale, status);
