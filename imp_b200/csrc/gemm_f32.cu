@@ -89,7 +89,7 @@ template <int MT> constexpr int gr_smem_floats() {
 // Grid (ctas x groups of 32 rows of W, groups of MT rows of A); a cluster along x of `ctas` = 1, 2 or 4.
 template <int MT, bool ALIGNED>
 __global__ void __launch_bounds__(GR_WARPS * 32) gemm_f32_rows_kernel(float* __restrict__ C, int64_t ldc, const float* __restrict__ A, int64_t lda,
-                                                                      const float* __restrict__ W, int64_t ldw, int M, int N, int K, int ctas) {
+                                                                      const float* __restrict__ W, int64_t ldw, int M, int N, int K, int ctas, int early) {
     extern __shared__ __align__(16) float gr_mem[];
     float* ws = gr_mem;                                              // [stage][GR_ROWS][GR_PITCH]
     float* as = ws + GR_STAGES * GR_ROWS * GR_PITCH;                 // [stage][MT][GR_K]
@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(GR_WARPS * 32) gemm_f32_rows_kernel(float* __r
     At ahead{run0, 0, 0};
     open(ahead);
     At now = ahead, first = ahead;
+    if (!early) pdl_wait();
 #pragma unroll
     for (int i = 0; i < GR_STAGES - 1; ++i)
         if (ahead.run < run0 + per) {
@@ -240,7 +241,7 @@ constexpr int GT_SMEM = (GT_STAGES * GT_STAGE + GT_OUTS) * 4;   // the ring and 
 // Grid (ctas x tiles of N, tiles of M); a cluster along x of `ctas` = 2 or 4.
 template <bool ALIGNED>
 __global__ void __launch_bounds__(GT_THREADS, 3) gemm_f32_tile_kernel(float* __restrict__ C, int64_t ldc, const float* __restrict__ A, int64_t lda,
-                                                                      const float* __restrict__ W, int64_t ldw, int M, int N, int K, int ctas) {
+                                                                      const float* __restrict__ W, int64_t ldw, int M, int N, int K, int ctas, int early) {
     extern __shared__ __align__(16) float gt_mem[];
     float* sums = gt_mem + GT_STAGES * GT_STAGE;   // [output of the thread][thread]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -262,6 +263,7 @@ __global__ void __launch_bounds__(GT_THREADS, 3) gemm_f32_tile_kernel(float* __r
     };
     auto stage = [&](int i) { return gt_mem + i * GT_STAGE; };
     static_assert(GT_M == GT_N, "one fetch for both operands");
+    if (!early) pdl_wait();
 #pragma unroll
     for (int i = 0; i < GT_STAGES - 1; ++i)
         if (b0 + i < b1) fetch(W, ldw, n0, N, stage(i) + GT_M * GT_PITCH, b0 + i);
@@ -370,20 +372,22 @@ cudaError_t gf_launch(void (*kernel)(KArgs...), dim3 grid, int threads, int smem
 constexpr int GF_ROWS_MAX = 32;   // rows of A up to which W is streamed
 
 template <int MT>
-cudaError_t gr_launch(bool aligned, float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M, int N, int K, cudaStream_t s) {
+cudaError_t gr_launch(bool aligned, float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M, int N, int K, int early, cudaStream_t s) {
     // a CTA does all four runs where the groups alone give every SM two CTAs
     const int groups = (int)(((int64_t)N + GR_ROWS - 1) / GR_ROWS), sms = imp_sm_count();
     const int ctas = groups >= 2 * sms ? 1 : groups >= sms ? 2 : 4;
     const dim3 grid((unsigned)groups * ctas, (M + MT - 1) / MT);
     constexpr int smem = gr_smem_floats<MT>() * 4;
-    if (aligned) return gf_launch(gemm_f32_rows_kernel<MT, true>, grid, GR_WARPS * 32, smem, ctas, s, C, ldc, A, lda, W, ldw, M, N, K, ctas);
-    return gf_launch(gemm_f32_rows_kernel<MT, false>, grid, GR_WARPS * 32, smem, ctas, s, C, ldc, A, lda, W, ldw, M, N, K, ctas);
+    if (aligned) return gf_launch(gemm_f32_rows_kernel<MT, true>, grid, GR_WARPS * 32, smem, ctas, s, C, ldc, A, lda, W, ldw, M, N, K, ctas, early);
+    return gf_launch(gemm_f32_rows_kernel<MT, false>, grid, GR_WARPS * 32, smem, ctas, s, C, ldc, A, lda, W, ldw, M, N, K, ctas, early);
 }
 
 }  // namespace
 
-IMP_API int imp_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M,
-                         int N, int K, void* stream) {
+// early: W is not written by anything still running on the stream (a model's weights): its first pieces are asked for before the
+// kernels ahead are done.
+IMP_API int imp_gemm_f32_ex(float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M,
+                            int N, int K, int early, void* stream) {
     if (M == 0 || N == 0) return 0;
     IMP_CHECK_ARG(C && A && W && M > 0 && N > 0 && K > 0, "imp_gemm_f32: bad argument");
     IMP_CHECK_ARG(ldc >= N && lda >= K && ldw >= K, "imp_gemm_f32: leading dimension too small");
@@ -393,21 +397,26 @@ IMP_API int imp_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, con
     const bool aligned = (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0 && lda % 4 == 0 && ldw % 4 == 0;
     cudaError_t e;
     if (M <= GF_ROWS_MAX) {
-        e = M == 1   ? gr_launch<1>(aligned, C, ldc, A, lda, W, ldw, M, N, K, s)
-            : M == 2 ? gr_launch<2>(aligned, C, ldc, A, lda, W, ldw, M, N, K, s)
-            : M <= 4 ? gr_launch<4>(aligned, C, ldc, A, lda, W, ldw, M, N, K, s)
-            : M <= 8 ? gr_launch<8>(aligned, C, ldc, A, lda, W, ldw, M, N, K, s)
-                     : gr_launch<16>(aligned, C, ldc, A, lda, W, ldw, M, N, K, s);
+        e = M == 1   ? gr_launch<1>(aligned, C, ldc, A, lda, W, ldw, M, N, K, early, s)
+            : M == 2 ? gr_launch<2>(aligned, C, ldc, A, lda, W, ldw, M, N, K, early, s)
+            : M <= 4 ? gr_launch<4>(aligned, C, ldc, A, lda, W, ldw, M, N, K, early, s)
+            : M <= 8 ? gr_launch<8>(aligned, C, ldc, A, lda, W, ldw, M, N, K, early, s)
+                     : gr_launch<16>(aligned, C, ldc, A, lda, W, ldw, M, N, K, early, s);
     } else {
         // two CTAs a tile where those fill the device's slots, else four (257 rows of 1,024 x 3,072: 77 us, with two 178)
         const int ctas = m_tiles * n_tiles * 2 >= 3 * imp_sm_count() ? 2 : 4;
         const dim3 grid((unsigned)(n_tiles * ctas), (unsigned)m_tiles);
-        e = aligned ? gf_launch(gemm_f32_tile_kernel<true>, grid, GT_THREADS, GT_SMEM, ctas, s, C, ldc, A, lda, W, ldw, M, N, K, ctas)
-                    : gf_launch(gemm_f32_tile_kernel<false>, grid, GT_THREADS, GT_SMEM, ctas, s, C, ldc, A, lda, W, ldw, M, N, K, ctas);
+        e = aligned ? gf_launch(gemm_f32_tile_kernel<true>, grid, GT_THREADS, GT_SMEM, ctas, s, C, ldc, A, lda, W, ldw, M, N, K, ctas, early)
+                    : gf_launch(gemm_f32_tile_kernel<false>, grid, GT_THREADS, GT_SMEM, ctas, s, C, ldc, A, lda, W, ldw, M, N, K, ctas, early);
     }
     if (e != cudaSuccess) {
         imp_set_error("imp_gemm_f32: %s", cudaGetErrorString(e));
         return (int)e;
     }
     IMP_RETURN_LAUNCH();
+}
+
+IMP_API int imp_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M,
+                         int N, int K, void* stream) {
+    return imp_gemm_f32_ex(C, ldc, A, lda, W, ldw, M, N, K, 0, stream);
 }

@@ -85,8 +85,8 @@ void embedding(Runtime& rt, Tensor out, const Tensor& table, const int32_t* ids,
 // ----------------------------------------------------------------------------- matrix products
 static void gemm_f32(Runtime& rt, Tensor out, const Tensor& a, const Tensor& w) {
     ++rt.launches;
-    check_launch(imp_gemm_f32((float*)out.data, out.stride0, (const float*)a.data, a.stride0, (const float*)w.data, w.stride0,
-                              (int)rows(a), (int)rows(w), (int)cols(a), rt.stream),
+    check_launch(imp_gemm_f32_ex((float*)out.data, out.stride0, (const float*)a.data, a.stride0, (const float*)w.data, w.stride0,
+                                 (int)rows(a), (int)rows(w), (int)cols(a), 1, rt.stream),
                  "gemm_f32");
 }
 

@@ -90,6 +90,8 @@ __global__ void __launch_bounds__(PN_BLOCK) proj_norm_kv_vec_kernel(
     const int n = is_k ? n_k : n_q;
     const float* b = is_k ? b_k : b_q;
     const float* w = is_k ? w_k : w_q;
+    pdl_wait();
+    pdl_launch_dependents();
     float wv[NV][PER], bv[NV][PER];
     auto load4 = [](float* dst, const float* src) {
         const float4 f = *reinterpret_cast<const float4*>(src);
@@ -109,8 +111,6 @@ __global__ void __launch_bounds__(PN_BLOCK) proj_norm_kv_vec_kernel(
             }
         }
     }
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float scratch[33];
     TA* row = qk + (int64_t)t * row_stride + (is_k ? n_q : 0);
     const int pos = positions[t];
