@@ -46,7 +46,12 @@ DeviceBuffer::DeviceBuffer(size_t bytes, bool zero) : n_(bytes) {
         fail(e == cudaErrorMemoryAllocation ? IMP_ERROR_OUT_OF_MEMORY : IMP_ERROR_CUDA,
              "cannot allocate " + std::to_string(bytes) + " bytes of device memory: " + cudaGetErrorString(e));
     }
-    if (zero) IMP_CUDA(cudaMemset(p_, 0, bytes));
+    if (zero) {
+        // The fill runs on the default stream, which the engine's own stream does not wait for, and the host does not wait for it
+        // either: a cache of 40 GB takes milliseconds, in which a first step would see its batch arrays and its new keys cleared.
+        IMP_CUDA(cudaMemset(p_, 0, bytes));
+        IMP_CUDA(cudaStreamSynchronize(nullptr));
+    }
 }
 DeviceBuffer::~DeviceBuffer() { reset(); }
 DeviceBuffer& DeviceBuffer::operator=(DeviceBuffer&& o) noexcept {

@@ -68,6 +68,30 @@ def test_long_decoding_and_first_tokens(dtype, model_folders):
         assert (err <= atol + rtol * ref[i].abs()).all(), f"position {i}: max error {err.max():.3g}"
 
 
+def test_first_step_behind_a_large_cache(tmp_path):
+    """36 GiB of cache (24 layers of 1.5 GiB) take milliseconds to clear. A first step right after the engine is made
+    must not see its batch arrays or its new keys cleared: same bits as with a small cache, for three engines."""
+    from conftest import TINY_A
+    from imp_b200 import StepEntry
+    from imp_b200.config.registry import config_from_dict
+    from imp_b200.weights.random_init import write_model_folder
+    folder = str(tmp_path)
+    write_model_folder(folder, config_from_dict(dict(TINY_A, num_hidden_layers=24)), seed=3, std=0.05)
+    per_token = 2 * TINY_A["num_key_value_heads"] * TINY_A["head_dim"] * 4
+    ids = prompts_for(TINY_A["vocab_size"], [40], seed=2)[0]
+
+    def first_steps(**kw):
+        eng = engine(folder, "float32", 256, **kw)
+        out = [np.array(eng.step_tokens([StepEntry("x", part, [len(part) - 1])])) for part in (ids[:39], ids[39:])]
+        eng.end("x")
+        return np.concatenate(out)
+
+    want = first_steps()
+    assert np.isfinite(want).all()
+    for _ in range(3):
+        assert np.array_equal(first_steps(kv_cache_tokens=(3 << 29) // per_token), want)
+
+
 def test_temperature_sampling_is_reproducible_and_independent_of_the_batch(model_folders):
     from imp_b200 import GenerateParams
     folder, cd, page = model_folders["B"]
