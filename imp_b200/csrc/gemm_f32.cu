@@ -87,6 +87,7 @@ template <int MT> constexpr int gr_smem_floats() {
 }
 
 // Grid (ctas x groups of 32 rows of W, groups of MT rows of A); a cluster along x of `ctas` = 1, 2 or 4.
+// early (see imp_early_weights): the first pieces of W are asked for before the kernels ahead are done.
 template <int MT, bool ALIGNED>
 __global__ void __launch_bounds__(GR_WARPS * 32) gemm_f32_rows_kernel(float* __restrict__ C, int64_t ldc, const float* __restrict__ A, int64_t lda,
                                                                       const float* __restrict__ W, int64_t ldw, int M, int N, int K, int ctas, int early) {
@@ -384,10 +385,8 @@ cudaError_t gr_launch(bool aligned, float* C, int64_t ldc, const float* A, int64
 
 }  // namespace
 
-// early: W is not written by anything still running on the stream (a model's weights): its first pieces are asked for before the
-// kernels ahead are done.
-IMP_API int imp_gemm_f32_ex(float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M,
-                            int N, int K, int early, void* stream) {
+IMP_API int imp_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M,
+                         int N, int K, void* stream) {
     if (M == 0 || N == 0) return 0;
     IMP_CHECK_ARG(C && A && W && M > 0 && N > 0 && K > 0, "imp_gemm_f32: bad argument");
     IMP_CHECK_ARG(ldc >= N && lda >= K && ldw >= K, "imp_gemm_f32: leading dimension too small");
@@ -395,6 +394,7 @@ IMP_API int imp_gemm_f32_ex(float* C, int64_t ldc, const float* A, int64_t lda, 
     IMP_CHECK_ARG(m_tiles <= 65535, "imp_gemm_f32: M %d too large for one launch", M);
     cudaStream_t s = (cudaStream_t)stream;
     const bool aligned = (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0 && lda % 4 == 0 && ldw % 4 == 0;
+    const int early = imp_early_weights();
     cudaError_t e;
     if (M <= GF_ROWS_MAX) {
         e = M == 1   ? gr_launch<1>(aligned, C, ldc, A, lda, W, ldw, M, N, K, early, s)
@@ -414,9 +414,4 @@ IMP_API int imp_gemm_f32_ex(float* C, int64_t ldc, const float* A, int64_t lda, 
         return (int)e;
     }
     IMP_RETURN_LAUNCH();
-}
-
-IMP_API int imp_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M,
-                         int N, int K, void* stream) {
-    return imp_gemm_f32_ex(C, ldc, A, lda, W, ldw, M, N, K, 0, stream);
 }

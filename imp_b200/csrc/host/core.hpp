@@ -190,6 +190,7 @@ struct Runtime {
     int32_t* status = nullptr;      // device status word
     Arena* arena = nullptr;
     int sm_count = 0;
+    bool early_weights = false;     // the matrices of its products are a model's weights, which no kernel of a step writes
     int64_t fallback_calls = 0;     // matrix products that ran on the plain fallback kernel
     int64_t launches = 0;           // launcher calls of this library
     int64_t split_norm_calls = 0;   // norms that added the unsummed parts of a product themselves

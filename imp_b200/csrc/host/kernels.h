@@ -69,8 +69,10 @@ int imp_gdr_scan_ex(const float* qn, const float* kn, const float* vc, const flo
 int imp_gdr_output(void* y, const float* o, const void* gate, int64_t gate_ld, const float* w, float eps, int n_tokens, int H, int Dv,
                    int act_dtype, void* stream);
 
-int imp_gemm_f32_ex(float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M, int N, int K,
-                 int early, void* stream);
+// Whether the products that this thread launches may ask for W before the kernels ahead on the stream are done; the value before.
+int imp_set_early_weights(int on);
+int imp_gemm_f32(float* C, int64_t ldc, const float* A, int64_t lda, const float* W, int64_t ldw, int M, int N, int K,
+                 void* stream);
 int imp_gemm_bf16_plain(void* C, int64_t ldc, int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, int M,
                         int N, int K, void* stream);
 int imp_gemm_bf16_small_m(void* C, int64_t ldc, int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw,

@@ -83,10 +83,17 @@ void embedding(Runtime& rt, Tensor out, const Tensor& table, const int32_t* ids,
 }
 
 // ----------------------------------------------------------------------------- matrix products
+// Lets this thread's products ask for W before the kernels ahead are done, where the runtime says what their W is.
+struct EarlyWeights {
+    const int before;
+    explicit EarlyWeights(const Runtime& rt) : before(imp_set_early_weights(rt.early_weights)) {}
+    ~EarlyWeights() { imp_set_early_weights(before); }
+};
+
 static void gemm_f32(Runtime& rt, Tensor out, const Tensor& a, const Tensor& w) {
     ++rt.launches;
-    check_launch(imp_gemm_f32_ex((float*)out.data, out.stride0, (const float*)a.data, a.stride0, (const float*)w.data, w.stride0,
-                                 (int)rows(a), (int)rows(w), (int)cols(a), 1, rt.stream),
+    check_launch(imp_gemm_f32((float*)out.data, out.stride0, (const float*)a.data, a.stride0, (const float*)w.data, w.stride0,
+                              (int)rows(a), (int)rows(w), (int)cols(a), rt.stream),
                  "gemm_f32");
 }
 
@@ -231,6 +238,7 @@ Branch linear(Runtime& rt, Tensor out, const Tensor& x, const Tensor& w, bool ma
     const int64_t M = M_of(x);
     need(cols(x) == cols(w) && rows(out) == M && cols(out) == rows(w), "linear: shapes do not agree");
     if (M == 0) return Branch::of(out);
+    const EarlyWeights early(rt);
     if (w.dtype == F32) {
         Tensor xf = x;
         if (x.dtype != F32) {
@@ -289,6 +297,7 @@ void linear_gated(Runtime& rt, Tensor out, const Tensor& x, const Tensor& w, Gat
     const int64_t M = M_of(x), F = cols(out);
     if (M == 0) return;
     need(act.kind >= 0 && act.kind <= 2, "linear_gated: unknown activation");
+    const EarlyWeights early(rt);
     const int epi = act.kind == 0 ? TC_OUT_SWIGLU : act.kind == 1 ? TC_OUT_GEGLU : TC_OUT_CLIPGLU;
     const bool bf16 = x.dtype == BF16 && w.dtype == BF16 && out.dtype == BF16;
     const bool lib = use_library_gemm();
@@ -315,6 +324,7 @@ void linear_relu2(Runtime& rt, Tensor out, const Tensor& x, const Tensor& w) {
     const int64_t M = M_of(x);
     if (M == 0) return;
     need(contiguous(out), "linear_relu2: the output must be dense");
+    const EarlyWeights early(rt);
     if (x.dtype == BF16 && w.dtype == BF16 && out.dtype == BF16 && !use_library_gemm() && M > stream_m_max()) {
         if (M <= TC_SWAP_MAX_M && gemm_tc_swap(rt, out, x, w, TC_OUT_RELU2)) return;
         if (M > TC_SWAP_MAX_M && gemm_tc(rt, out, x, w, TC_OUT_RELU2)) return;

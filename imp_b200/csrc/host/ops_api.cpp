@@ -18,7 +18,7 @@ Runtime runtime_for(void* stream, int32_t* status) {
     if (!g_arena) g_arena = std::make_unique<Arena>(0, (size_t)1 << 22);
     // scratch of one call stays valid during the next one (unsummed parts travel from a product to a norm)
     g_arena->next_layer();
-    Runtime rt;
+    Runtime rt;         // early_weights stays off: a kernel still running may be writing the caller's matrix
     rt.stream = (cudaStream_t)stream;
     rt.status = status;
     rt.arena = g_arena.get();

@@ -23,6 +23,14 @@ int imp_pdl_enabled() {
     return enabled;
 }
 
+static thread_local int g_early_weights = 0;
+extern "C" int imp_set_early_weights(int on) {
+    const int before = g_early_weights;
+    g_early_weights = on ? 1 : 0;
+    return before;
+}
+int imp_early_weights() { return g_early_weights; }
+
 IMP_API int imp_abi_version(void) { return 1; }
 
 // Compute capability of the current device as major*10+minor, or a negative CUDA error.

@@ -176,6 +176,27 @@ def test_gemm_f32_edges(K, M, N, K_):
     assert torch.equal(K.gemm_f32(torch.empty(M, N, device=DEV), wide[:, 3:3 + K_], w), out)
 
 
+# A product may ask for a model's weights before the kernels ahead are done; a caller's matrix may still be being written by one of
+# them.  Here a cast writes all of W (25 million values, tens of microseconds) right in front of the product.
+@pytest.mark.parametrize("M", [1, 8, 20, 100, 300])
+@pytest.mark.parametrize("op", ["linear", "linear_swiglu", "linear_clipped", "linear_relu2", "gemm_f32"])
+def test_products_wait_for_a_matrix_that_is_being_written(K, M, op):
+    N, Kd = 6144, 4096
+    x, src = rnd(M, Kd, seed=61).to(DEV), rnd(N, Kd, seed=62, scale=0.02).to(torch.bfloat16).to(DEV)
+    run = {"linear": K.linear, "linear_swiglu": K.linear_swiglu, "linear_relu2": K.linear_relu2, "gemm_f32": K.gemm_f32,
+           "linear_clipped": lambda o, a, w: K.linear_gated(o, a, w, "clipped", 1.5)}[op]
+    out = torch.empty(M, N // 2 if op in ("linear_swiglu", "linear_clipped") else N, device=DEV)
+    w = K.cast(torch.empty(N, Kd, device=DEV), src)
+    torch.cuda.synchronize()
+    want = run(out, x, w).clone()
+    for _ in range(3):
+        w.fill_(float("nan"))
+        torch.cuda.synchronize()
+        K.cast(w, src)
+        run(out, x, w)
+        assert torch.equal(out, want)
+
+
 # Routed rows on the tensor-memory products.  The average number of rows a group decides the kernel (tiles of 32, 64 and 128 of the
 # list's rows beside streamed weights; pairs of CTAs), so every kernel meets groups without rows, with one, with a whole tile, one more,
 # and many tiles; a list shorter than its buffer; matrices that are no multiple of a tile; every epilogue.
