@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
         ++q_issue;
         if (++i_stage == n_stages) { i_stage = 0; i_tile += gridDim.x; }
     };
-    // The weights of the first steps do not depend on the kernel before this one: request them, then
+    // The weights of the first steps do not depend on the kernel before this one (see imp_launch_product): request them, then
     // wait for it, then request the activations of the same steps.
     {
         const int q0 = q_issue, t0 = i_tile, s0 = i_stage;
@@ -219,7 +219,7 @@ static cudaError_t launch_stream_st(TO* C, int64_t ldc, const __nv_bfloat16* A, 
     // One tile per CTA measured faster than two persistent CTAs per SM on every shape of the 8B model
     // (the kernel itself takes any grid size: a CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...).
     const int grid = n_tiles;
-    return imp_launch(gemm_stream_kernel<NT, TO, SWIGLU, STAGES, RG>, dim3(grid), dim3(GS_WARPS * 32 * RG), gs_smem_bytes(NT, STAGES, RG), s, C, ldc,
+    return imp_launch_product(gemm_stream_kernel<NT, TO, SWIGLU, STAGES, RG>, dim3(grid), dim3(GS_WARPS * 32 * RG), gs_smem_bytes(NT, STAGES, RG), s, C, ldc,
                       A, lda, W, ldw, M, N, K, gate_act);
 }
 

@@ -989,7 +989,7 @@ __global__ void __launch_bounds__(128, 1) gemm_tc_swap_kernel(const __grid_const
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + TCS_STAGES), accum_bar = smem_u32(bars + 2 * TCS_STAGES);
 
     // Nothing before pdl_wait() reads or writes what an earlier kernel of the stream may still be
-    // working on: barriers, tensor memory and the weight tiles of the first stages only.
+    // working on: barriers, tensor memory and the weight tiles of the first stages only (see imp_launch_product).
     if (threadIdx.x == 0) {
         for (int s = 0; s < TCS_STAGES; ++s) {
             mbar_init(full0 + 8 * s, 1);
@@ -1411,7 +1411,7 @@ static int launch_tcs(void* C, int64_t ldc, int64_t split_stride, const CUtensor
         attr_set = true;
     }
     dim3 grid((N + tile_rows - 1) / tile_rows, 1, splits);
-    cudaError_t e = imp_launch(gemm_tc_swap_kernel<BN, EPI, WROWS>, grid, dim3(128), (size_t)tcs_rows_smem_bytes<BN, WROWS>(), s, mw, mx,
+    cudaError_t e = imp_launch_product(gemm_tc_swap_kernel<BN, EPI, WROWS>, grid, dim3(128), (size_t)tcs_rows_smem_bytes<BN, WROWS>(), s, mw, mx,
                                C, ldc, split_stride, M, N, K, kb_per_split, tile_rows, status, g_tcs_wait_limit, g_tcs_skip_kb, gate_act, TcGroups{});
     if (e != cudaSuccess) { imp_set_error("gemm_tc_swap: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;

@@ -179,16 +179,20 @@ def test_gemm_f32_edges(K, M, N, K_):
 # A product may ask for a model's weights before the kernels ahead are done; a caller's matrix may still be being written by one of
 # them.  Here a cast writes all of W (25 million values, tens of microseconds) right in front of the product.
 @pytest.mark.parametrize("M", [1, 8, 20, 100, 300])
-@pytest.mark.parametrize("op", ["linear", "linear_swiglu", "linear_clipped", "linear_relu2", "gemm_f32"])
-def test_products_wait_for_a_matrix_that_is_being_written(K, M, op):
+@pytest.mark.parametrize("op", ["linear", "linear_swiglu", "linear_clipped", "linear_relu2", "gemm_f32", "gemm_bf16_stream", "gemm_bf16_tc_swap", "gemm_bf16_tc"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_products_wait_for_a_matrix_that_is_being_written(K, M, op, dtype):
+    if ("f32" in op) != (dtype == torch.float32) and op.startswith("gemm") or (op.endswith("stream") and M > 16) or (op.endswith("swap") and M > 128):
+        pytest.skip("not a size or type of this product")
     N, Kd = 6144, 4096
-    x, src = rnd(M, Kd, seed=61).to(DEV), rnd(N, Kd, seed=62, scale=0.02).to(torch.bfloat16).to(DEV)
-    run = {"linear": K.linear, "linear_swiglu": K.linear_swiglu, "linear_relu2": K.linear_relu2, "gemm_f32": K.gemm_f32,
-           "linear_clipped": lambda o, a, w: K.linear_gated(o, a, w, "clipped", 1.5)}[op]
-    out = torch.empty(M, N // 2 if op in ("linear_swiglu", "linear_clipped") else N, device=DEV)
-    w = K.cast(torch.empty(N, Kd, device=DEV), src)
+    x, src = rnd(M, Kd, seed=61).to(dtype).to(DEV), rnd(N, Kd, seed=62, scale=0.02).to(torch.bfloat16).to(DEV)
+    src = src.float() if dtype == torch.bfloat16 else src        # a cast that changes the type
+    run = lambda o, a, w: K.linear_gated(o, a, w, "clipped", 1.5) if op == "linear_clipped" else getattr(K, op)(o, a, w)  # noqa: E731
+    out = torch.empty(M, N // 2 if op in ("linear_swiglu", "linear_clipped") else N, dtype=dtype, device=DEV)
+    w = K.cast(torch.empty(N, Kd, dtype=dtype, device=DEV), src)
     torch.cuda.synchronize()
-    want = run(out, x, w).clone()
+    run(out, x, w)
+    want = out.clone()
     for _ in range(3):
         w.fill_(float("nan"))
         torch.cuda.synchronize()
