@@ -189,29 +189,24 @@ void set_variant_resolver(VariantResolver fn) {
     g_resolver = fn;
 }
 
-// All sequences in tiles of 32 tokens; those with 64 tokens and more in tiles of 128; the others in tiles of 32; the
+// All sequences in tiles of 32 tokens; those with 64 tokens and more in tiles of 128; the others in tiles of 32; and the
 // first and the third again without the sequences that bring a single token (those go to the decode kernel when they
-// stand at the head of a mixed batch); and all but those in tiles of 128.
+// stand at the head of a mixed batch).
+//
+// Deep portions (2 ... 63 tokens behind many keys) go to the tensor-memory kernel too: the 32-token kernel's CTA, one a tile
+// and group of heads, walks all their keys alone (16 tokens behind 1,984 of an 8B model: 150 us a layer; the other kernel's tile
+// walks 128 keys in about 1.2 us behind about 12 us of start and end: 30).  From about 256 keys on it is the faster one; up to
+// DEEP_KEYS the portions keep the kernel, and the rounding, of a short prompt.  A portion's length and place alone
+// decide, not what else is in the step.
 std::vector<TilingSpec> attention_tilings() {
-    return {TilingSpec{TILE, 0, 0}, TilingSpec{WIDE_TILE, WIDE_MIN, 0}, TilingSpec{TILE, 0, WIDE_MIN},
-            TilingSpec{TILE, 2, 0}, TilingSpec{TILE, 2, WIDE_MIN}, TilingSpec{WIDE_TILE, 2, 0}};
+    return {TilingSpec{TILE, 0, 0, 0}, TilingSpec{WIDE_TILE, WIDE_MIN, 0, WIDE_MIN}, TilingSpec{TILE, 0, WIDE_MIN, WIDE_MIN},
+            TilingSpec{TILE, 2, 0, 0}, TilingSpec{TILE, 2, WIDE_MIN, WIDE_MIN}};
 }
 
-// Whether the tensor-memory kernel takes all portions of a step, the short ones too: where a short portion stands behind many
-// keys, which the 32-token kernel's CTA, one a tile and group of heads, then walks alone (16 tokens behind 1,984 of an 8B
-// model: 150 us a layer; the other kernel's tile walks 128 keys in about 1.2 us behind about 12 us of start and end: 30).  From about 256
-// keys on it is the faster one; behind up to 1,024 the short portions keep the kernel, and the rounding, of a short prompt.
-constexpr int DEEP_KEYS = 1024;
-static bool wide_for_all(const Step& st, const AttentionGeometry& g, bool singles) {
-    bool deep = false;
-    for (int i = 0; i < st.B(); ++i) {
-        const int n = st.q_lens[(size_t)i];
-        if (n == 1 && !singles) return false;      // single tokens without the decode kernel: tiles of one row of the other kernel
-        const int behind = g.window != 0 ? std::min(st.starts[(size_t)i], std::abs(g.window)) : st.starts[(size_t)i];
-        deep = deep || (n > 1 && n < WIDE_MIN && behind + n > DEEP_KEYS);
-    }
-    return deep;
-}
+// A mixer whose window or chunk holds fewer keys than that has no deep portions.
+static bool takes_deep(const AttentionGeometry& g) { return g.window == 0 || std::abs(g.window) >= DEEP_KEYS; }
+static int wide_tiles(const Tiles& t, const AttentionGeometry& g) { return takes_deep(g) ? t.count : t.shallow; }
+static int short_tiles(const Tiles& t, const AttentionGeometry& g) { return takes_deep(g) ? t.shallow : t.count; }
 
 // The bulk-copy kernel (page sizes that are multiples of 16) keeps two CTAs resident per SM: with fewer
 // (token, kv head) pairs than such slots the keys are split until the slots are full.  With more, the
@@ -306,13 +301,13 @@ bool decode_attention_fused(Step& st, Tensor out, const Tensor& qkv, const Atten
 }
 
 static void prefill_attention(Step& st, Tensor out, const Tensor& q, const AttentionGeometry& g, const LayerCache& cache,
-                              const Tiles& tiles) {
+                              const Tiles& tiles, int n_tiles) {
     Runtime& rt = *st.rt;
     MmaVariant& lib = mma_variant(g.dh);
     const ImpCacheView& c = cache.view;
     check_variant(rt,
                   lib.prefill(out.data, out.stride0, q.data, q.stride0, c.k_pages, c.v_pages, c.block_table, c.bt_stride,
-                              st.view.seq_of_token, st.view.positions, tiles.tok0, tiles.rows, tiles.count, st.B(), g.hq, g.hkv,
+                              st.view.seq_of_token, st.view.positions, tiles.tok0, tiles.rows, n_tiles, st.B(), g.hq, g.hkv,
                               c.page_size, c.num_pages, g.scale, g.window, rt.status, rt.stream),
                   "attention prefill", lib.last_error);
 }
@@ -337,7 +332,7 @@ static bool bias_attention_mma(Step& st, Tensor out, const Tensor& q, const Atte
     if (generic_only || rt.is_f32() || q.dtype != BF16 || g.dh % 16 || g.dh > 256) return false;
     if ((ex.bias && !ex.bias_l2) || (ex.sink && !ex.sink_l2)) return false;
     if (q.stride0 % 8 || out.stride0 % 2 || (uintptr_t)q.data % 16 || (uintptr_t)c.k_pages % 16 || (uintptr_t)c.v_pages % 16) return false;
-    if (!st.decode_only() && tiling_ids.size() != 6) return false;
+    if (!st.decode_only() && tiling_ids.size() != 5) return false;
     MmaVariant& lib = mma_variant(g.dh);
     auto decode = [&](Tensor o, const Tensor& qq) {
         const int T = (int)rows(qq), G = g.hq / g.hkv;
@@ -366,27 +361,27 @@ static bool bias_attention_mma(Step& st, Tensor out, const Tensor& q, const Atte
     for (int i = n_single; singles && i < st.B(); ++i)
         if (st.q_lens[(size_t)i] == 1) singles = false;
     if (singles) decode(first_rows(out, n_single), first_rows(q, n_single));
-    // portions of 64 tokens and more on the tensor-memory kernel in tiles of 128, where it takes the geometry and the
-    // caller has the table in that kernel's padded layout
-    const bool all_wide = wide_for_all(st, g, singles);
-    const Tiles& wide = st.tiles.at((size_t)tiling_ids[all_wide ? 5 : 1]);
-    const bool tc = wide.count && prefill_tc_supported(q, out, g, c) &&
+    // portions of 64 tokens and more, and deep ones, on the tensor-memory kernel in tiles of 128, where it takes the geometry
+    // and the caller has the table in that kernel's padded layout
+    const Tiles& wide = st.tiles.at((size_t)tiling_ids[1]);
+    const int n_wide = wide_tiles(wide, g);
+    const bool tc = n_wide && prefill_tc_supported(q, out, g, c) &&
                     (!ex.bias || (ex.bias_pad_l2 && tc_variant(g.dh).bias_pad() == ex.pad));   // a sink alone needs no table
     if (tc) {
         TcVariant& tlib = tc_variant(g.dh);
         check_variant(rt,
                       tlib.prefill_bias(out.data, out.stride0, q.data, q.stride0, (int)rows(q), c.k_pages, c.v_pages, c.block_table,
-                                        c.bt_stride, st.view.seq_of_token, st.view.positions, wide.tok0, wide.rows, wide.count, st.B(),
+                                        c.bt_stride, st.view.seq_of_token, st.view.positions, wide.tok0, wide.rows, n_wide, st.B(),
                                         g.hq, g.hkv, c.page_size, c.num_pages, g.scale, g.window, ex.bias_pad_l2, ex.n_dist, ex.sink_l2,
                                         rt.status, rt.stream),
                       "attention prefill (tcgen05, bias, sink)", tlib.last_error);
-        if (all_wide) return true;
     }
     const Tiles& tiles = st.tiles.at((size_t)tiling_ids[tc ? (singles ? 4 : 2) : (singles ? 3 : 0)]);
-    if (tiles.count)
+    const int n_tiles = tc ? short_tiles(tiles, g) : tiles.count;
+    if (n_tiles)
         check_variant(rt,
                       lib.prefill_bias(out.data, out.stride0, q.data, q.stride0, c.k_pages, c.v_pages, c.block_table, c.bt_stride,
-                                       st.view.seq_of_token, st.view.positions, tiles.tok0, tiles.rows, tiles.count, st.B(), g.hq, g.hkv,
+                                       st.view.seq_of_token, st.view.positions, tiles.tok0, tiles.rows, n_tiles, st.B(), g.hq, g.hkv,
                                        c.page_size, c.num_pages, g.scale, g.window, ex.bias_l2, ex.n_dist, ex.sink_l2, rt.status,
                                        rt.stream),
                       "attention prefill (bias, sink)", lib.last_error);
@@ -423,7 +418,7 @@ void paged_attention(Step& st, Tensor out, const Tensor& q, const AttentionGeome
         decode_attention(st, out, q, g, cache);
         return;
     }
-    need(tiling_ids.size() == 6, "attention: the step holds no tilings for this mixer");
+    need(tiling_ids.size() == 5, "attention: the step holds no tilings for this mixer");
     // Sequences that decode beside the portions of prompts: as a tile of one row each, a CTA walks all their keys alone
     // (8 decoding sequences at context 4,096 beside a 512-token portion: 19.2 ms a step against 4.0 + 9.1 for the two
     // alone).  The scheduler puts them first, one token each, so they are the batch's first rows: the split-key decode
@@ -436,20 +431,20 @@ void paged_attention(Step& st, Tensor out, const Tensor& q, const AttentionGeome
         if (st.q_lens[(size_t)i] == 1) singles = false;      // single tokens further on: no leading block, the tiled kernels take all
     if (singles) decode_attention(st, first_rows(out, n_single), first_rows(q, n_single), g, cache);
     const Tiles& all = st.tiles.at((size_t)tiling_ids[singles ? 3 : 0]);
-    const bool all_wide = wide_for_all(st, g, singles);
-    const Tiles& wide = st.tiles.at((size_t)tiling_ids[all_wide ? 5 : 1]);
+    const Tiles& wide = st.tiles.at((size_t)tiling_ids[1]);
     const Tiles& rest = st.tiles.at((size_t)tiling_ids[singles ? 4 : 2]);
-    if (wide.count && prefill_tc_supported(q, out, g, c)) {
+    const int n_wide = wide_tiles(wide, g), n_rest = short_tiles(rest, g);
+    if (n_wide && prefill_tc_supported(q, out, g, c)) {
         TcVariant& lib = tc_variant(g.dh);
         check_variant(rt,
                       lib.prefill(out.data, out.stride0, q.data, q.stride0, (int)rows(q), c.k_pages, c.v_pages, c.block_table,
-                                  c.bt_stride, st.view.seq_of_token, st.view.positions, wide.tok0, wide.rows, wide.count, st.B(),
+                                  c.bt_stride, st.view.seq_of_token, st.view.positions, wide.tok0, wide.rows, n_wide, st.B(),
                                   g.hq, g.hkv, c.page_size, c.num_pages, g.scale, g.window, rt.status, rt.stream),
                       "attention prefill (tcgen05)", lib.last_error);
-        if (rest.count && !all_wide) prefill_attention(st, out, q, g, cache, rest);
+        if (n_rest) prefill_attention(st, out, q, g, cache, rest, n_rest);
         return;
     }
-    if (all.count) prefill_attention(st, out, q, g, cache, all);
+    if (all.count) prefill_attention(st, out, q, g, cache, all, all.count);
 }
 
 bool linear_qkv_rope(Step& st, Tensor q_out, const Tensor& x, const Tensor& w, const AttentionGeometry& g, const LayerCache& cache,

@@ -92,14 +92,16 @@ struct QkNorm {
     float eps = 1e-6f;
 };
 
-// The tilings the attention kernels want of a step (see TilingSpec): every portion in 32-token
-// tiles; portions of 64 tokens and more in 128-token tiles; the shorter ones in 32-token tiles.
+// The tilings the attention kernels want of a step (see TilingSpec): every portion in 32-token tiles; portions of 64 tokens and
+// more in 128-token tiles, behind them the deep ones; the shorter ones in 32-token tiles, the deep ones last; the first and
+// the third again without single tokens.
 std::vector<TilingSpec> attention_tilings();
 
-// out[t] = softmax(scale q[t] K^T) V over the cached positions token t may see.  float32: the plain
-// kernel (fixed reduction order per token).  bfloat16: the split-key decode kernel when every sequence
-// brings one token, else the tiled prefill kernels (tensor-memory kernel for long portions where the
-// head and page sizes allow it).  `tiling_ids`: where Step::tiles holds the three tilings above.
+// out[t] = softmax(scale q[t] K^T) V over the cached positions token t may see.  float32: the float32
+// kernel, or the plain one where that declines (both with a fixed reduction order per token).  bfloat16: the split-key decode
+// kernel for the sequences that bring one token in a decode step or at the head of a batch, the tiled prefill kernels for the rest
+// (tensor-memory kernel for long and deep portions where the head and page sizes allow it).  `tiling_ids`: where Step::tiles
+// holds the tilings above.
 // `extras`: a score bias by distance, bias [hq, n_dist] (score of key j for a query at p += bias[h][min(p - j,
 // n_dist - 1)]), and a sink per query head (exp(sink[h]) joins the softmax denominator); either may be null.
 struct AttentionExtras {

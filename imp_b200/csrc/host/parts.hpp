@@ -73,15 +73,19 @@ inline int first_visible(int pos, int window) {
 
 // How a mixer wants the new tokens of each sequence cut: runs of up to `tile` consecutive tokens
 // of one sequence, over the sequences whose portion holds min_len <= n < max_len tokens
-// (max_len == 0: no upper bound).  The step function fills what the model's mixers declared.
+// (max_len == 0: no upper bound).  The deep portions, 2 <= n < deep_below tokens that end behind more than DEEP_KEYS
+// keys, stand last in the list, also where they are shorter than min_len: a mixer may take the list with them or without.
+// The step function fills what the model's mixers declared.
+constexpr int DEEP_KEYS = 1024;
 struct TilingSpec {
-    int tile = 32, min_len = 0, max_len = 0;
-    bool operator==(const TilingSpec& o) const { return tile == o.tile && min_len == o.min_len && max_len == o.max_len; }
+    int tile = 32, min_len = 0, max_len = 0, deep_below = 0;
+    bool operator==(const TilingSpec& o) const { return tile == o.tile && min_len == o.min_len && max_len == o.max_len && deep_below == o.deep_below; }
 };
 struct Tiles {
     const int32_t* tok0 = nullptr;   // device: first token of each tile (index into the batch)
     const int32_t* rows = nullptr;   // device: tokens in each tile
-    int count = 0;
+    int count = 0;                   // all of them
+    int shallow = 0;                 // those of other than deep portions
 };
 
 // What a norm may do to the rows it has just normalised, in the same kernel, when whoever arranges it asks (Step::row_op): in a

@@ -191,25 +191,28 @@ Step& Stepper::prepare(const StepEntryView* entries, int B) {
             std::fill(row + width, row + buf_.max_pages, -1);
         }
     }
-    std::vector<int> tile_counts(tilings_.size(), 0);
+    std::vector<std::pair<int, int>> tile_counts(tilings_.size());   // without the deep portions' tiles, and with them
     if (!decode_only) {
         // Each declared tiling: runs of up to `tile` consecutive tokens of every sequence whose portion length
-        // lies in [min_len, max_len).
+        // lies in [min_len, max_len), and behind them the deep portions'.
         for (size_t k = 0; k < tilings_.size(); ++k) {
             const TilingSpec& ts = tilings_[k];
             int32_t* tok0 = host + buf_.off_tile0[k];
             int32_t* tn = host + buf_.off_tilen[k];
             int c = 0;
-            for (int s = 0; s < B; ++s) {
-                const int n = st.q_lens[(size_t)s];
-                if (n < ts.min_len || (ts.max_len > 0 && n >= ts.max_len)) continue;
-                for (int a = 0; a < n; a += ts.tile) {
-                    tok0[c] = q_start[s] + a;
-                    tn[c] = std::min(ts.tile, n - a);
-                    ++c;
+            for (const bool want_deep : {false, true}) {
+                for (int s = 0; s < B; ++s) {
+                    const int n = st.q_lens[(size_t)s];
+                    const bool deep = n >= 2 && n < ts.deep_below && st.starts[(size_t)s] + n > DEEP_KEYS;
+                    if (deep != want_deep || (!deep && (n < ts.min_len || (ts.max_len > 0 && n >= ts.max_len)))) continue;
+                    for (int a = 0; a < n; a += ts.tile) {
+                        tok0[c] = q_start[s] + a;
+                        tn[c] = std::min(ts.tile, n - a);
+                        ++c;
+                    }
                 }
+                (want_deep ? tile_counts[k].second : tile_counts[k].first) = c;
             }
-            tile_counts[k] = c;
         }
     }
     buf_.upload(which, B, rt_->stream);
@@ -243,7 +246,7 @@ Step& Stepper::prepare(const StepEntryView* entries, int B) {
     st.bt_stride = buf_.max_pages;
     st.tiles.assign(tilings_.size(), Tiles());
     for (size_t k = 0; k < tilings_.size(); ++k)
-        st.tiles[k] = Tiles{d + buf_.off_tile0[k], d + buf_.off_tilen[k], tile_counts[k]};
+        st.tiles[k] = Tiles{d + buf_.off_tile0[k], d + buf_.off_tilen[k], tile_counts[k].second, tile_counts[k].first};
     return st;
 }
 

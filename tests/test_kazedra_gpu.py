@@ -214,6 +214,45 @@ def test_long_prompt_on_wide_heads():
     close(out, want[1100:], dtype, "portion")
 
 
+@pytest.mark.parametrize("n", [2, 16, 63])
+def test_short_portions_behind_many_keys(n):
+    """Bias and sink in a portion of 2 to 63 tokens at the line of 1,024 keys from which it goes to the tensor-memory kernel:
+    alone, behind a leading single token, beside a fresh short prompt and a portion of 64 and more."""
+    c = {"heads": 4, "kv_heads": 2, "dim": 128, "vdim": 128, "bias_max": 300, "scale": 1.3 / math.sqrt(128), "q_temp": {"coef": 0.4, "every": 64}}
+    dtype = torch.bfloat16
+    bench = PartBench("bfloat16", [PagedKVSpec(2, 128, 0)], page_size=16, num_pages=400, slots=8, max_tokens=2304, max_seq_len=2304)
+    w = {k: v.to(dtype) for k, v in left_weights(128, c, 16, seed=400, strong=2.0).items()}
+    params = {"hidden_size": 128, "num_heads": 4, "num_kv_heads": 2, "head_dim": 128, "scale": c["scale"], "norm_eps": 2e-5,
+              "q_temp_coef": 0.4, "q_temp_every": 64, "bias_max_distance": 300}
+    part = bench.build("mixer", PartSpec("sink_bias_attention", params), {LEFT_NAMES[k]: v.to(DEV) for k, v in w.items()})
+    W = {"m." + k: v.double() for k, v in w.items()}
+    x = rnd(2304, 128, seed=401).to(dtype)
+    want = K.sink_bias_attention(x.double(), W, "m.", c, 2e-5)
+
+    def run(pieces):
+        ctx = bench.prepare([(r, [1] * m, []) for r, _, m in pieces])
+        out = run_mixer(bench, part, torch.cat([x[a:a + m] for _, a, m in pieces]), ctx, bench.cache_view(0))
+        bench.commit()
+        at = 0
+        for r, a, m in pieces:
+            close(out[at:at + m], want[a:a + m], dtype, f"{r} from {a}")
+            at += m
+
+    for behind in (1024 - n, 1025 - n, 2000):
+        for beside in ("alone", "single", "all"):
+            run([("deep", 0, behind)])
+            run([("long", 0, 50)])
+            run([("one", 0, 33)])
+            step = [("deep", behind, n)]
+            if beside != "alone":
+                step = [("one", 33, 1)] + step
+            if beside == "all":
+                step += [("fresh", 0, 40), ("long", 50, 70)]
+            run(step)
+            for r in {"deep", "long", "one"} | {r for r, _, _ in step}:
+                bench.end(r)
+
+
 # ----------------------------------------------------- the recurrent mixer alone
 RIGHT_CASES = [
     dict(heads=6, kv_heads=3, dim=20, vdim=12, conv=3, d=72),

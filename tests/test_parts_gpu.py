@@ -260,3 +260,75 @@ def test_prenorm_block_hands_the_second_sum_on(dtype):
                      wf["down_proj"].float())
     close(h, hp, dtype)
     close(pending, f, dtype)
+
+
+# Portions of 2 to 63 tokens behind more than 1,024 keys go to the tensor-memory kernel, whatever else is in the step; the others
+# of that length stay with the 32-token tiles.  Around that line: alone, behind leading single tokens, beside a fresh short prompt
+# and a portion of 64 and more.  (window 300: no deep portions; 1,500: windows in the tensor-memory kernel.)
+@pytest.mark.parametrize("window", [0, 300, 1500])
+@pytest.mark.parametrize("n", [2, 16, 63])
+def test_short_portions_behind_many_keys(window, n):
+    Hq, Hkv, Dh, d, dtype = 4, 2, 128, 96, torch.bfloat16
+    bench = PartBench("bfloat16", [PagedKVSpec(Hkv, Dh, 0)], page_size=16, num_pages=1200, slots=8, max_tokens=2304, max_seq_len=2304)
+    params = {"hidden_size": d, "num_heads": Hq, "num_kv_heads": Hkv, "head_dim": Dh, "window": window, "qk_norm": False,
+              "position": {"kind": "rotary", "params": {"head_dim": Dh, "theta": 1e4, "max_positions": 4096}}}
+    w = {"q_proj": rnd(Hq * Dh, d, seed=10, scale=0.15), "k_proj": rnd(Hkv * Dh, d, seed=11, scale=0.15),
+         "v_proj": rnd(Hkv * Dh, d, seed=12, scale=0.2), "o_proj": rnd(d, Hq * Dh, seed=13, scale=0.2)}
+    w = {k: v.to(dtype) for k, v in w.items()}
+    part = bench.build("mixer", PartSpec("gqa_attention", params), {k: v.to(DEV) for k, v in w.items()})
+    w = {k: v.double() for k, v in w.items()}
+    x = rnd(2304, d, seed=30).to(dtype)
+    want = plain_attention_part(x.double(), w, Hq, Hkv, Dh, window, qk_norm=False)
+
+    def run(pieces):    # (request, first token, tokens): the output rows of one step
+        ctx = bench.prepare([(r, [1] * m, []) for r, _, m in pieces])
+        out = run_mixer(bench, part, torch.cat([x[a:a + m] for _, a, m in pieces]), ctx, bench.cache_view(0))
+        bench.commit()
+        at = 0
+        for r, a, m in pieces:
+            close(out[at:at + m], want[a:a + m], dtype)
+            at += m
+        return out
+
+    for behind in (1023 - n, 1024 - n, 1025 - n, 1024, 2000):
+        for beside in ("alone", "singles", "all", "single last"):
+            run([("deep", 0, behind)])
+            run([("long", 0, 50)])
+            run([("one", 0, 33)])
+            step = [("deep", behind, n)]
+            if beside in ("singles", "all"):
+                step = [("one", 33, 1)] + step
+            if beside == "all":
+                step += [("fresh", 0, 40), ("long", 50, 70)]
+            if beside == "single last":
+                step += [("fresh", 0, 40), ("one", 33, 1)]
+            run(step)
+            for r in {"deep", "long", "one"} | {r for r, _, _ in step}:
+                bench.end(r)
+
+
+@pytest.mark.parametrize("position", [0, 1])
+def test_a_short_prompt_does_not_depend_on_a_deep_portion_beside_it(position):
+    """The same fresh prompt beside 16 tokens behind 100 keys and beside 16 behind 2,000: the same bits."""
+    Hq, Hkv, Dh, d, dtype = 4, 2, 128, 96, torch.bfloat16
+    bench = PartBench("bfloat16", [PagedKVSpec(Hkv, Dh, 0)], page_size=16, num_pages=400, slots=4, max_tokens=2304, max_seq_len=2304)
+    params = {"hidden_size": d, "num_heads": Hq, "num_kv_heads": Hkv, "head_dim": Dh, "window": 0, "qk_norm": False,
+              "position": {"kind": "rotary", "params": {"head_dim": Dh, "theta": 1e4, "max_positions": 4096}}}
+    w = {"q_proj": rnd(Hq * Dh, d, seed=10, scale=0.15), "k_proj": rnd(Hkv * Dh, d, seed=11, scale=0.15),
+         "v_proj": rnd(Hkv * Dh, d, seed=12, scale=0.2), "o_proj": rnd(d, Hq * Dh, seed=13, scale=0.2)}
+    part = bench.build("mixer", PartSpec("gqa_attention", params), {k: v.to(dtype).to(DEV) for k, v in w.items()})
+    x = rnd(2304, d, seed=30).to(dtype)
+    got = []
+    for behind in (100, 2000):
+        run_mixer(bench, part, x[:behind], bench.prepare([("a", [1] * behind, [])]), bench.cache_view(0))
+        bench.commit()
+        pieces = [("a", x[behind:behind + 16]), ("fresh", x[500:540])]
+        if position:
+            pieces.reverse()
+        ctx = bench.prepare([(r, [1] * len(p), []) for r, p in pieces])
+        out = run_mixer(bench, part, torch.cat([p for _, p in pieces]), ctx, bench.cache_view(0))
+        bench.commit()
+        got.append(out[:40] if position else out[16:])
+        bench.end("a")
+        bench.end("fresh")
+    assert torch.equal(got[0], got[1])
