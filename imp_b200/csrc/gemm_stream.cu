@@ -181,8 +181,13 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
                     gate += gate_act.bias[n0 + (l >> 2)];
                     up += gate_act.bias[n0 + (l >> 2) + 8];
                 }
-                if (n0 + (l >> 2) + 8 < N && tok < M)
-                    C[(int64_t)tok * ldc + col] = from_float<TO>(sizeof(TO) == 2 ? gated_fast_f(gate, up, gate_act) : gated_f(gate, up, gate_act));
+                if (n0 + (l >> 2) + 8 < N && tok < M) {
+                    const float g1[1] = {gate}, u1[1] = {up};
+                    float o1[1];
+                    if (sizeof(TO) == 2) gated_many(o1, g1, u1, gate_act);
+                    else o1[0] = gated_f(gate, up, gate_act);
+                    C[(int64_t)tok * ldc + col] = from_float<TO>(o1[0]);
+                }
             }
         } else {
             // 16 rows x 8*NT tokens = NT*128 sums; thread i takes register slot i / 32 of lane i % 32.

@@ -74,6 +74,14 @@ template <int EPI> __device__ __forceinline__ void plain_act(float (&v)[32], con
     }
 }
 
+// Columns 16j..16j+7 of 32 are gate, 16j+8..16j+15 the matching up.
+__device__ __forceinline__ void tc_gate_up(const float (&v)[32], float (&gate)[16], float (&up)[16]) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) gate[8 * j + i] = v[16 * j + i], up[8 * j + i] = v[16 * j + 8 + i];
+}
+
 // Store 32 consecutive accumulator columns of one row (converted as the epilogue asks).
 template <int EPI>
 __device__ __forceinline__ void tc_store32(void* __restrict__ Cv, int64_t ldc, int row, int col0, int M, int N,
@@ -106,16 +114,14 @@ __device__ __forceinline__ void tc_store32(void* __restrict__ Cv, int64_t ldc, i
             for (int i = 0; i < 32 && col0 + i < N; ++i) dst[i] = __float2bfloat16_rn(v[i]);
         }
     } else {
-        // columns 16j..16j+7 are gate, 16j+8..16j+15 the matching up: 32 columns give 16 outputs
+        // 32 columns of gate and up give 16 outputs
         __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(Cv) + (int64_t)row * ldc + (col0 >> 1);
         __align__(16) __nv_bfloat16 o[16];
+        float gate[16], up[16], y[16];
+        tc_gate_up(v, gate, up);
+        gated_many(y, gate, up, gate_act);
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float gate = v[16 * j + i], up = v[16 * j + 8 + i];
-                o[8 * j + i] = __float2bfloat16_rn(gated_fast_f(gate, up, gate_act));
-            }
+        for (int i = 0; i < 16; ++i) o[i] = __float2bfloat16_rn(y[i]);
         if (col0 + 32 <= N && (ldc % 8) == 0) {
             reinterpret_cast<uint4*>(dst)[0] = *reinterpret_cast<uint4*>(&o[0]);
             reinterpret_cast<uint4*>(dst)[1] = *reinterpret_cast<uint4*>(&o[8]);
@@ -820,6 +826,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                     if (storer) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     uint4 q[8];
+                    float top = 0.f;                                        // of the gates' sizes, see gated_fast
                     if constexpr (EPI == TC_OUT_F32) {
                         float v[32];
                         tc_ld32(taddr + (uint32_t)(j * 32), v);
@@ -839,16 +846,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                         // 32 accumulator columns = gate (8), up (8), gate (8), up (8): 16 outputs
 #pragma unroll
                         for (int cc = 0; cc < 4; ++cc) {
-                            float v[32], o[16];
+                            float v[32], gate[16], up[16], o[16];
                             tc_ld32(taddr + (uint32_t)((4 * j + cc) * 32), v);
                             gate_bias32(v, gate_act, n0 + (4 * j + cc) * 32, N);
-#pragma unroll
-                            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                                for (int i = 0; i < 8; ++i) {
-                                    const float gate = v[16 * h + i], up = v[16 * h + 8 + i];
-                                    o[8 * h + i] = gated_fast_f(gate, up, gate_act);
-                                }
+                            tc_gate_up(v, gate, up);
+                            gated_fast(o, gate, up, gate_act, top);
                             q[2 * cc] = tc2_pack8(o);
                             q[2 * cc + 1] = tc2_pack8(o + 8);
                         }
@@ -856,6 +858,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                     unsigned char* rowp = buf + r * 128;
 #pragma unroll
                     for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(rowp + ((c ^ (r & 7)) << 4)) = q[c];
+                    if (EPI == TC_OUT_SWIGLU_BF16 && __any_sync(0xffffffffu, top > GATE_TOP)) {
+#pragma unroll 1
+                        for (int cc = 0; cc < 4; ++cc) {
+                            float v[32], gate[16], up[16], o[16];
+                            tc_ld32(taddr + (uint32_t)((4 * j + cc) * 32), v);
+                            gate_bias32(v, gate_act, n0 + (4 * j + cc) * 32, N);
+                            tc_gate_up(v, gate, up);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) o[i] = gated_apart_f(gate[i], up[i], gate_act.kind, gate_act.limit);
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) *reinterpret_cast<uint4*>(rowp + (((2 * cc + h) ^ (r & 7)) << 4)) = tc2_pack8(o + 8 * h);
+                        }
+                    }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (storer) {
@@ -1085,12 +1100,23 @@ __global__ void __launch_bounds__(128, 1) gemm_tc_swap_kernel(const __grid_const
                 // Lanes r and r + 8 hold the gate and the up value of one output column.  The gate's lane finishes the first 16
                 // tokens and the up value's the other 16, each giving the other what it needs.  (With the gate's lane alone at
                 // work a tile of 64 tokens took 4.7 us longer than a plain one.)
+                float gate[16], up[16], o[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const float other = __shfl_xor_sync(0xffffffffu, is_gate ? v[16 + i] : v[i], 8);
-                    const float gate = is_gate ? v[i] : other, up = is_gate ? other : v[16 + i];
+                    gate[i] = is_gate ? v[i] : other, up[i] = is_gate ? other : v[16 + i];
+                }
+                // lanes beyond the tile's weight rows hold whatever the stage held, columns beyond M in a list of groups another
+                // group's rows or what lies behind the list: none of them may send the others to the division
+                if (GROUPED && c * 32 + 32 > M)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (c * 32 + (is_gate ? i : 16 + i) >= M) gate[i] = 0.f;
+                gated_many(o, gate, up, gate_act, there);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
                     const int tok = c * 32 + (is_gate ? i : 16 + i);
-                    if (there && tok < M) base[(int64_t)tok * ldc + ocol] = __float2bfloat16_rn(gated_fast_f(gate, up, gate_act));
+                    if (there && tok < M) base[(int64_t)tok * ldc + ocol] = __float2bfloat16_rn(o[i]);
                 }
             } else if (col < N && r < tile_rows) {
                 if (EPI == TC_OUT_F32) {

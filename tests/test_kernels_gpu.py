@@ -1167,9 +1167,46 @@ def test_gated_epilogues_divide_exactly(K, M):
     assert run(z, x, w, K.TC_OUT_F32, status) and run(out, x, w, K.TC_OUT_SWIGLU, status)
     K.check_status(status)
     want = K.swiglu(torch.empty(M, F, device=DEV), z, 8)
-    # (beyond e^87 the fused forms hold the divisor: what is left is below 1e-30 either way)
+    # (what is left below 1e-30 is the next test's)
     tiny = want.abs() < 1e-30
     assert float(z.abs().max()) > 100 and torch.equal(out[~tiny], want.bfloat16()[~tiny]) and (out[tiny].abs() < 1e-30).all()
+
+
+# The same over gates of all sizes: small ones, both ends of the exponential's range, far beyond them, infinite ones and no
+# numbers; few rows (weights streamed, weights on the M side), and pairs of CTAs.  A gate is the sum of three 16-bit pieces in W, which every product adds up exactly, so that the float32
+# product with the division behind it meets the same 32-bit gates.
+def gate_values():
+    big = torch.logspace(-24, 38.5, 900, dtype=torch.float64)
+    ends = torch.tensor([math.inf, math.nan, 1e30, 3e38, 3.3e38, 87.0, 87.3365, 87.5, 88.0, 88.72, 88.7228, 88.723, 88.73, 89.0, 100.0, 51.5, 52.13,
+                         52.2, 103.0, 104.0, 16.6, 17.4, 0.0], dtype=torch.float64)
+    every = torch.cat([torch.linspace(0.01, 110, 2200, dtype=torch.float64), big, ends])
+    every = torch.cat([every, -every]).float()
+    return torch.cat([every, torch.ones(-every.numel() % 8)])
+
+
+@pytest.mark.parametrize("M", [1, 3, 8, 40, 70, 128, 300])
+@pytest.mark.parametrize("act", ["silu", "clipped"])
+def test_gated_epilogues_divide_exactly_at_every_size(K, M, act):
+    g = gate_values()
+    F, Kd = g.numel(), 64
+    pieces, rest = [], g.clone()
+    for _ in range(3):
+        p = rest.bfloat16()
+        pieces.append(p)
+        rest = torch.where(torch.isfinite(rest), rest - p.float(), torch.zeros(()))
+    gate, up = torch.zeros(F, Kd, dtype=torch.bfloat16), torch.zeros(F, Kd, dtype=torch.bfloat16)
+    gate[:, :3] = torch.stack(pieces, 1)
+    up[:, 3] = torch.tensor([1.0, -3.0, 1.5, 0.0625, math.inf, -math.inf, 0.0])[torch.arange(F) % 7]
+    x = torch.zeros(M, Kd, dtype=torch.bfloat16, device=DEV)
+    x[:, :4] = 1
+    w = K.interleave_gate_up(gate, up).to(DEV)
+    out = K.linear_gated(torch.empty(M, F, dtype=torch.bfloat16, device=DEV), x, w, act, 60.0)
+    z = K.linear(torch.empty(M, F, device=DEV), x, gate.to(DEV)).cpu()
+    met = (z == g) | (z.isnan() & g.isnan())
+    assert met.all(), [(float(g[j]), float(z[i, j])) for i, j in (~met).nonzero()[:8].tolist()]      # the pieces' sums are the gates
+    want = K.linear_gated(torch.empty(M, F, device=DEV), x.float(), w.float(), act, 60.0).bfloat16()
+    same = (out.view(torch.int16) == want.view(torch.int16)) | (out.isnan() & want.isnan())
+    assert same.all(), [(float(g[j]), float(out[i, j]), float(want[i, j])) for i, j in (~same).nonzero()[:8].tolist()]
 
 
 @pytest.mark.parametrize("Hq,Hkv,Dh,page,with_norm", [(32, 8, 128, 16, True), (3, 1, 64, 8, True), (5, 2, 128, 32, False),
