@@ -626,8 +626,10 @@ struct TcGroups {
     const int* seg;
     int count;
 };
-constexpr int TC2_MAX_GROUPS = 256;
-constexpr int TC2_GROUP_BYTES = (TC2_MAX_GROUPS + 1) * 4;
+constexpr int TC2_MAX_GROUPS = 1024;   // of a list
+// The pair kernel's table: the first unit of every group, of every second to fourth of more than 256 (all that the ring leaves
+// is 1.7 KB); between two entries the units are counted from the list's offsets.
+constexpr int TC2_TABLE = 256, TC2_GROUP_BYTES = (TC2_TABLE + 1) * 4;
 static_assert(TC2_SMEM_BYTES + TC2_GROUP_BYTES <= 227 * 1024, "the pair kernel's shared memory with a table of groups");
 
 // GROUPED: the units are the groups' tiles, group after group (a group's row tiles fastest, then the columns: the tiles
@@ -656,15 +658,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
     const int num_m = (M + TC2_BM - 1) / TC2_BM, num_n = (N + TC2_BN - 1) / TC2_BN;
     const int n_tiles = num_m * num_n;
     int total = n_tiles * splits;                  // units: all tiles of part 0, then all of part 1, ...
-    int* first_unit = reinterpret_cast<int*>(tmem_slot + 1);   // GROUPED: of every group, and the number of units
+    int* first_unit = reinterpret_cast<int*>(tmem_slot + 1);   // GROUPED: of every group (every `stride`th), and the number of units
+    const int stride = GROUPED ? (groups.count + TC2_TABLE - 1) / TC2_TABLE : 1, entries = GROUPED ? (groups.count + stride - 1) / stride : 0;
     // Where unit u lies: first row and column, part of K, first row of the group's weights, end of the rows.
     struct Unit { int m0, n0, z, w0, rows; };
     auto locate = [&](int u) -> Unit {
         if constexpr (GROUPED) {
-            int g = 0;
-            for (int step = TC2_MAX_GROUPS / 2; step > 0; step >>= 1)
-                if (g + step < groups.count && first_unit[g + step] <= u) g += step;
-            const int a = groups.seg[g], b = groups.seg[g + 1], mt = (b - a + TC2_BM - 1) / TC2_BM, local = u - first_unit[g];
+            int entry = 0;
+            for (int step = TC2_TABLE / 2; step > 0; step >>= 1)
+                if (entry + step < entries && first_unit[entry + step] <= u) entry += step;
+            int g = entry * stride, a = groups.seg[g], b = groups.seg[g + 1], mt = (b - a + TC2_BM - 1) / TC2_BM, local = u - first_unit[entry];
+            while (local >= mt * num_n) {   // never with an entry a group
+                local -= mt * num_n;
+                a = b, b = groups.seg[++g + 1], mt = (b - a + TC2_BM - 1) / TC2_BM;
+            }
             return Unit{a + local % mt * TC2_BM, local / mt * TC2_BN, 0, g * N, b};
         } else {
             const int t = u % n_tiles;
@@ -712,13 +719,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                     const int below = __shfl_up_sync(0xffffffffu, upto, o);
                     if (lane >= o) upto += below;
                 }
-                if (g < groups.count) first_unit[g] = before + upto - mine;
+                if (g < groups.count && g % stride == 0) first_unit[g / stride] = before + upto - mine;
                 before += __shfl_sync(0xffffffffu, upto, 31);
             }
-            if (lane == 0) first_unit[groups.count] = before;
+            if (lane == 0) first_unit[entries] = before;
         }
         __syncthreads();
-        total = first_unit[groups.count];
+        total = first_unit[entries];
     }
 
     if (warp == 0) {

@@ -238,7 +238,7 @@ int imp_moe_combine(void* out, const void* y, const int* pair_row, const float* 
 
 // Epilogues of the products over groups (imp_grouped_gemm_ex).
 enum { GROUPED_PLAIN = 0, GROUPED_RELU2 = 2, GROUPED_SIGMOID_GATE = 3 };
-constexpr int IMP_TC_GROUPS_MAX = 256;   // groups that imp_gemm_bf16_tc_grouped takes
+constexpr int IMP_TC_GROUPS_MAX = 1024;   // groups that imp_gemm_bf16_tc_grouped takes
 // Epilogues of the tcgen05 products.
 enum { TC_OUT_BF16 = 0, TC_OUT_F32 = 1, TC_OUT_SWIGLU = 2, TC_OUT_GEGLU = 4, TC_OUT_CLIPGLU = 5, TC_OUT_RELU2 = 6 };
 // 2 / 4: act(gate) * up, act silu / gelu (tanh form); 5: gate and up clipped to a limit; 6: max(., 0)^2, no gate

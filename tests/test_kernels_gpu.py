@@ -242,6 +242,17 @@ def test_gemm_bf16_tc_grouped(K, counts, N, K_, spare, epi):
         close(out[lo:lo + n, :cols], z, torch.bfloat16, max(float(z.abs().max()), 1.0) if n else 1.0)
 
 
+# More groups than the pair kernel's table has entries (257: two groups an entry; 600: three; 1,024: four), and the kernels of fewer rows a group.
+MANY_GROUPS = [[1, 0, 5] * 85 + [40, 3], [50, 3, 0, 40] * 100 + [9], [130, 0, 257, 1, 0, 300, 256, 128] * 33, [150] * 257, [0, 0, 0, 500, 1, 300] * 100,
+               [0, 700, 0, 1, 0] * 204 + [129, 3, 0, 0], [0] * 1023 + [140000]]
+
+
+@pytest.mark.parametrize("counts", MANY_GROUPS)
+@pytest.mark.parametrize("N,K_,spare,epi", [(48, 40, 0, 2), (272, 136, 5, 0)])
+def test_gemm_bf16_tc_grouped_many(K, counts, N, K_, spare, epi):
+    test_gemm_bf16_tc_grouped(K, counts, N, K_, spare, epi)
+
+
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 7, 8, 9, 16])
 @pytest.mark.parametrize("N,K_", [(10, 64), (257, 200), (96, 4104), (50, 100)])
 @pytest.mark.parametrize("odtype", [torch.bfloat16, torch.float32])

@@ -315,6 +315,7 @@ MOE_CASES = [
     dict(d=40, experts=16, top=1, ff=40, shared=0),        # one expert a token: its weight is 1; no shared expert
     dict(d=72, experts=3, top=3, ff=12, shared=20),        # every expert chosen; a shared size that is no multiple of 8
     dict(d=64, experts=70, top=6, ff=8, shared=8),
+    dict(d=64, experts=600, top=4, ff=8, shared=8),
 ]
 
 
