@@ -65,13 +65,13 @@ class HostPool:
                 self._free.remove(block)
                 return block
             unused = sorted(self._free)
+            if self._held - sum(s for s, _ in unused) + size > self._limit:    # not even without them: they stay
+                return None
             while unused and self._held + size > self._limit:    # blocks of sizes no longer asked for make room
                 s, address = unused.pop()
                 self._free.remove((s, address))
                 self._release(address)
                 self._held -= s
-            if self._held + size > self._limit:
-                return None
             address = self._alloc(size)
             if not address:
                 return None

@@ -55,6 +55,17 @@ def test_limit_and_other_sizes():
     assert pool.array((0, 7)).shape == (0, 7)
 
 
+def test_a_request_beyond_the_limit_leaves_the_free_blocks():
+    heap, pool = make(4 * GRAIN)
+    small, lent = pool.array((GRAIN // 4,)), pool.array((GRAIN // 2,))
+    address = small.ctypes.data
+    del small
+    assert pool.array((8 * GRAIN,)).size == 8 * GRAIN               # larger than the pool
+    assert pool.array((3 * GRAIN // 4,)).size == 3 * GRAIN // 4     # does not fit beside what is lent out
+    assert pool.held == 3 * GRAIN and heap.made == 2
+    assert pool.array((GRAIN // 4,)).ctypes.data == address and lent.size
+
+
 def test_close_frees_now_and_later():
     heap, pool = make(1 << 24)
     a, b = pool.array((10,)), pool.array((10,))
