@@ -183,6 +183,7 @@ _SIGNATURES = {
     "imp_step_tokens": (_E, [_H, POINTER(ImpStepEntry), c_int, c_void_p, c_size_t]),
     "imp_end": (_E, [_H, c_int64]),
     "imp_host_alloc": (_E, [c_size_t, POINTER(c_void_p)]),
+    "imp_context_host_alloc": (_E, [_H, c_size_t, POINTER(c_void_p)]),
     "imp_host_free": (None, [c_void_p]),
     # parts and architectures
     "imp_register_part": (_E, [c_char_p, c_char_p, POINTER(ImpPartVTable)]),

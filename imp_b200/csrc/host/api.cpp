@@ -412,10 +412,7 @@ IMP_EXPORT ImpError imp_end(ImpContext ctx, int64_t id) {
     IMP_CATCH
 }
 
-IMP_EXPORT ImpError imp_host_alloc(size_t bytes, void** out) {
-    IMP_TRY
-    need_arg(out != nullptr && bytes > 0, "imp_host_alloc: out must not be null and bytes must be positive");
-    *out = nullptr;
+static void host_alloc(size_t bytes, void** out) {
     const cudaError_t e = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
     if (e != cudaSuccess) {
         *out = nullptr;
@@ -423,6 +420,22 @@ IMP_EXPORT ImpError imp_host_alloc(size_t bytes, void** out) {
         fail(e == cudaErrorMemoryAllocation ? IMP_ERROR_OUT_OF_MEMORY : IMP_ERROR_CUDA,
              std::string("cannot allocate pinned host memory: ") + cudaGetErrorString(e));
     }
+}
+
+IMP_EXPORT ImpError imp_host_alloc(size_t bytes, void** out) {
+    IMP_TRY
+    need_arg(out != nullptr && bytes > 0, "imp_host_alloc: out must not be null and bytes must be positive");
+    *out = nullptr;
+    host_alloc(bytes, out);
+    IMP_CATCH
+}
+
+IMP_EXPORT ImpError imp_context_host_alloc(ImpContext ctx, size_t bytes, void** out) {
+    IMP_TRY
+    need_arg(ctx && out != nullptr && bytes > 0, "imp_context_host_alloc: ctx and out must not be null and bytes must be positive");
+    *out = nullptr;
+    ctx->e->make_current();
+    host_alloc(bytes, out);
     IMP_CATCH
 }
 

@@ -219,7 +219,7 @@ class Engine:
         capi.check(capi.load().imp_context_create(model._h, ctypes.byref(c), ctypes.byref(ctx)))
         self._ctx = ctx
         self.vocab_size = model.vocab_size
-        self._host_pool = HostPool()            # step_tokens: where logits land
+        self._host_pool = HostPool(context=ctx)  # step_tokens: where logits land
         self._outs = (capi.ImpStepOutput * max(self.config.max_batch_size * 2, 8))()
 
     # ------------------------------------------------------------ construction

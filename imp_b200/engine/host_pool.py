@@ -34,13 +34,14 @@ class _Block:
 
 
 class HostPool:
-    """Blocks of page-locked memory behind float32 arrays.  Any thread may ask for arrays and drop them."""
+    """Blocks of page-locked memory behind float32 arrays.  Any thread may ask for arrays and drop them.  `context`: the engine's,
+    whose device a thread works on that asks for an array (one that never chose would set up the first device)."""
 
-    def __init__(self, limit: int = POOL_BYTES, alloc=None, free=None):
+    def __init__(self, limit: int = POOL_BYTES, alloc=None, free=None, context=None):
         self._limit, self._held, self._closed = limit, 0, False
         self._free: List[Tuple[int, int]] = []       # (size, address)
         self._lock = threading.RLock()                # re-entrant: a collection inside it may drop an array
-        self._alloc, self._release = alloc or _host_alloc, free or _host_free
+        self._alloc, self._release = alloc or (lambda size: _host_alloc(context, size)), free or _host_free
 
     @property
     def held(self) -> int:
@@ -96,9 +97,10 @@ class HostPool:
             self._release(address)
 
 
-def _host_alloc(size: int) -> int:
-    p = ctypes.c_void_p()
-    return (p.value or 0) if capi.load().imp_host_alloc(size, ctypes.byref(p)) == 0 else 0
+def _host_alloc(context, size: int) -> int:
+    p, lib = ctypes.c_void_p(), capi.load()
+    rc = lib.imp_context_host_alloc(context, size, ctypes.byref(p)) if context else lib.imp_host_alloc(size, ctypes.byref(p))
+    return (p.value or 0) if rc == 0 else 0
 
 
 def _host_free(address: int) -> None:

@@ -228,8 +228,11 @@ IMP_EXPORT ImpError imp_step_tokens(ImpContext ctx, const ImpStepEntry* entries,
 IMP_EXPORT ImpError imp_end(ImpContext ctx, int64_t id);
 
 /* Page-locked host memory for `logits_out`: the device writes it directly at the bus's rate, ordinary memory is filled by
- * the driver piece by piece.  Allocating costs about as much as one such fill: keep and reuse it.  Any thread; null may be freed. */
+ * the driver piece by piece.  Allocating costs about as much as one such fill: keep and reuse it.  Any thread; null may be freed.
+ * imp_host_alloc works on the calling thread's current device (the first one, if it never chose); imp_context_host_alloc
+ * chooses the context's device first, as imp_step_tokens does. */
 IMP_EXPORT ImpError imp_host_alloc(size_t bytes, void** out);
+IMP_EXPORT ImpError imp_context_host_alloc(ImpContext ctx, size_t bytes, void** out);
 IMP_EXPORT void imp_host_free(void* p);
 
 #ifdef __cplusplus

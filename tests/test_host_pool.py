@@ -83,6 +83,23 @@ def test_no_page_locked_memory():
     assert pool.array((5, 5)).shape == (5, 5) and pool.held == 0
 
 
+def test_an_engines_pool_allocates_on_the_engines_device(monkeypatch):
+    calls = []
+
+    class Library:
+        def imp_host_alloc(self, size, out):
+            calls.append(None)
+            return 1
+
+        def imp_context_host_alloc(self, ctx, size, out):
+            calls.append((ctx, size))
+            return 1
+
+    monkeypatch.setattr("imp_b200.engine.host_pool.capi.load", Library)
+    assert HostPool(context=77).array((GRAIN,)).size == GRAIN and calls == [(77, 4 * GRAIN)]
+    assert HostPool().array((5,)).size == 5 and calls[1:] == [None]
+
+
 def test_threads():
     heap, pool = make(64 * GRAIN)
     wrong = []
