@@ -4,8 +4,9 @@
 `compute_dtype`, `prefill_chunk_size`, `enable_cuda_graphs` come from
 include/imp/config.h:11-81 (defaults: src/api/imp_api.cpp:35-72);
 `kv_block_size` from src/runtime/engine.h:59.  `max_batch_tokens` (the token
-budget of one step) and `lookahead` are this engine's own.  The dataclass
-mirrors the C API's `ImpConfig` (include/imp_b200/imp.h).
+budget of one step), `lookahead` and `host_pool_bytes` are this engine's own.
+The dataclass mirrors the C API's `ImpConfig` (include/imp_b200/imp.h), beside
+which a C caller places its results itself.
 """
 from __future__ import annotations
 
@@ -29,6 +30,7 @@ class EngineConfig:
     gpu_memory_fraction: float = 0.8  # of free memory to the cache when nothing else sizes it
     state_slots: int = 0              # fixed-size state slots; 0 = max_batch_size
     lookahead: bool = True            # launch the next decode step before reading the last one's tokens
+    host_pool_bytes: int = 512 << 20  # page-locked memory that step_tokens' results may hold; 0 = ordinary memory (Python only)
 
     def validate(self) -> None:
         if self.compute_dtype not in ("bfloat16", "float32"):
@@ -36,8 +38,9 @@ class EngineConfig:
         for name in ("max_batch_size", "max_seq_len", "kv_block_size", "max_batch_tokens"):
             if getattr(self, name) <= 0:
                 raise ValueError(f"{name} must be positive")
-        if self.prefill_chunk_size < 0:
-            raise ValueError("prefill_chunk_size must be >= 0")
+        for name in ("prefill_chunk_size", "host_pool_bytes"):
+            if getattr(self, name) < 0:
+                raise ValueError(f"{name} must be >= 0")
         if self.max_batch_tokens < self.max_batch_size:
             raise ValueError("max_batch_tokens must be at least max_batch_size (one token per decoding request)")
 

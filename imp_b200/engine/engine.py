@@ -219,7 +219,7 @@ class Engine:
         capi.check(capi.load().imp_context_create(model._h, ctypes.byref(c), ctypes.byref(ctx)))
         self._ctx = ctx
         self.vocab_size = model.vocab_size
-        self._host_pool = HostPool(context=ctx)  # step_tokens: where logits land
+        self._host_pool = HostPool(self.config.host_pool_bytes, context=ctx)  # step_tokens: where logits land
         self._outs = (capi.ImpStepOutput * max(self.config.max_batch_size * 2, 8))()
 
     # ------------------------------------------------------------ construction
@@ -354,8 +354,9 @@ class Engine:
 
     def step_tokens(self, entries: Sequence[StepEntry]):
         """Run given tokens as one batch (no scheduling, no sampling).  Returns the logits of the wanted rows
-        as a float32 numpy array [wanted, vocab], in the order of the entries and of each `want` (in page-locked memory
-        that serves a later call once nothing refers to the array any more)."""
+        as a float32 numpy array [wanted, vocab], in the order of the entries and of each `want`.  The array lies in page-locked
+        memory that serves a later call once nothing refers to it any more; a caller that keeps every result pays for new
+        memory in each call, and beyond `EngineConfig.host_pool_bytes` gets ordinary memory: copy what is to be kept."""
         n = len(entries)
         arr = (capi.ImpStepEntry * max(n, 1))()
         keep = []

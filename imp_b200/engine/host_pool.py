@@ -15,7 +15,6 @@ import numpy as np
 
 from .. import capi
 
-POOL_BYTES = 512 << 20    # of page-locked memory a pool holds at most, lent out or free; beyond it arrays are ordinary ones
 GRAIN = 1 << 16           # sizes are rounded up to this, so that a step with a row more finds a block too
 
 
@@ -34,10 +33,11 @@ class _Block:
 
 
 class HostPool:
-    """Blocks of page-locked memory behind float32 arrays.  Any thread may ask for arrays and drop them.  `context`: the engine's,
+    """Blocks of page-locked memory behind float32 arrays, `limit` bytes at most, lent out or free; beyond it arrays are ordinary ones.
+     Any thread may ask for arrays and drop them.  `context`: the engine's,
     whose device a thread works on that asks for an array (one that never chose would set up the first device)."""
 
-    def __init__(self, limit: int = POOL_BYTES, alloc=None, free=None, context=None):
+    def __init__(self, limit: int, alloc=None, free=None, context=None):
         self._limit, self._held, self._closed = limit, 0, False
         self._free: List[Tuple[int, int]] = []       # (size, address)
         self._lock = threading.RLock()                # re-entrant: a collection inside it may drop an array

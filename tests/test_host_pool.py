@@ -96,8 +96,9 @@ def test_an_engines_pool_allocates_on_the_engines_device(monkeypatch):
             return 1
 
     monkeypatch.setattr("imp_b200.engine.host_pool.capi.load", Library)
-    assert HostPool(context=77).array((GRAIN,)).size == GRAIN and calls == [(77, 4 * GRAIN)]
-    assert HostPool().array((5,)).size == 5 and calls[1:] == [None]
+    assert HostPool(1 << 24, context=77).array((GRAIN,)).size == GRAIN and calls == [(77, 4 * GRAIN)]
+    assert HostPool(1 << 24).array((5,)).size == 5 and calls[1:] == [None]
+    assert HostPool(0, context=77).array((5,)).size == 5 and len(calls) == 2      # no page-locked memory at all
 
 
 def test_threads():
