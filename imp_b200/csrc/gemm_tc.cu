@@ -709,20 +709,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
     pdl_launch_dependents();
     if constexpr (GROUPED) {
         if (warp == 0) {
-            int before = 0;
-            for (int g0 = 0; g0 < groups.count; g0 += 32) {
-                const int g = g0 + lane;
-                const int mine = g < groups.count ? (groups.seg[g + 1] - groups.seg[g] + TC2_BM - 1) / TC2_BM * num_n : 0;
-                int upto = mine;
+            // a lane for `per` neighbouring groups, whose loads go out together: their units, the sum over the lanes below, the entries
+            const int per = (groups.count + 31) / 32, g0 = lane * per;
+            auto units = [&](int i) {   // of the lane's group i
+                return (groups.seg[min(g0 + i + 1, groups.count)] - groups.seg[min(g0 + i, groups.count)] + TC2_BM - 1) / TC2_BM * num_n;
+            };
+            int mine = 0;
+#pragma unroll 8
+            for (int i = 0; i < per; ++i) mine += units(i);
+            int upto = mine;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int below = __shfl_up_sync(0xffffffffu, upto, o);
-                    if (lane >= o) upto += below;
-                }
-                if (g < groups.count && g % stride == 0) first_unit[g / stride] = before + upto - mine;
-                before += __shfl_sync(0xffffffffu, upto, 31);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += below;
             }
-            if (lane == 0) first_unit[entries] = before;
+            int before = upto - mine;
+            for (int i = 0; i < per && g0 + i < groups.count; ++i) {
+                if ((g0 + i) % stride == 0) first_unit[(g0 + i) / stride] = before;
+                before += units(i);
+            }
+            if (lane == 31) first_unit[entries] = upto;
         }
         __syncthreads();
         total = first_unit[entries];
@@ -978,25 +984,37 @@ __global__ void __launch_bounds__(128, 1) gemm_tc_swap_kernel(const __grid_const
     int w0 = n0, row0 = 0;                          // the tile's first rows in W and in the list
     if constexpr (GROUPED) {
         pdl_wait();
-        int tile = blockIdx.y, g = -1, end = 0;
-        for (int base = 0; base < groups.count && g < 0; base += 32) {   // every warp for itself, 32 groups at a time
-            const int e = base + lane, a = e < groups.count ? groups.seg[e] : 0, b = e < groups.count ? groups.seg[e + 1] : 0;
-            const int mine = (b - a + BN - 1) / BN;
-            int upto = mine;
+        // Every warp for itself.  A lane counts the tiles of `per` neighbouring groups (its loads go out together), then the lanes
+        // look at the groups of the one that holds this tile: two trips to the memory, however many groups there are.
+        int tile = blockIdx.y, g = -1, end = 0, first = 0;
+        const int per = (groups.count + 31) / 32;
+        for (int step = per; g < 0; step = 1) {
+            const int e0 = first + lane * step;
+            const bool mine = step > 1 || lane < per || per == 1;
+            int a = groups.seg[min(e0, groups.count)], b = a, n = 0;
+            const int a0 = a;
+            if (mine)
+#pragma unroll 8
+                for (int i = 1; i <= step; ++i) {
+                    a = b;
+                    b = groups.seg[min(e0 + i, groups.count)];
+                    n += (b - a + BN - 1) / BN;
+                }
+            int upto = n;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int below = __shfl_up_sync(0xffffffffu, upto, o);
                 if (lane >= o) upto += below;
             }
             const uint32_t past = __ballot_sync(0xffffffffu, tile < upto);
-            if (past) {
-                const int l = __ffs(past) - 1;
-                g = base + l;
-                row0 = __shfl_sync(0xffffffffu, a + (tile - (upto - mine)) * BN, l);
-                end = __shfl_sync(0xffffffffu, b, l);
-            } else {
-                tile -= __shfl_sync(0xffffffffu, upto, 31);
-            }
+            if (!past) break;                                   // beyond the last tile
+            const int l = __ffs(past) - 1;
+            tile -= __shfl_sync(0xffffffffu, upto - n, l);
+            first += l * step;
+            if (step > 1) continue;
+            g = first;
+            row0 = __shfl_sync(0xffffffffu, a0, l) + tile * BN;
+            end = __shfl_sync(0xffffffffu, b, l);
         }
         if (g < 0) return;
         w0 = g * N + n0;
