@@ -456,11 +456,14 @@ bool linear_qkv_rope(Step& st, Tensor q_out, const Tensor& x, const Tensor& w, c
     const int T = (int)rows(x);
     if (T < 256 || (g.dh != 64 && g.dh != 128) || rot.rot_dim != g.dh) return false;
     // The fused epilogue takes about 10 us a tile, twice the plain one and more, which the next tiles' multiply-adds hide only where
-    // a pair of CTAs has several tiles of a long K; elsewhere the plain product and the kernel behind it are faster.  Fused against
-    // plain and rotary kernel, q,k,v of 6144 x 4096: 512 tokens 37.1 / 31.3 us, 576 36.5 / 34.8, 1,024 56.8 / 54.7, 2,048 81.4 / 87.6;
-    // 7168 x 5120: 512 42.3 / 39.6, 576 56.7 / 66.1, 2,048 116 / 129; 4096 x 1024: 512 20.2 / 15.4, 2,048 34.2 / 29.7.  The same bits.
+    // a pair of CTAs has several tiles of a long enough K; elsewhere the plain product and the kernel behind it are faster, or as fast.
+    // Fused against plain and rotary kernel, heads of 128, us behind a flushed L2.  No more tiles than pairs: 512 rows of K 1,024, 2,048,
+    // 3,072, 4,096: 27.5 / 23.6, 31.7 / 27.6, 37.9 / 33.8, 44.0 / 39.9; 768 rows of 6,144 x 4,096 (72 tiles) 46.0 / 46.1.  More: 1,536,
+    // 2,048 and 4,096 rows of 4,096 x 1,024 33.7 / 35.8, 41.8 / 39.9, 62.3 / 62.5 (inside a prompt 2,048: 34.2 / 29.7), of 4,096 x 2,048
+    // 39.9 / 46.0, 48.1 / 50.2, 72.7 / 80.9, of 6,144 x 2,560 52.2 / 56.3, 68.5 / 72.7, 109.6 / 128.0, of 6,144 x 4,096 66.5 / 70.7,
+    // 87.0 / 95.2, 148.3 / 175.1; 1,024 rows of 6,144 x 2,048, 2,560 and 4,096 48.0 / 44.0, 50.2 / 50.2, 64.5 / 64.5.  The same bits.
     const int64_t tiles = (int64_t)((T + 255) / 256) * ((rows(w) + 255) / 256), pairs = std::max(rt.sm_count / 2, 1);
-    if (tiles <= pairs || cols(x) < 4096) return false;
+    if (tiles <= pairs || cols(x) < 2048) return false;
     check_cache(cache, g);
     const ImpCacheView& c = cache.view;
     need(rows(w) == (int64_t)(g.hq + 2 * g.hkv) * g.dh && cols(w) == cols(x) && q_out.dtype == BF16 && rows(q_out) == T &&
