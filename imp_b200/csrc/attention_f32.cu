@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(AF_WARPS * 32, MIN_CTAS) attention_f32_kernel(
     pdl_launch_dependents();
     constexpr int DH = 32 * DV;
     __shared__ int64_t offs[AF_WARPS][AF_KEYS];
-    __shared__ float part[CTA_A_TOKEN ? AF_WARPS * GH * DH : 1], part_m[AF_WARPS][GH], part_l[AF_WARPS][GH];
+    __shared__ __align__(16) float part[CTA_A_TOKEN ? AF_WARPS * GH * DH : 4];   // written 16 bytes at a time
+    __shared__ float part_m[AF_WARPS][GH], part_l[AF_WARPS][GH];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = a.Hq / a.Hkv, sets = (G + GH - 1) / GH, hk = blockIdx.y / sets, h0 = hk * G + blockIdx.y % sets * GH;
     const int n_heads = min(GH, (hk + 1) * G - h0);
