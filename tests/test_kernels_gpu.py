@@ -674,6 +674,56 @@ def test_attention_f32_forms(K, Hq, Hkv, Dh, page, window):
     close(out[:T].view(T, Hq, Dh), want, torch.float32)
 
 
+# What a key without a page, an infinite or undefined score does there, in both forms: a missing key is left out and reported, a score of
+# -inf weighs nothing, one of +inf or NaN leaves no number behind, nor do scores that are all -inf.
+@pytest.mark.parametrize("Hq,Hkv,Dh,page", [(16, 8, 128, 16), (3, 1, 64, 8), (2, 2, 256, 4)])
+@pytest.mark.parametrize("case", ["missing", "own missing", "all missing", "-inf", "every -inf", "+inf", "nan", "nan value"])
+def test_attention_f32_missing_keys_and_infinities(K, Hq, Hkv, Dh, page, case):
+    n, G = 300, Hq // Hkv
+    bt, num_pages, kc, vc, dense, toks, q = attention_case([n], [n], Hq, Hkv, Dh, page, torch.float32)
+    q[:, :, 0] = 1.0
+    bad = {"missing": range(64, 112), "own missing": range(n - n % page if n % page else n - page, n), "all missing": range(n), "-inf": range(64, 140), "every -inf": range(n), "+inf": [97], "nan": [33],
+           "nan value": [70]}[case]
+    k, v = dense[0][1].double(), dense[0][2].double()
+    there = torch.ones(n, dtype=torch.bool)
+    for j in bad:
+        where = (int(bt[0, j // page]), slice(None), j % page)
+        if "missing" in case:
+            there[j] = False
+        elif case == "nan value":
+            vc[where], v[j] = math.nan, math.nan
+        else:
+            kc[where + (0,)] = k[j, :, 0] = {"-inf": -math.inf, "every -inf": -math.inf, "+inf": math.inf, "nan": math.nan}[case]
+    if "missing" in case:
+        bt[0, [j // page for j in bad]] = -1
+    want = torch.zeros(n, Hq, Dh, dtype=torch.float64)
+    for p in range(n):
+        at = there[:p + 1].nonzero()[:, 0]
+        if len(at):
+            sc = torch.einsum("hd,jhd->hj", q[p].double(), k[at].repeat_interleave(G, 1)) / math.sqrt(Dh)
+            w = torch.softmax(sc, 1)
+            w = torch.where(((sc == math.inf) | sc.isnan()).any(1, keepdim=True), torch.full_like(w, math.nan), w)
+            want[p] = torch.einsum("hj,jhd->hd", w, v[at].repeat_interleave(G, 1))
+    seq, pos = torch.zeros(n, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV)
+    q, kc, vc, bt = q.reshape(n, Hq * Dh).to(DEV), kc.to(DEV), vc.to(DEV), bt.to(DEV)
+    status = K.new_status(DEV)
+    many = torch.empty(8 * n, Hq * Dh, device=DEV)
+    K.paged_attention_generic(many, q.repeat(8, 1), Hq, Hkv, Dh, kc, vc, bt, seq.repeat(8), pos.repeat(8), 1 / math.sqrt(Dh), 0, status)
+    few = torch.empty(n, Hq * Dh, device=DEV)
+    for a in range(0, n, 4):
+        K.paged_attention_generic(few[a:a + 4], q[a:a + 4], Hq, Hkv, Dh, kc, vc, bt, seq[a:a + 4], pos[a:a + 4], 1 / math.sqrt(Dh), 0, status)
+    if "missing" in case:
+        with pytest.raises(Exception, match="page"):
+            K.check_status(status)
+    else:
+        K.check_status(status)
+    want = want.view(n, -1)
+    for got in (many[:n].cpu(), many[-n:].cpu(), few.cpu()):
+        assert torch.equal(got.isnan(), want.isnan())
+        close(torch.nan_to_num(got), torch.nan_to_num(want), torch.float32)
+        assert torch.equal(torch.nan_to_num(got), torch.nan_to_num(few.cpu()))
+
+
 ALL_HEAD_DIMS = list(range(16, 257, 16))
 
 
