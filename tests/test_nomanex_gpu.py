@@ -474,8 +474,9 @@ def test_routed_experts_with_softmax_scores_and_groups(dtype, case):
         assert (N.moe(x.double(), W, "f.", free) - want).abs().max() > 0.05 * want.abs().max(), "the groups decide"
 
 
-def test_experts_of_long_portions_take_the_dense_products():
-    """Enough work an expert that its rows go to the tensor-memory products with the squared relu in their epilogue."""
+def test_experts_of_long_portions_on_pairs_of_ctas():
+    """Thousands of rows an expert: the tensor-memory products over groups on pairs of CTAs, the squared relu in their epilogue.  200,
+    80 and 30 tokens (half as many rows an expert): weights streamed beside tiles of 128, 64 and 32 of the list's rows."""
     d, c = 512, {"router": {"experts": 2, "top": 1}, "expert": {"ff": 1024}}
     w = {k: v.to(torch.bfloat16) for k, v in moe_weights(d, c, seed=510).items()}
     bench = PartBench("bfloat16", [], max_tokens=9216, max_seq_len=9216)
@@ -483,8 +484,10 @@ def test_experts_of_long_portions_take_the_dense_products():
     part = bench.build("feed_forward", PartSpec("routed_experts", moe_params(d, c)), {names[k]: v.to(DEV) for k, v in w.items()})
     x = rnd(9000, d, seed=511).to(torch.bfloat16)
     out = run_part(bench, part, x, bench.prepare([("a", [1] * 9000, [])]))
-    few = run_part(bench, part, x[:200], bench.prepare([("b", [1] * 200, [])]))     # the grouped products
-    close(out[:200], few, torch.bfloat16, "dense against grouped products")
+    for n in (200, 80, 30):
+        few = run_part(bench, part, x[:n], bench.prepare([(f"b{n}", [1] * n, [])]))
+        close(out[:n], few, torch.bfloat16, f"a long portion against {n} tokens")
+        bench.end(f"b{n}")
     W = {"f." + k: v.float() for k, v in w.items()}
     at = torch.arange(0, 9000, 450)
     sure = N.route_margin(x[at].float(), W, "f.", c) > 1e-2

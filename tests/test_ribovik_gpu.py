@@ -393,8 +393,9 @@ def test_routed_clipped_experts_with_identities_and_a_shared_one(dtype, d, c):
         assert far(R.moe(x.double(), free, "f.", c)), "the correction decides"
 
 
-def test_experts_of_long_portions_take_the_dense_products():
-    """Enough work an expert that its rows go to the tensor-memory products with the clipped gate in their epilogue."""
+def test_experts_of_long_portions_on_pairs_of_ctas():
+    """Thousands of rows an expert: the tensor-memory products over groups on pairs of CTAs, the clipped gate in their epilogue.  100, 40
+    and 20 tokens (as many rows an expert at most): weights streamed beside tiles of 128, 64 and 32 of the list's rows."""
     d, c = 512, moe_config(2, 1, 2, 1024, 1.1, None)
     w = {k: v.to(torch.bfloat16) for k, v in moe_weights(d, c, seed=510).items()}
     bench = PartBench("bfloat16", [], max_tokens=9216, max_seq_len=9216)
@@ -403,8 +404,10 @@ def test_experts_of_long_portions_take_the_dense_products():
     x = rnd(9000, d, seed=511).to(torch.bfloat16)
     run_part(bench, part, x[:7000], bench.prepare([("c", [1] * 7000, [])]))         # leaves the workspace full of other numbers
     out = run_part(bench, part, x, bench.prepare([("a", [1] * 9000, [])]))
-    few = run_part(bench, part, x[:200], bench.prepare([("b", [1] * 200, [])]))     # the grouped products
-    close(out[:200], few, torch.bfloat16, "dense against grouped products")
+    for n in (200, 100, 40, 20):
+        few = run_part(bench, part, x[:n], bench.prepare([(f"b{n}", [1] * n, [])]))
+        close(out[:n], few, torch.bfloat16, f"a long portion against {n} tokens")
+        bench.end(f"b{n}")
     W = {"f." + k: v.float() for k, v in w.items()}
     at = torch.arange(0, 9000, 450)
     sure = R.route_margin(x[at].float(), W, "f.", c) > 5e-3
