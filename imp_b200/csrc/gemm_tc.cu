@@ -639,14 +639,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
     gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                         void* __restrict__ Cv, int64_t ldc, int M, int N, int K, int* status,
                         const __grid_constant__ QkvRopeArgs qkv, int splits, int kb_per_split, int64_t split_stride,
-                        const __grid_constant__ CUtensorMap map_c, int tma_store, GateAct gate_act, TcGroups groups, int bn_rt) {
+                        const __grid_constant__ CUtensorMap map_c, int tma_store, GateAct gate_act, TcGroups groups) {
     // tma_store: C goes out through shared memory and TMA stores described by map_c (boxes of 128 rows x 64 columns, 32 of
     // 32-bit values, the parts of a cut K range one below the other) instead of 16-byte stores from every thread.
     // splits > 1 (32-bit output only): the K range is cut into `splits` parts, each (tile, part) is a unit of work of its
     // own and writes its partial product split_stride elements after the part before; the caller adds the parts in order.
-    // bn_rt: columns of a tile (tc2_tile_cols), 256 in the epilogues with a fixed width.
-    constexpr bool ANY_COLS = !GROUPED && (EPI == TC_OUT_BF16 || EPI == TC_OUT_F32);
-    const int bn = ANY_COLS ? bn_rt : TC2_BN;
     IMP_TL_BEGIN(20 + EPI)
     extern __shared__ unsigned char tc_smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -658,7 +655,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
     const uint32_t rank = cluster_rank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int k_blocks = (K + TC_BK - 1) / TC_BK;
-    const int num_m = (M + TC2_BM - 1) / TC2_BM, num_n = (N + bn - 1) / bn;
+    const int num_m = (M + TC2_BM - 1) / TC2_BM, num_n = (N + TC2_BN - 1) / TC2_BN;
     const int n_tiles = num_m * num_n;
     int total = n_tiles * splits;                  // units: all tiles of part 0, then all of part 1, ...
     int* first_unit = reinterpret_cast<int*>(tmem_slot + 1);   // GROUPED: of every group (every `stride`th), and the number of units
@@ -678,7 +675,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             return Unit{a + local % mt * TC2_BM, local / mt * TC2_BN, 0, g * N, b};
         } else {
             const int t = u % n_tiles;
-            return Unit{(t % num_m) * TC2_BM, (t / num_m) * bn, u / n_tiles, 0, M};
+            return Unit{(t % num_m) * TC2_BM, (t / num_m) * TC2_BN, u / n_tiles, 0, M};
         }
     };
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + TC2_STAGES);
@@ -745,14 +742,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             for (int u = pair; u < total && ok; u += n_pairs) {
                 const Unit at = locate(u);
                 const int kb_lo = at.z * kb_per_split, kb_hi = min(k_blocks, kb_lo + kb_per_split);
-                const int m0 = at.m0 + (int)rank * 128, n0 = at.w0 + at.n0 + (int)rank * (bn / 2);
+                const int m0 = at.m0 + (int)rank * 128, n0 = at.w0 + at.n0 + (int)rank * 128;
                 for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
                     const uint32_t s = it % TC2_STAGES;
                     ok = mbar_wait(empty0 + 8 * s, ((it / TC2_STAGES) & 1u) ^ 1u, status);
                     if (!ok) break;
                     const uint32_t a_dst = smem_u32(tiles + s * TC2_STAGE_BYTES), b_dst = a_dst + TC2_HALF_BYTES;
                     const uint32_t full_even = cluster_map(full0 + 8 * s, 0);
-                    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (TC2_HALF_BYTES + (uint32_t)(bn / 2) * TC_BK * 2));   // both CTAs' copies
+                    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * TC2_STAGE_BYTES);   // both CTAs' copies
                     tma_load_2d_pair(a_dst, &map_a, kb * TC_BK, m0, full_even);
                     tma_load_2d_pair(b_dst, &map_w, kb * TC_BK, n0, full_even);
                 }
@@ -765,7 +762,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
             // ------------------------------------------------------------ MMA issuer (even CTA)
-            const uint32_t idesc = tc_instr_desc(TC2_BM, bn);
+            const uint32_t idesc = tc_instr_desc(TC2_BM, TC2_BN);
             uint32_t it = 0, local = 0;
             bool ok = true;
             for (int u = pair; u < total && ok; u += n_pairs, ++local) {
@@ -826,13 +823,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             // TMA stores only for a CTA's 128 rows that all lie inside C (and whole 64-column pieces): a store that the
             // tensor map clips measured far slower than the threads' own stores (2048 x 24576 outputs cut at 320 rows:
             // 97 us against 78), so the last, partly filled row block of a matrix takes the plain path.
-            const bool whole = m0 + 128 <= rows && n0 + bn <= N;
+            const bool whole = m0 + 128 <= rows && n0 + TC2_BN <= N;
             if (EPI == TC_OUT_QKV_ROPE) {
                 const QkvStage stg{tma_store && m0 + 128 <= rows ? out_stage : nullptr, &map_c, storer, quarter * 32 + lane, m0};
                 qkv_rope_row(qkv, taddr, row, n0, N, row < rows, status, stg);
             } else if (EPI != TC_OUT_QKV_ROPE && tma_store && whole) {
                 constexpr int COLS = EPI == TC_OUT_F32 ? 32 : 64;           // of a sub-tile: rows of 128 bytes
-                const int SUBS = (EPI == TC_OUT_SWIGLU_BF16 ? 128 : bn) / COLS;
+                constexpr int SUBS = (EPI == TC_OUT_SWIGLU_BF16 ? 128 : 256) / COLS;
                 const int x0 = EPI == TC_OUT_SWIGLU_BF16 ? n0 >> 1 : n0;
                 const int r = quarter * 32 + lane;                          // row in the CTA's half of the tile
 #pragma unroll 1
@@ -896,7 +893,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                 }
             } else {
 #pragma unroll 1
-                for (int c = 0; c < bn / 32; ++c) {
+                for (int c = 0; c < TC2_BN / 32; ++c) {
                     float v[32];
                     tc_ld32(taddr + (uint32_t)(c * 32), v);
                     plain_act<EPI>(v, gate_act, n0 + c * 32, N);
@@ -1255,24 +1252,8 @@ static int make_map(CUtensorMap* map, const void* base, int rows, int K, int64_t
     return 0;
 }
 
-// Columns of a tile of the pair kernel: the width whose rounds of tiles take least.
-static int tc2_tile_cols(int M, int N, int k_blocks) {
-    static const int fixed = [] { const char* e = getenv("IMP_B200_TC_TILE_COLS"); return e ? atoi(e) : 256; }();   // 256, 192 or 128: no choice
-    if (fixed == 256 || fixed == 192 || fixed == 128) return fixed;
-    const int pairs = imp_sm_count() / 2 > 0 ? imp_sm_count() / 2 : 1;
-    const int64_t num_m = (M + TC2_BM - 1) / TC2_BM;
-    int best = TC2_BN;
-    double least = 0;
-    for (int bn : {256, 192, 128}) {
-        const int64_t tiles = num_m * ((N + bn - 1) / bn), rounds = (tiles + pairs - 1) / pairs;
-        const double us = rounds * (k_blocks * (bn == 256 ? 0.32 : bn == 192 ? 0.25 : 0.18)) + 1.5 * (bn / 256.0);
-        if (bn == 256 || us < 0.95 * least) least = us, best = bn;
-    }
-    return best;
-}
-
 template <int EPI>
-static int launch_tc(void* C, int64_t ldc, const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mw128, const void* W, int64_t ldw, int M,
+static int launch_tc(void* C, int64_t ldc, const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mw128, int M,
                      int N, int K, int* status, cudaStream_t s, GateAct gate_act = GateAct()) {
     static bool attr_set = false;
     if (!attr_set) {
@@ -1300,12 +1281,8 @@ static int launch_tc(void* C, int64_t ldc, const CUtensorMap& ma, const CUtensor
     static int pair_min_rows = -1;   // IMP_B200_TC_PAIR_ROWS: rows from which CTA pairs take the product (default 129)
     if (pair_min_rows < 0) { const char* e = getenv("IMP_B200_TC_PAIR_ROWS"); pair_min_rows = e ? atoi(e) : 129; }
     if (mode == 0 && pair_mode == 1 && M >= pair_min_rows) {
-        const int bn = EPI == TC_OUT_BF16 || EPI == TC_OUT_F32 ? tc2_tile_cols(M, N, (K + TC_BK - 1) / TC_BK) : TC2_BN;
-        const int tiles2 = ((M + TC2_BM - 1) / TC2_BM) * ((N + bn - 1) / bn);
+        const int tiles2 = ((M + TC2_BM - 1) / TC2_BM) * ((N + TC2_BN - 1) / TC2_BN);
         const int pairs = tiles2 < sms / 2 ? tiles2 : sms / 2;
-        CUtensorMap mwh = mw128;       // W's rows in halves of a tile
-        if (bn != TC2_BN)
-            if (int rc = make_map(&mwh, W, N, K, ldw, bn / 2)) return rc;
         // bfloat16 outputs leave through TMA stores where C's rows allow them (16-byte strides)
         static int tma_out = -1;       // IMP_B200_TC_TMA_STORE=0: every thread stores its own row
         if (tma_out < 0) { const char* e = getenv("IMP_B200_TC_TMA_STORE"); tma_out = e ? atoi(e) : 1; }
@@ -1313,8 +1290,8 @@ static int launch_tc(void* C, int64_t ldc, const CUtensorMap& ma, const CUtensor
         int tma_store = 0;
         if (tma_out && ldc % 8 == 0)
             tma_store = make_map(&mc, C, M, EPI == TC_OUT_SWIGLU_BF16 ? N / 2 : N, ldc, 128, EPI == TC_OUT_F32) == 0 ? 1 : 0;
-        cudaError_t e = imp_launch(gemm_tc_pair_kernel<EPI>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)TC2_SMEM_BYTES, s, ma, mwh,
-                                   C, ldc, M, N, K, status, QkvRopeArgs{}, 1, (K + TC_BK - 1) / TC_BK, (int64_t)0, mc, tma_store, gate_act, TcGroups{}, bn);
+        cudaError_t e = imp_launch(gemm_tc_pair_kernel<EPI>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)TC2_SMEM_BYTES, s, ma, mw128,
+                                   C, ldc, M, N, K, status, QkvRopeArgs{}, 1, (K + TC_BK - 1) / TC_BK, (int64_t)0, mc, tma_store, gate_act, TcGroups{});
         if (e != cudaSuccess) { imp_set_error("gemm_tc: %s", cudaGetErrorString(e)); return (int)e; }
         return 0;
     }
@@ -1353,9 +1330,9 @@ IMP_API int imp_gemm_bf16_tc_act(void* C, int64_t ldc, int epilogue, float limit
     cudaStream_t s = (cudaStream_t)stream;
     CUtensorMap mw128;   // the W tile in halves of 128 rows, for CTA pairs
     if (int rc = make_map(&mw128, W, N, K, ldw, 128)) return rc;
-    if (epilogue == TC_OUT_BF16) return launch_tc<TC_OUT_BF16>(C, ldc, ma, mw, mw128, W, ldw, M, N, K, status, s, gate_act);
-    if (epilogue == TC_OUT_F32) return launch_tc<TC_OUT_F32>(C, ldc, ma, mw, mw128, W, ldw, M, N, K, status, s);
-    return launch_tc<TC_OUT_SWIGLU_BF16>(C, ldc, ma, mw, mw128, W, ldw, M, N, K, status, s, gate_act);
+    if (epilogue == TC_OUT_BF16) return launch_tc<TC_OUT_BF16>(C, ldc, ma, mw, mw128, M, N, K, status, s, gate_act);
+    if (epilogue == TC_OUT_F32) return launch_tc<TC_OUT_F32>(C, ldc, ma, mw, mw128, M, N, K, status, s);
+    return launch_tc<TC_OUT_SWIGLU_BF16>(C, ldc, ma, mw, mw128, M, N, K, status, s, gate_act);
 }
 
 IMP_API int imp_gemm_bf16_tc(void* C, int64_t ldc, int epilogue, const void* A, int64_t lda, const void* W, int64_t ldw, int M, int N,
@@ -1421,7 +1398,7 @@ IMP_API int imp_gemm_bf16_tc_partials(float* scratch, const void* A, int64_t lda
     const int pairs = units < sms / 2 ? units : sms / 2;
     cudaError_t e = imp_launch(gemm_tc_pair_kernel<TC_OUT_F32>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)TC2_SMEM_BYTES,
                                (cudaStream_t)stream, ma, mw128, (void*)scratch, (int64_t)N, M, N, K, status, QkvRopeArgs{}, splits,
-                               kb_per_split, (int64_t)M * N, mc, tma_store, 0, TcGroups{}, TC2_BN);
+                               kb_per_split, (int64_t)M * N, mc, tma_store, 0, TcGroups{});
     if (e != cudaSuccess) { imp_set_error("imp_gemm_bf16_tc_partials: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;
 }
@@ -1650,7 +1627,7 @@ static int launch_grouped_pair(void* C, int64_t ldc, const void* A, int64_t lda,
     const int64_t units = ((int64_t)M / TC2_BM + groups.count) * ((N + TC2_BN - 1) / TC2_BN);   // at most
     const int pairs = (int)std::min<int64_t>(units, std::max(imp_sm_count() / 2, 1));
     e = imp_launch(gemm_tc_pair_kernel<EPI, true>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)smem, s, ma, mw, C, ldc, M, N, K, status,
-                   QkvRopeArgs{}, 1, (K + TC_BK - 1) / TC_BK, (int64_t)0, mc, tma_store, act, groups, TC2_BN);
+                   QkvRopeArgs{}, 1, (K + TC_BK - 1) / TC_BK, (int64_t)0, mc, tma_store, act, groups);
     if (e != cudaSuccess) { imp_set_error("gemm_tc_grouped: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;
 }
@@ -1752,7 +1729,7 @@ IMP_API int imp_gemm_bf16_tc_qkv_rope(const void* A, int64_t lda, const void* W,
     }
     cudaError_t e = imp_launch(gemm_tc_pair_kernel<TC_OUT_QKV_ROPE>, dim3(2 * pairs), dim3(TCP_THREADS), (size_t)TC2_SMEM_BYTES,
                                (cudaStream_t)stream, ma, mw128, (void*)nullptr, (int64_t)0, M, N, K, status, a, 1,
-                               (K + TC_BK - 1) / TC_BK, (int64_t)0, mq, q_tma, 0, TcGroups{}, TC2_BN);
+                               (K + TC_BK - 1) / TC_BK, (int64_t)0, mq, q_tma, 0, TcGroups{});
     if (e != cudaSuccess) { imp_set_error("imp_gemm_bf16_tc_qkv_rope: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;
 }
