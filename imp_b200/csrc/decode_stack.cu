@@ -338,7 +338,7 @@ struct Consumer {
     // x = rmsnorm(h) * w, from the shares of the sums of squares.  The stream is asked for before the sums are there.
     template <int XS>
     __device__ __forceinline__ void norm_x(uint32_t (&x)[XS][16], float eps) {
-        constexpr int AHEAD = XS < 2 ? XS : 2;       // parts on their way at a time: a trip to the L2 takes 2 us beside the weights' stream
+        constexpr int AHEAD = XS <= 4 ? XS : 3;      // parts on their way at a time: a trip to the L2 takes 2 us beside the weights' stream
         float s = 0.f;
         if (warp < a.T) {
 #pragma unroll
@@ -782,16 +782,6 @@ __device__ __forceinline__ void grid_wait(const StackArgs& a, Shared& sh, unsign
     consumers_sync();
 }
 
-// The attention phase is a function of its own, not inlined: beside the products' code it cost 400 bytes of spilled registers a thread.
-__device__ __noinline__ Ring attention_phase(const StackArgs& a, const StackLayer& L, Ring at) {
-    const int tid = threadIdx.x, lane = tid & 31;
-    Shared& sh = *reinterpret_cast<Shared*>(stack_smem);
-    Consumer c{a, sh, reinterpret_cast<float*>(stack_smem + a.scratch_at), stack_smem + a.ring_at, nullptr, smem_u32(sh.full), smem_u32(sh.empty), tid, lane, tid >> 5,
-               lane >> 2, lane & 3, at};
-    c.attention(L);
-    return c.at;
-}
-
 template <int XS>
 __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_constant__ StackArgs a) {
     Shared& sh = *reinterpret_cast<Shared*>(stack_smem);
@@ -899,7 +889,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
                     *reinterpret_cast<float4*>(sh.qk_norm[0] + e) = __ldg(reinterpret_cast<const float4*>(e < DH ? L.q_norm + e : L.k_norm + (e - DH)));
                 }
                 grid_wait(a, sh, target += all);
-                c.at = attention_phase(a, L, c.at);
+                c.attention(L);
             }
             grid_arrive(a);
             grid_wait(a, sh, target += all);
