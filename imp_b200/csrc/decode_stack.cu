@@ -329,16 +329,15 @@ struct Consumer {
             x[8 * i] = u.x, x[8 * i + 1] = u.y, x[8 * i + 2] = u.z, x[8 * i + 3] = u.w, x[8 * i + 4] = v.x, x[8 * i + 5] = v.y, x[8 * i + 6] = v.z, x[8 * i + 7] = v.w;
         }
     }
-    // The norm's weights into shared memory, between arriving at the barrier behind which the stream is ready and waiting there.
+    // The norm's weights into shared memory, before the barrier behind which the stream is ready.
     __device__ __forceinline__ void load_norm(const void* src) const {
 #pragma unroll 1
-        for (int i = tid - 32; i < a.d / 8; i += CT - 32)       // the first warp waits at the barrier
-            if (i >= 0) norm_s[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
+        for (int i = tid; i < a.d / 8; i += CT) norm_s[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
     }
     // x = rmsnorm(h) * w, from the shares of the sums of squares.  The stream is asked for before the sums are there.
     template <int XS>
     __device__ __forceinline__ void norm_x(uint32_t (&x)[XS][16], float eps) {
-        constexpr int AHEAD = XS <= 4 ? XS : 3;      // parts on their way at a time: a trip to the L2 takes 2 us beside the weights' stream
+        constexpr int AHEAD = XS < 2 ? XS : 2;       // parts on their way at a time
         float s = 0.f;
         if (warp < a.T) {
 #pragma unroll
@@ -759,19 +758,18 @@ struct Consumer {
     }
 };
 
-// Everybody's stores before grid_arrive, everybody's loads after grid_wait.  All consumer threads call both; `target`: arrivals of all CTAs so far and
-// at this one.  (A word a CTA, which all others read, instead of one counter: 8 us instead of 2.)
-__device__ __forceinline__ void grid_arrive(const StackArgs& a) {
+// Everybody's stores before, everybody's loads after.  All consumer threads call it.  A CTA says in a word of its own how many barriers it has
+// reached, and a thread a CTA waits for that word: the arrivals do not queue at one address.
+__device__ __forceinline__ void grid_sync(const StackArgs& a, Shared& sh, unsigned reached) {
     consumers_sync();
-    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.sync) : "memory");
-}
-__device__ __forceinline__ void grid_wait(const StackArgs& a, Shared& sh, unsigned target) {
-    if (threadIdx.x == 0) {
+    unsigned* flags = a.sync + 2 + a.T * a.hkv;
+    if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + blockIdx.x), "r"(reached) : "memory");
+    if (threadIdx.x < gridDim.x) {
 #pragma unroll 1
         for (uint32_t i = 0;; ++i) {
             unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.sync) : "memory");
-            if (v >= target || sh.dead) break;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flags + threadIdx.x) : "memory");
+            if (v >= reached || sh.dead) break;
             if (i == TC_WAIT_LIMIT) {
                 sh.dead = 1;
                 imp_report(a.status, IMP_WAIT_TIMEOUT);
@@ -871,33 +869,25 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
         Consumer c{a, sh, reinterpret_cast<float*>(stack_smem + a.scratch_at), stack_smem + a.ring_at, reinterpret_cast<uint4*>(stack_smem + a.norm_at), full, empty, tid, lane, warp, lane >> 2, lane & 3};
-        const unsigned all = gridDim.x;
-        unsigned target = all;
+        unsigned reached = 0;
         c.first_squares(d0, d1);
-        grid_arrive(a);
         c.load_norm(layers[0].norm1);
-        grid_wait(a, sh, target);
+        grid_sync(a, sh, ++reached);
 #pragma unroll 1
         for (int i = 0; i < a.n_layers * 2; ++i) {       // one copy of each product's code: what a layer runs must stay in the instruction cache
             const StackLayer& L = layers[i >> 1];
             const bool ffn = i & 1;
             c.normed_product<XS>(ffn ? a.eps2 : a.eps1, ffn ? f0 : qkv0, ffn ? f1 : qkv1, ffn, ffn ? a.hid : a.qkv, ffn ? a.F : qkv);
             if (!ffn) {
-                grid_arrive(a);
-                if (L.q_norm && tid >= CT - 64) {
-                    const int e = (tid - (CT - 64)) * 4;
-                    *reinterpret_cast<float4*>(sh.qk_norm[0] + e) = __ldg(reinterpret_cast<const float4*>(e < DH ? L.q_norm + e : L.k_norm + (e - DH)));
-                }
-                grid_wait(a, sh, target += all);
+                if (L.q_norm && tid < 2 * DH) sh.qk_norm[tid / DH][tid % DH] = __ldg((tid < DH ? L.q_norm : L.k_norm) + tid % DH);
+                grid_sync(a, sh, ++reached);
                 c.attention(L);
             }
-            grid_arrive(a);
-            grid_wait(a, sh, target += all);
+            grid_sync(a, sh, ++reached);
             c.branch_product(ffn ? a.hid : a.attn, ffn ? a.F : a.hq * DH, d0, d1);
             if (i + 1 < a.n_layers * 2) {
-                grid_arrive(a);
                 c.load_norm(ffn ? layers[(i >> 1) + 1].norm1 : L.norm2);
-                grid_wait(a, sh, target += all);
+                grid_sync(a, sh, ++reached);
             }
         }
     }
@@ -907,7 +897,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         __threadfence();
         if (atomicAdd(a.sync + 1, 1u) == gridDim.x - 1) {
 #pragma unroll 1
-            for (int i = 0; i < 2 + a.T * a.hkv; ++i) a.sync[i] = 0u;
+            for (int i = 0; i < 2 + a.T * a.hkv + (int)gridDim.x; ++i) a.sync[i] = 0u;
             __threadfence();
         }
     }
@@ -956,7 +946,7 @@ IMP_API int imp_decode_stack_items(int T, int hkv) { return T * hkv > stack_ctas
 
 IMP_API int imp_decode_stack_supported(int d, int F, int hq, int hkv, int dh, int page_size, int n_layers) {
     const int ctas = stack_ctas();
-    if (ctas < 1 || ctas > STACK_SS_STRIDE || dh != DH || hkv <= 0 || hq % hkv || hq / hkv > 8) return 0;
+    if (ctas < 1 || ctas > CT || dh != DH || hkv <= 0 || hq % hkv || hq / hkv > 8) return 0;
     if (d <= 0 || d % 64 || d > 6 * KC || F <= 0 || F % 64 || page_size <= 0 || page_size % 16 || n_layers <= 0 || n_layers > STACK_MAX_LAYERS) return 0;
     return (d + ctas - 1) / ctas <= TILES * TILE;
 }

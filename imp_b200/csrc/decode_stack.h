@@ -24,7 +24,7 @@ struct StackArgs {
     void *qkv, *attn, *hid;
 #endif
     float *ss, *part_o, *part_ml;
-    unsigned* sync;             // [2 + T hkv], zero between launches
+    unsigned* sync;             // [2 + T hkv + STACK_SS_STRIDE], zero between launches
     const int *positions, *seq_of_token, *block_table;
     int bt_stride, n_seqs, page_size, num_pages;
     const float *cos_tab, *sin_tab;   // [max_pos, 64]

@@ -520,7 +520,7 @@ void DeviceModel::build_stack() {
     }
     stack_layers_ = DeviceBuffer(layers.size() * sizeof(StackLayer));
     IMP_CUDA(cudaMemcpy(stack_layers_.data(), layers.data(), layers.size() * sizeof(StackLayer), cudaMemcpyHostToDevice));
-    stack_sync_ = DeviceBuffer((size_t)(2 + STACK_MAX_TOKENS * stack_.hkv) * 4, true);
+    stack_sync_ = DeviceBuffer((size_t)(2 + STACK_MAX_TOKENS * stack_.hkv + STACK_SS_STRIDE) * 4, true);
     IMP_CUDA(cudaStreamSynchronize(rt_->stream));
     stack_on_ = true;
 }
