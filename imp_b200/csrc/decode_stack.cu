@@ -37,19 +37,20 @@ constexpr int PW = 4;                         // producer warps: a warpgroup
 constexpr int THREADS = CT + PW * 32;
 constexpr int KW = 128;                       // of the contraction a warp and stage
 constexpr int KC = KW * CW;                   // of the contraction in a stage
-constexpr int ROWS = 8, TILE = 2 * ROWS;      // rows of W in a stage: a tile
+constexpr int ROWS = 8;                       // rows of W in a stage
 constexpr int ROW_BYTES = KC * 2;
-constexpr int STAGE_BYTES = TILE * ROW_BYTES;
+constexpr int STAGE_BYTES = ROWS * ROW_BYTES;
+constexpr int TILE = 2 * ROWS;                // rows of W in a product's tile: two stages
 constexpr int BATCH = 4;                      // tiles whose sums meet at once
 constexpr int SLOTS = CT / (TILE * 8);        // of them at a time: a thread an output
 constexpr int TILES = 3;                      // most tiles of a CTA's share of the stream's columns
 constexpr int BX = 3;                         // parts of the contraction whose x is on its way
-constexpr int UNIT = 32;                      // keys a warp takes at a time; a stage holds two such blocks
+constexpr int UNIT = 32;                      // keys in a stage
 constexpr int RUN_BYTES = 16 * DH * 2;        // 16 keys lie in one page
 constexpr int MIN_UNITS = 4;                  // of a part of the keys
 constexpr int MAX_T = STACK_MAX_TOKENS;
-constexpr int MAX_STAGES = 8;
-static_assert(4 * UNIT * DH * 2 <= STAGE_BYTES, "a stage holds 64 keys and values");
+constexpr int MAX_STAGES = 16;
+static_assert(2 * UNIT * DH * 2 <= STAGE_BYTES, "a stage holds 32 keys and values");
 
 struct Shared {
     uint64_t full[MAX_STAGES], empty[MAX_STAGES];
@@ -61,12 +62,9 @@ struct Shared {
     float m[CW][8], l[CW][8];                 // attention: per warp and query head
     alignas(16) uint32_t own_k[DH / 2];       // the token's own key and value
     alignas(16) uint32_t own_v[DH / 2];
-    int own_page[MAX_T];                      // where they go
-    alignas(16) float turn[MAX_T][DH];        // cosines and sines of the tokens' positions
-    alignas(16) float qk_norm[2][DH];         // this layer's
 };
 constexpr int SHARED_BYTES = (sizeof(Shared) + 127) / 128 * 128;
-extern __shared__ __align__(128) unsigned char stack_smem[];    // Shared | layers | scratch | norm | ring
+extern __shared__ __align__(128) unsigned char stack_smem[];    // Shared | layers | scratch | ring
 
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, Shared& sh, int* status) {
 #pragma unroll 1
@@ -95,7 +93,7 @@ struct Ring {
 // c[16 x 8] += a[16 x 16] b[16 x 8]: rows g and g + 8 (a0 a2 and a1 a3) on the left, column g on the right; c[0], c[1]: row g, columns 2t and
 // 2t + 1; c[2], c[3]: row g + 8.
 __device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -159,11 +157,11 @@ struct Producer {
         ok = __shfl_sync(0xffffffffu, (int)got, 0) != 0;
         return ok;
     }
-    // The first sixteen lanes' copies make up a stage.
+    // The first eight lanes' copies make up a stage.
     __device__ __forceinline__ void issue(uint32_t dst, const void* src, uint32_t bytes) {
         uint32_t total = bytes;
 #pragma unroll
-        for (int o = 1; o < 16; o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        for (int o = 1; o < 8; o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
         if (lane == 0) mbar_expect_tx(full + 8 * at.slot, total);
         __syncwarp();
         if (bytes)
@@ -176,19 +174,23 @@ struct Producer {
     __device__ __forceinline__ void rows(const __nv_bfloat16* w, int row, int K, int chunk) {
         if (!mine() || !slot_free()) return;
         const int k = chunk * KC, n = min(KC, K - k);
-        issue(ring + at.slot * STAGE_BYTES + (lane & 15) * ROW_BYTES, w + (int64_t)row * K + k, lane < 16 && row >= 0 ? (uint32_t)n * 2 : 0u);
+        issue(ring + at.slot * STAGE_BYTES + (lane & 7) * ROW_BYTES, w + (int64_t)row * K + k, lane < 8 && row >= 0 ? (uint32_t)n * 2 : 0u);
     }
     // The stages of a product.  by_tile (x stays in registers): all of the contraction for a tile of rows, then the next tile; else all tiles
-    // for a part of the contraction, then the next part.  A tile is sixteen rows or (gated) eight gate rows and their up rows.
+    // for a part of the contraction, then the next part.  A tile is two stages a part of the contraction: eight rows and eight more, or
+    // (gated) eight gate rows and their up rows; the last tile may want the first only.
     __device__ __forceinline__ void product(const __nv_bfloat16* w, int r0, int r1, int K, bool by_tile, bool gated) {
-        const int chunks = (K + KC - 1) / KC, per = gated ? ROWS : TILE, tiles = (r1 - r0 + per - 1) / per, l = lane & (per - 1);
+        const int chunks = (K + KC - 1) / KC, per = gated ? ROWS : TILE, tiles = (r1 - r0 + per - 1) / per, l = lane & 7;
         int tile = 0, chunk = 0;
 #pragma unroll 1
-        for (int i = 0; i < tiles * chunks; ++i) {
-            int row = r0 + tile * per + l;
-            if (row >= r1) row = -1;
-            else if (gated) row = row / 8 * 16 + row % 8 + (lane & 8);   // gate and up rows alternate in runs of 8
-            rows(w, row, K, chunk);
+        for (int i = 0; i < tiles * chunks * 2; ++i) {
+            const int half = i & 1, r = r0 + tile * per + (gated ? 0 : half * ROWS);
+            if (gated || r < r1) {
+                int row = r + l < r1 ? r + l : -1;
+                if (gated && row >= 0) row = row / 8 * 16 + row % 8 + half * 8;   // gate and up rows alternate in runs of 8
+                rows(w, row, K, chunk);
+            }
+            if (!half) continue;
             if (by_tile) {
                 if (++chunk == chunks) chunk = 0, ++tile;
             } else if (++tile == tiles) {
@@ -196,7 +198,7 @@ struct Producer {
             }
         }
     }
-    // Keys and values of this CTA's items, 64 a stage.  A lane looks up the page of one run of 16 keys for eight stages at once.
+    // Keys and values of this CTA's items.  A lane looks up the page of one run of 16 keys for sixteen blocks of 32 at once.
     __device__ __forceinline__ void keys(const StackLayer& L) {
         const int n_items = sh.item0[a.T];
 #pragma unroll 1
@@ -207,20 +209,20 @@ struct Producer {
 #pragma unroll 1
             for (int u0 = it.unit0; u0 < it.unit1; u0 += 16) {
                 const int j_lane = u0 * UNIT + lane * 16;
-                const int page_lane = j_lane <= pos && u0 + (lane >> 1) < it.unit1 ? bt[(unsigned)j_lane / (unsigned)a.page_size] : -1;
-                const int last = min(u0 + 16, it.unit1);
+                const int page_lane = j_lane <= pos && u0 + (lane >> 1) < it.unit1 ? bt[j_lane / a.page_size] : -1;
 #pragma unroll 1
-                for (int u = u0; u < last; u += 2) {
-                    const int run = lane & 3, j = u * UNIT + run * 16;
+                for (int u = u0; u < min(u0 + 16, it.unit1); ++u) {
+                    const int run = lane & 1;
+                    const int j = u * UNIT + run * 16;
                     const int page = __shfl_sync(0xffffffffu, page_lane, (u - u0) * 2 + run);
-                    const bool wanted = j <= pos && u + (run >> 1) < last, good = wanted && page >= 0 && page < a.num_pages;
+                    const bool wanted = j <= pos, good = wanted && page >= 0 && page < a.num_pages;
                     if (!mine()) continue;
-                    if (wanted && !good && lane < 4) imp_report(a.status, IMP_BAD_PAGE);
+                    if (wanted && !good && lane < 2) imp_report(a.status, IMP_BAD_PAGE);
                     if (!slot_free()) return;
-                    const int64_t off = (((int64_t)page * a.hkv + it.kvh) * a.page_size + (unsigned)j % (unsigned)a.page_size) * DH;
-                    const bool value = lane & 4;
-                    issue(ring + at.slot * STAGE_BYTES + (value ? 4 * RUN_BYTES : 0) + run * RUN_BYTES,
-                          (const __nv_bfloat16*)(value ? L.v_pages : L.k_pages) + off, lane < 8 && good ? (uint32_t)RUN_BYTES : 0u);
+                    const int64_t off = (((int64_t)page * a.hkv + it.kvh) * a.page_size + j % a.page_size) * DH;
+                    const bool value = lane & 2;
+                    issue(ring + at.slot * STAGE_BYTES + (value ? 2 * RUN_BYTES : 0) + run * RUN_BYTES,
+                          (const __nv_bfloat16*)(value ? L.v_pages : L.k_pages) + off, lane < 4 && good ? (uint32_t)RUN_BYTES : 0u);
                 }
             }
         }
@@ -242,12 +244,9 @@ struct Consumer {
     Shared& sh;
     float* scratch;        // partial sums of the warps; of attention: their outputs
     unsigned char* ring_mem;
-    uint4* norm_s;         // the next norm's weights
     uint32_t full, empty;
     int tid, lane, warp, g, t;
     Ring at;
-    mutable uint32_t own_raw[2];
-    mutable uint2 own_val;
 
     // Hides from the compiler that these are the same in every phase: it would keep what all phases work out from them in registers throughout.
     __device__ __forceinline__ void forget() { asm volatile("" : "+r"(tid), "+r"(lane), "+r"(warp), "+r"(g), "+r"(t)); }
@@ -264,39 +263,33 @@ struct Consumer {
         const uint4 a0 = reinterpret_cast<const uint4*>(p)[odd], a1 = reinterpret_cast<const uint4*>(p)[!odd];
         u0 = odd ? a1 : a0, u1 = odd ? a0 : a1;
     }
-    // The warp's part of a stage, in registers: rows g (u) and g + 8 (v), two 64s of the contraction.  The stage is given back at once.
-    struct Tile {
-        uint4 u[4], v[4];
-    };
-    __device__ __forceinline__ void fetch(Tile& f, bool second) {
-        const unsigned char* mine = ring_mem + at.slot * STAGE_BYTES + g * ROW_BYTES + warp * (KW * 2) + t * 32;
+    // A tile's two stages (or its only one): the warp's part of the contraction for sixteen rows.  x: elements 16 t ... 16 t + 15 of
+    // token g's 64 and the next 64, two a register.  Not `live`: the contraction ends before this warp's part, where the stage holds
+    // what it held before.
+    __device__ __forceinline__ void tile_mma(float (&c0)[4], float (&c1)[4], const uint32_t (&x)[16], bool second, int live) {
+        const unsigned char* mine = ring_mem + g * ROW_BYTES + warp * (KW * 2) + t * 32;
+        const int slot0 = at.slot;
         wait_stage();
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            fragment(f.u[2 * i], f.u[2 * i + 1], mine + 128 * i);
-            if (second) fragment(f.v[2 * i], f.v[2 * i + 1], mine + ROWS * ROW_BYTES + 128 * i);
-            else f.v[2 * i] = f.v[2 * i + 1] = make_uint4(0u, 0u, 0u, 0u);
-        }
-        release();
-    }
-    // x: elements 16 t ... 16 t + 15 of token g's 64 and of the next 64, two a register.  `live`: how many of the warp's two 64s there are;
-    // beyond the contraction's end a stage holds what it held before.
-    __device__ __forceinline__ void multiply(float (&c0)[4], float (&c1)[4], const Tile& f, const uint32_t (&x)[16], int live) const {
+        at.next(a.n_stages);
+        const int slot1 = at.slot;
+        if (second) wait_stage();
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             if (i >= live) break;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const uint4 u = f.u[2 * i + j], v = f.v[2 * i + j];
-                mma(c0, u.x, v.x, u.y, v.y, x[8 * i + 4 * j], x[8 * i + 4 * j + 1]);
-                mma(c1, u.z, v.z, u.w, v.w, x[8 * i + 4 * j + 2], x[8 * i + 4 * j + 3]);
-            }
+            uint4 u0, u1, v0 = make_uint4(0u, 0u, 0u, 0u), v1 = v0;
+            fragment(u0, u1, mine + slot0 * STAGE_BYTES + 128 * i);
+            if (second) fragment(v0, v1, mine + slot1 * STAGE_BYTES + 128 * i);
+            mma(c0, u0.x, v0.x, u0.y, v0.y, x[8 * i], x[8 * i + 1]);
+            mma(c1, u0.z, v0.z, u0.w, v0.w, x[8 * i + 2], x[8 * i + 3]);
+            mma(c0, u1.x, v1.x, u1.y, v1.y, x[8 * i + 4], x[8 * i + 5]);
+            mma(c1, u1.z, v1.z, u1.w, v1.w, x[8 * i + 6], x[8 * i + 7]);
         }
-    }
-    // One tile, and the next one into the same registers: its wait and its way from shared memory run beside the tensor operations.
-    __device__ __forceinline__ void tile_mma(float (&c0)[4], float (&c1)[4], Tile& f, const uint32_t (&x)[16], int live, bool more, bool second) {
-        multiply(c0, c1, f, x, live);
-        if (more) fetch(f, second);
+        __syncwarp();
+        if (lane == 0) {
+            mbar_arrive(empty + 8 * slot0);
+            if (second) mbar_arrive(empty + 8 * slot1);
+        }
+        if (second) at.next(a.n_stages);
     }
     __device__ __forceinline__ int live(int chunk, int K) const { return (K - chunk * KC - warp * KW) / 64; }   // 64s of the warp's part there are
     // Sums of a tile: [row][token].
@@ -329,73 +322,56 @@ struct Consumer {
             x[8 * i] = u.x, x[8 * i + 1] = u.y, x[8 * i + 2] = u.z, x[8 * i + 3] = u.w, x[8 * i + 4] = v.x, x[8 * i + 5] = v.y, x[8 * i + 6] = v.z, x[8 * i + 7] = v.w;
         }
     }
-    // The norm's weights into shared memory, before the barrier behind which the stream is ready.
-    __device__ __forceinline__ void load_norm(const void* src) const {
-#pragma unroll 1
-        for (int i = tid; i < a.d / 8; i += CT) norm_s[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
-    }
     // x = rmsnorm(h) * w, from the shares of the sums of squares.  The stream is asked for before the sums are there.
     template <int XS>
-    __device__ __forceinline__ void norm_x(uint32_t (&x)[XS][16], float eps) {
-        constexpr int AHEAD = XS < 2 ? XS : 2;       // parts on their way at a time
+    __device__ __forceinline__ void norm_x(uint32_t (&x)[XS][16], const float* w, float eps) {
         float s = 0.f;
-        if (warp < a.T) {
+        if (warp < a.T)
+#pragma unroll 1
+            for (int i = lane; i < (int)gridDim.x; i += 32) s += __ldcg(a.ss + warp * STACK_SS_STRIDE + i);
 #pragma unroll
-            for (int i = 0; i < STACK_SS_STRIDE / 32; ++i)
-                if (lane + 32 * i < (int)gridDim.x) s += __ldcg(a.ss + warp * STACK_SS_STRIDE + lane + 32 * i);
-        }
+        for (int c = 0; c < XS; ++c) {
+            float4 v[8];
 #pragma unroll
-        for (int c0 = 0; c0 < XS; c0 += AHEAD) {
-            float4 v[AHEAD][8];
-#pragma unroll
-            for (int c = 0; c < AHEAD; ++c)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int k = (c0 + c) * KC + warp * KW + 64 * (j / 4);
-                    v[c][j] = g < a.T && k < a.d ? __ldcg(reinterpret_cast<const float4*>(a.h + g * a.d + k + 16 * t) + j % 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            if (c0 == 0) {
+            for (int j = 0; j < 8; ++j) {
+                const int k = c * KC + warp * KW + 64 * (j / 4);
+                v[j] = g < a.T && k < a.d ? __ldcg(reinterpret_cast<const float4*>(a.h + g * a.d + k + 16 * t) + j % 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            if (c == 0) {
                 s = warp_sum(s);
                 if (lane == 0 && warp < a.T) sh.inv[warp] = rsqrtf(s / (float)a.d + eps);
                 consumers_sync();
             }
             const float inv = g < a.T ? sh.inv[g] : 0.f;
 #pragma unroll
-            for (int c = 0; c < AHEAD; ++c)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int k = (c0 + c) * KC + warp * KW + 64 * (j / 4);
-                    const uint4 q = k < a.d ? norm_s[(k + 16 * t) / 8 + j / 2 % 2] : make_uint4(0u, 0u, 0u, 0u);
-                    const float2 w0 = unpack(j % 2 ? q.z : q.x), w1 = unpack(j % 2 ? q.w : q.y);
-                    x[c0 + c][2 * j] = pack(v[c][j].x * inv * w0.x, v[c][j].y * inv * w0.y);
-                    x[c0 + c][2 * j + 1] = pack(v[c][j].z * inv * w1.x, v[c][j].w * inv * w1.y);
-                }
+            for (int j = 0; j < 8; ++j) {
+                const int k = c * KC + warp * KW + 64 * (j / 4);
+                float4 wv = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (g < a.T && k < a.d) wv = __ldg(reinterpret_cast<const float4*>(w + k + 16 * t) + j % 4);
+                x[c][2 * j] = pack(v[j].x * inv * wv.x, v[j].y * inv * wv.y);
+                x[c][2 * j + 1] = pack(v[j].z * inv * wv.z, v[j].w * inv * wv.w);
+            }
         }
     }
 
     // Phases 1 and 4.
     template <int XS>
-    __device__ __forceinline__ void normed_product(float eps, int r0, int r1, bool gated, __nv_bfloat16* out, int ld) {
+    __device__ __forceinline__ void normed_product(const float* norm_w, float eps, int r0, int r1, bool gated, __nv_bfloat16* out, int ld) {
         forget();
         uint32_t x[XS][16];
-        norm_x(x, eps);
+        norm_x(x, norm_w, eps);
         const int per = gated ? ROWS : TILE, n_tiles = (r1 - r0 + per - 1) / per, chunks = (a.d + KC - 1) / KC;
         const int slot = tid / (TILE * MAX_T), e = tid % (TILE * MAX_T), tok = e % MAX_T, j = e / MAX_T;
-        auto second = [&](int tile) { return gated || r0 + tile * TILE + ROWS < r1; };   // rows in the tile's lower half
-        Tile f;
-        if (n_tiles > 0) fetch(f, second(0));
 #pragma unroll 1
         for (int b = 0; b < n_tiles; b += BATCH) {
             const int n = min(BATCH, n_tiles - b);
 #pragma unroll 1
             for (int i = 0; i < n; ++i) {
                 float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+                const bool second = gated || r0 + (b + i) * TILE + ROWS < r1;
 #pragma unroll
                 for (int c = 0; c < XS; ++c)
-                    if (c < chunks) {
-                        const bool end = c + 1 == chunks;
-                        tile_mma(c0, c1, f, x[c], live(c, a.d), !end || b + i + 1 < n_tiles, second(b + i + end));
-                    }
+                    if (c < chunks) tile_mma(c0, c1, x[c], second, live(c, a.d));
                 put_sums(i, c0, c1);
             }
             consumers_sync();
@@ -427,17 +403,11 @@ struct Consumer {
         float c[TILES][4];
 #pragma unroll
         for (int i = 0; i < TILES; ++i) c[i][0] = c[i][1] = c[i][2] = c[i][3] = 0.f;
-        auto second = [&](int tile) { return r0 + tile * TILE + ROWS < r1; };
-        Tile f;
-        if (n_tiles > 0) fetch(f, second(0));
 #pragma unroll 1
         for (int k = 0; k < chunks; ++k) {
 #pragma unroll
             for (int i = 0; i < TILES; ++i)
-                if (i < n_tiles) {
-                    const bool end = i + 1 == n_tiles;
-                    tile_mma(c[i], c[i], f, x[0], live(k, K), !end || k + 1 < chunks, second(end ? 0 : i + 1));
-                }
+                if (i < n_tiles) tile_mma(c[i], c[i], x[0], r0 + i * TILE + ROWS < r1, live(k, K));
 #pragma unroll
             for (int b = 0; b + 1 < BX; ++b)
 #pragma unroll
@@ -484,8 +454,6 @@ struct Consumer {
         put_squares(sq);
     }
 
-    // Which of the first blocks of 32 keys a warp takes: stages go to the pairs of warps 0, 3, 2, 1 in turn.
-    __device__ static __forceinline__ int place_of(int warp) { return (CW / 2 - (warp >> 1)) % (CW / 2) * 2 + (warp & 1); }
     // Phase 2.
     __device__ __forceinline__ void attention(const StackLayer& L) {
         forget();
@@ -495,51 +463,50 @@ struct Consumer {
             const Item it = item_of(sh, item, a.T);
             const int pos = sh.pos[it.tok], n_units = it.unit1 - it.unit0, n_warps = min(CW, n_units);
             const __nv_bfloat16* row = a.qkv + (int64_t)it.tok * qkv_ld;
-            const float *cs = sh.turn[it.tok], *sn = cs + DH / 2;
+            const float* cs = a.cos_tab + (int64_t)pos * (DH / 2);
+            const float* sn = a.sin_tab + (int64_t)pos * (DH / 2);
             uint32_t q[4][4];         // block b: dimensions 32 b + 8 t ... + 7 of head g
             float o[8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // heads 2 t and 2 t + 1
-            const bool used = place_of(warp) < n_units;
-            const bool own = it.part == it.parts - 1 && (n_units - 1) % CW == place_of(warp);   // the last block holds the token's own key
-            if (used) {
-                if (own) ask_own(row, it);
-                load_q(q, row + (int64_t)(it.kvh * G + g) * DH, g < G, L.q_norm ? sh.qk_norm[0] : nullptr, cs, sn);
-                if (own) make_own(it, pos, L, cs, sn);
+            const bool own = it.part == it.parts - 1 && (n_units - 1) % CW == warp;   // the last block holds the token's own key
+            if (warp < n_warps) {
+                load_q(q, row + (int64_t)(it.kvh * G + g) * DH, g < G, L.q_norm, cs, sn);
+                if (own) make_own(row, it, pos, L, cs, sn);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
             }
 #pragma unroll 1
-            for (int u = 0; u < n_units; u += 2) {
+            for (int u = 0; u < n_units; ++u) {
                 wait_stage();
-                const int b = warp & 1;          // the warp's block of the stage
-                if ((u / 2 + (warp >> 1)) % (CW / 2) == 0 && u + b < n_units) {
-                    unsigned char* ksm = ring_mem + at.slot * STAGE_BYTES + b * 2 * RUN_BYTES;
-                    unsigned char* vsm = ksm + 4 * RUN_BYTES;
-                    const int j0 = (it.unit0 + u + b) * UNIT;
-                    if (own && u + b == n_units - 1) {
-                        const int r = pos - j0;
-                        reinterpret_cast<uint2*>(ksm + r * DH * 2)[lane] = reinterpret_cast<const uint2*>(sh.own_k)[lane];
-                        reinterpret_cast<uint2*>(vsm + r * DH * 2)[lane] = reinterpret_cast<const uint2*>(sh.own_v)[lane];
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // a copy refills the stage later
-                        __syncwarp();
-                    }
-                    keys32(q, o, m, l, ksm, vsm, j0, pos);
+                if (u % CW != warp) {    // passed by all the same: a stage is refilled when every warp has seen it
+                    release();
+                    continue;
                 }
-                release();      // every warp passes every stage
+                unsigned char* ksm = ring_mem + at.slot * STAGE_BYTES;
+                unsigned char* vsm = ksm + 2 * RUN_BYTES;
+                const int j0 = (it.unit0 + u) * UNIT;
+                if (own && u == n_units - 1) {
+                    const int r = pos - j0;
+                    reinterpret_cast<uint2*>(ksm + r * DH * 2)[lane] = reinterpret_cast<const uint2*>(sh.own_k)[lane];
+                    reinterpret_cast<uint2*>(vsm + r * DH * 2)[lane] = reinterpret_cast<const uint2*>(sh.own_v)[lane];
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // a copy refills the stage later
+                    __syncwarp();
+                }
+                keys32(q, o, m, l, ksm, vsm, j0, pos);
+                release();
             }
-            if (used) {
-                const int place = place_of(warp);
+            if (warp < n_warps) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
 #pragma unroll
                     for (int x = 4; x < 32; x <<= 1) l[h] += __shfl_xor_sync(0xffffffffu, l[h], x);
                     if (2 * t + h >= G) continue;
-                    float* dst = scratch + (place * G + 2 * t + h) * DH + 8 * g;     // [place][head][DH]
+                    float* dst = scratch + (warp * G + 2 * t + h) * DH + 8 * g;     // [warp][head][DH]
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
                         *reinterpret_cast<float4*>(dst + 64 * b) = make_float4(o[4 * b][h], o[4 * b][2 + h], o[4 * b + 1][h], o[4 * b + 1][2 + h]);
                         *reinterpret_cast<float4*>(dst + 64 * b + 4) = make_float4(o[4 * b + 2][h], o[4 * b + 2][2 + h], o[4 * b + 3][h], o[4 * b + 3][2 + h]);
                     }
-                    if (g == 0) sh.m[place][2 * t + h] = m[h], sh.l[place][2 * t + h] = l[h];
+                    if (g == 0) sh.m[warp][2 * t + h] = m[h], sh.l[warp][2 * t + h] = l[h];
                 }
             }
             consumers_sync();
@@ -575,11 +542,11 @@ struct Consumer {
         consumers_sync();
         if (tid == 0) {
             unsigned* count = a.sync + 2 + it.tok * a.hkv + it.kvh;
-            unsigned before;
-            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(count) : "memory");
-            const bool last = before == (unsigned)it.parts - 1;
+            __threadfence();
+            const bool last = atomicAdd(count, 1u) == (unsigned)it.parts - 1;
             sh.last = last;
             if (last) *reinterpret_cast<volatile unsigned*>(count) = 0u;
+            __threadfence();
         }
         consumers_sync();
         if (!sh.last) return;
@@ -589,25 +556,25 @@ struct Consumer {
             const int h = e / DH;
             float M = -INFINITY, s = 0.f, L = 0.f;
 #pragma unroll 1
-            for (int p0 = 0; p0 < it.parts; p0 += 4) {     // four parts on their way at a time, added in part order
-                float2 ml[4];
-                float v[4];
+            for (int p0 = 0; p0 < it.parts; p0 += 8) {     // eight parts on their way at a time, added in part order
+                float2 ml[8];
+                float v[8];
 #pragma unroll
-                for (int p = 0; p < 4; ++p)
+                for (int p = 0; p < 8; ++p)
                     if (p0 + p < it.parts) {
                         ml[p] = __ldcg(reinterpret_cast<const float2*>(a.part_ml) + (int64_t)(first + p0 + p) * G + h);
                         v[p] = __ldcg(a.part_o + (int64_t)(first + p0 + p) * G * DH + e);
                     }
                 float top = M;
 #pragma unroll
-                for (int p = 0; p < 4; ++p)
+                for (int p = 0; p < 8; ++p)
                     if (p0 + p < it.parts) top = fmaxf(top, ml[p].x);
                 const float f0 = exp2f(M - top);
                 s *= f0;
                 L *= f0;
                 M = top;
 #pragma unroll
-                for (int p = 0; p < 4; ++p)
+                for (int p = 0; p < 8; ++p)
                     if (p0 + p < it.parts) {
                         const float f = exp2f(ml[p].x - M);
                         s += v[p] * f;
@@ -636,7 +603,7 @@ struct Consumer {
             for (int b = 0; b < 4; ++b)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float2 w = *reinterpret_cast<const float2*>(norm_w + 32 * b + 8 * t + 2 * j);
+                    const float2 w = __ldg(reinterpret_cast<const float2*>(norm_w + 32 * b + 8 * t + 2 * j));
                     v[b][j].x = v[b][j].x * inv * w.x;
                     v[b][j].y = v[b][j].y * inv * w.y;
                 }
@@ -645,38 +612,34 @@ struct Consumer {
         for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float2 c = *reinterpret_cast<const float2*>(cs + 32 * b + 8 * t + 2 * j), s = *reinterpret_cast<const float2*>(sn + 32 * b + 8 * t + 2 * j);
+                const float2 c = __ldg(reinterpret_cast<const float2*>(cs + 32 * b + 8 * t + 2 * j)), s = __ldg(reinterpret_cast<const float2*>(sn + 32 * b + 8 * t + 2 * j));
                 const float2 x = v[b][j], y = v[b + 2][j];
                 qa[b][j] = pack(x.x * c.x - y.x * s.x, x.y * c.y - y.y * s.y);
                 qa[b + 2][j] = pack(x.x * s.x + y.x * c.x, x.y * s.y + y.y * c.y);
             }
     }
-    // The token's key and value on their way while q is made.
-    __device__ __forceinline__ void ask_own(const __nv_bfloat16* row, const Item& it) const {
-        const __nv_bfloat16* k = row + (int64_t)(a.hq + it.kvh) * DH;
-        own_raw[0] = __ldcg(reinterpret_cast<const uint32_t*>(k) + lane), own_raw[1] = __ldcg(reinterpret_cast<const uint32_t*>(k + DH / 2) + lane);
-        own_val = __ldcg(reinterpret_cast<const uint2*>(k + (int64_t)a.hkv * DH) + lane);
-    }
     // The token's own key and value, written to their page and kept for the copy in shared memory.
-    __device__ __forceinline__ void make_own(const Item& it, int pos, const StackLayer& L, const float* cs, const float* sn) const {
-        float2 x = unpack(own_raw[0]), y = unpack(own_raw[1]);
-        const uint2 val = own_val;
+    __device__ __forceinline__ void make_own(const __nv_bfloat16* row, const Item& it, int pos, const StackLayer& L, const float* cs, const float* sn) const {
+        const __nv_bfloat16* k = row + (int64_t)(a.hq + it.kvh) * DH;
+        const __nv_bfloat16* v = k + (int64_t)a.hkv * DH;
+        float2 x = unpack(__ldcg(reinterpret_cast<const uint32_t*>(k) + lane)), y = unpack(__ldcg(reinterpret_cast<const uint32_t*>(k + DH / 2) + lane));
+        const uint2 val = __ldcg(reinterpret_cast<const uint2*>(v) + lane);
         const float ss = warp_sum(x.x * x.x + x.y * x.y + y.x * y.x + y.y * y.y);
         if (L.k_norm) {
             const float inv = rsqrtf(ss / (float)DH + a.qk_eps);
-            const float2 w0 = reinterpret_cast<const float2*>(sh.qk_norm[1])[lane], w1 = reinterpret_cast<const float2*>(sh.qk_norm[1] + DH / 2)[lane];
+            const float2 w0 = __ldg(reinterpret_cast<const float2*>(L.k_norm) + lane), w1 = __ldg(reinterpret_cast<const float2*>(L.k_norm + DH / 2) + lane);
             x.x = x.x * inv * w0.x, x.y = x.y * inv * w0.y;
             y.x = y.x * inv * w1.x, y.y = y.y * inv * w1.y;
         }
-        const float2 c = reinterpret_cast<const float2*>(cs)[lane], s = reinterpret_cast<const float2*>(sn)[lane];
+        const float2 c = __ldg(reinterpret_cast<const float2*>(cs) + lane), s = __ldg(reinterpret_cast<const float2*>(sn) + lane);
         const uint32_t lo = pack(x.x * c.x - y.x * s.x, x.y * c.y - y.y * s.y), hi = pack(x.x * s.x + y.x * c.x, x.y * s.y + y.y * c.y);
         sh.own_k[lane] = lo;
         sh.own_k[32 + lane] = hi;
         reinterpret_cast<uint2*>(sh.own_v)[lane] = val;
         __syncwarp();
-        const int page = sh.own_page[it.tok];
+        const int page = a.block_table[(int64_t)sh.seq[it.tok] * a.bt_stride + pos / a.page_size];
         if (page < 0 || page >= a.num_pages) return;   // the producer reports it
-        const int64_t off = (((int64_t)page * a.hkv + it.kvh) * a.page_size + (unsigned)pos % (unsigned)a.page_size) * DH;
+        const int64_t off = (((int64_t)page * a.hkv + it.kvh) * a.page_size + pos % a.page_size) * DH;
         reinterpret_cast<uint32_t*>((__nv_bfloat16*)L.k_pages + off)[lane] = lo;
         reinterpret_cast<uint32_t*>((__nv_bfloat16*)L.k_pages + off + DH / 2)[lane] = hi;
         reinterpret_cast<uint2*>((__nv_bfloat16*)L.v_pages + off)[lane] = val;
@@ -758,18 +721,16 @@ struct Consumer {
     }
 };
 
-// Everybody's stores before, everybody's loads after.  All consumer threads call it.  A CTA says in a word of its own how many barriers it has
-// reached, and a thread a CTA waits for that word: the arrivals do not queue at one address.
-__device__ __forceinline__ void grid_sync(const StackArgs& a, Shared& sh, unsigned reached) {
+// Everybody's stores before, everybody's loads after.  All consumer threads call it; `target`: arrivals of all CTAs so far and at this one.
+__device__ __forceinline__ void grid_sync(const StackArgs& a, Shared& sh, unsigned target) {
     consumers_sync();
-    unsigned* flags = a.sync + 2 + a.T * a.hkv;
-    if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + blockIdx.x), "r"(reached) : "memory");
-    if (threadIdx.x < gridDim.x) {
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.sync) : "memory");
 #pragma unroll 1
         for (uint32_t i = 0;; ++i) {
             unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flags + threadIdx.x) : "memory");
-            if (v >= reached || sh.dead) break;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.sync) : "memory");
+            if (v >= target || sh.dead) break;
             if (i == TC_WAIT_LIMIT) {
                 sh.dead = 1;
                 imp_report(a.status, IMP_WAIT_TIMEOUT);
@@ -778,6 +739,12 @@ __device__ __forceinline__ void grid_sync(const StackArgs& a, Shared& sh, unsign
         }
     }
     consumers_sync();
+}
+
+// A line of a small vector that everybody reads two phases from now: asked into the L2 by one CTA.
+__device__ __forceinline__ void ask(const float* p, int n, int tid) {
+    if (p && tid == 0 && (int)blockIdx.x * 32 < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + blockIdx.x * 32));
+    if (p && tid == 32 && (int)(blockIdx.x + gridDim.x) * 32 < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (blockIdx.x + gridDim.x) * 32));
 }
 
 template <int XS>
@@ -816,12 +783,6 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         }
     }
     if (!good) return;
-    if (tid < a.T) sh.own_page[tid] = a.block_table[(int64_t)sh.seq[tid] * a.bt_stride + sh.pos[tid] / a.page_size];
-#pragma unroll 1
-    for (int i = tid; i < a.T * DH; i += THREADS) {
-        const int t = i / DH, e = i % DH;
-        sh.turn[t][e] = e < DH / 2 ? a.cos_tab[(int64_t)sh.pos[t] * (DH / 2) + e] : a.sin_tab[(int64_t)sh.pos[t] * (DH / 2) + e - DH / 2];
-    }
     if (tid == 0) {
         // Parts of the keys: the fewest blocks a part (at least MIN_UNITS) with which the items do not outnumber the CTAs.
         int total = 0, longest = 0;
@@ -868,27 +829,29 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         p.drain();
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
-        Consumer c{a, sh, reinterpret_cast<float*>(stack_smem + a.scratch_at), stack_smem + a.ring_at, reinterpret_cast<uint4*>(stack_smem + a.norm_at), full, empty, tid, lane, warp, lane >> 2, lane & 3};
-        unsigned reached = 0;
+        Consumer c{a, sh, reinterpret_cast<float*>(stack_smem + a.scratch_at), stack_smem + a.ring_at, full, empty, tid, lane, warp, lane >> 2, lane & 3};
+        unsigned arrived = ctas;
         c.first_squares(d0, d1);
-        c.load_norm(layers[0].norm1);
-        grid_sync(a, sh, ++reached);
+        grid_sync(a, sh, arrived);
 #pragma unroll 1
         for (int i = 0; i < a.n_layers * 2; ++i) {       // one copy of each product's code: what a layer runs must stay in the instruction cache
             const StackLayer& L = layers[i >> 1];
             const bool ffn = i & 1;
-            c.normed_product<XS>(ffn ? a.eps2 : a.eps1, ffn ? f0 : qkv0, ffn ? f1 : qkv1, ffn, ffn ? a.hid : a.qkv, ffn ? a.F : qkv);
+            c.normed_product<XS>(ffn ? L.norm2 : L.norm1, ffn ? a.eps2 : a.eps1, ffn ? f0 : qkv0, ffn ? f1 : qkv1, ffn, ffn ? a.hid : a.qkv, ffn ? a.F : qkv);
             if (!ffn) {
-                if (L.q_norm && tid < 2 * DH) sh.qk_norm[tid / DH][tid % DH] = __ldg((tid < DH ? L.q_norm : L.k_norm) + tid % DH);
-                grid_sync(a, sh, ++reached);
+                ask(L.norm2, a.d, tid);
+            } else if (i + 1 < a.n_layers * 2) {
+                ask(layers[(i >> 1) + 1].norm1, a.d, tid);
+                ask(layers[(i >> 1) + 1].q_norm, DH, tid);
+                ask(layers[(i >> 1) + 1].k_norm, DH, tid);
+            }
+            grid_sync(a, sh, arrived += ctas);
+            if (!ffn) {
                 c.attention(L);
+                grid_sync(a, sh, arrived += ctas);
             }
-            grid_sync(a, sh, ++reached);
             c.branch_product(ffn ? a.hid : a.attn, ffn ? a.F : a.hq * DH, d0, d1);
-            if (i + 1 < a.n_layers * 2) {
-                c.load_norm(ffn ? layers[(i >> 1) + 1].norm1 : L.norm2);
-                grid_sync(a, sh, ++reached);
-            }
+            if (i + 1 < a.n_layers * 2) grid_sync(a, sh, arrived += ctas);
         }
     }
     __syncthreads();
@@ -897,7 +860,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         __threadfence();
         if (atomicAdd(a.sync + 1, 1u) == gridDim.x - 1) {
 #pragma unroll 1
-            for (int i = 0; i < 2 + a.T * a.hkv + (int)gridDim.x; ++i) a.sync[i] = 0u;
+            for (int i = 0; i < 2 + a.T * a.hkv; ++i) a.sync[i] = 0u;
             __threadfence();
         }
     }
@@ -946,7 +909,7 @@ IMP_API int imp_decode_stack_items(int T, int hkv) { return T * hkv > stack_ctas
 
 IMP_API int imp_decode_stack_supported(int d, int F, int hq, int hkv, int dh, int page_size, int n_layers) {
     const int ctas = stack_ctas();
-    if (ctas < 1 || ctas > CT || dh != DH || hkv <= 0 || hq % hkv || hq / hkv > 8) return 0;
+    if (ctas < 1 || ctas > STACK_SS_STRIDE || dh != DH || hkv <= 0 || hq % hkv || hq / hkv > 8) return 0;
     if (d <= 0 || d % 64 || d > 6 * KC || F <= 0 || F % 64 || page_size <= 0 || page_size % 16 || n_layers <= 0 || n_layers > STACK_MAX_LAYERS) return 0;
     return (d + ctas - 1) / ctas <= TILES * TILE;
 }
@@ -961,11 +924,10 @@ IMP_API int imp_decode_stack(const StackArgs* args, void* stream) {
     const int G = a.hq / a.hkv;
     const int sums = BATCH * CW * TILE * MAX_T * 4, outputs = CW * G * DH * 4;
     a.scratch_at = (SHARED_BYTES + a.n_layers * (int)sizeof(StackLayer) + 127) / 128 * 128;
-    a.norm_at = a.scratch_at + (sums > outputs ? sums : outputs);
-    a.ring_at = (a.norm_at + a.d * 2 + 127) / 128 * 128;
+    a.ring_at = a.scratch_at + (sums > outputs ? sums : outputs);
     const int fit = (MOST_SMEM - a.ring_at) / STAGE_BYTES;
     a.n_stages = fit < MAX_STAGES ? fit : MAX_STAGES;
-    if (a.n_stages < 3) return IMP_ERR_UNSUPPORTED;
+    if (a.n_stages < 4) return IMP_ERR_UNSUPPORTED;
     const size_t smem = (size_t)a.ring_at + (size_t)a.n_stages * STAGE_BYTES;
     const int xs = (a.d + KC - 1) / KC, ctas = stack_ctas();
     cudaStream_t s = (cudaStream_t)stream;

@@ -4,11 +4,11 @@
 
 constexpr int STACK_MAX_TOKENS = 8;     // columns of one tensor operation
 constexpr int STACK_MAX_LAYERS = 128;
-constexpr int STACK_SS_STRIDE = 256;    // floats between two tokens' shares of the sums of squares: most CTAs
+constexpr int STACK_SS_STRIDE = 256;    // floats between two tokens' shares of the sums of squares
 
 struct StackLayer {
     const void *w_qkv, *w_o, *w_gu, *w_down;      // bfloat16, dense; gate and up rows alternate in runs of 8
-    const void *norm1, *norm2;                    // bfloat16 [d]
+    const float *norm1, *norm2;                   // [d]
     const float *q_norm, *k_norm;                 // [128] or both null
     void *k_pages, *v_pages;                      // bfloat16 [pages, hkv, page_size, 128]
 };
@@ -24,7 +24,7 @@ struct StackArgs {
     void *qkv, *attn, *hid;
 #endif
     float *ss, *part_o, *part_ml;
-    unsigned* sync;             // [2 + T hkv + STACK_SS_STRIDE], zero between launches
+    unsigned* sync;             // [2 + T hkv], zero between launches
     const int *positions, *seq_of_token, *block_table;
     int bt_stride, n_seqs, page_size, num_pages;
     const float *cos_tab, *sin_tab;   // [max_pos, 64]
@@ -33,5 +33,5 @@ struct StackArgs {
     int act;                    // GateAct's kinds, without a bias
     float act_limit;
     int* status;
-    int n_stages, scratch_at, norm_at, ring_at;    // filled in by the launcher
+    int n_stages, scratch_at, ring_at;    // filled in by the launcher
 };

@@ -505,7 +505,7 @@ void DeviceModel::build_stack() {
         const ImpCacheView& v = lc.view;
         if (cache_count_[j] != 1 || !blocks_[(size_t)order_[j]]->stackable(&l)) return;
         if (!lc.paged() || !v.writes || lc.group != layer_caches_[(size_t)cache_first_[0]].group || v.kv_heads != l.hkv || v.head_dim != l.dh) return;
-        for (const Tensor* w : {&l.w_qkv, &l.w_o, &l.w_gu, &l.w_down, &l.norm1, &l.norm2})
+        for (const Tensor* w : {&l.w_qkv, &l.w_o, &l.w_gu, &l.w_down})
             if (w->dtype != BF16 || !contiguous(*w) || (uintptr_t)w->data % 16) return;
         if (!imp_decode_stack_supported((int)cols(l.w_qkv), (int)cols(l.w_down), l.hq, l.hkv, l.dh, v.page_size, (int)order_.size())) return;
         if (rows(l.w_o) != cols(l.w_qkv) || rows(l.w_down) != cols(l.w_qkv) || numel(l.norm1) != cols(l.w_qkv) || numel(l.norm2) != cols(l.w_qkv)) return;
@@ -513,14 +513,24 @@ void DeviceModel::build_stack() {
         if (!stack_.same_constants(l)) return;
         StackLayer d{};
         d.w_qkv = l.w_qkv.data, d.w_o = l.w_o.data, d.w_gu = l.w_gu.data, d.w_down = l.w_down.data;
-        d.norm1 = l.norm1.data, d.norm2 = l.norm2.data;
         d.q_norm = l.q_norm, d.k_norm = l.k_norm;
         d.k_pages = v.k_pages, d.v_pages = v.v_pages;
         layers.push_back(d);
     }
+    if (stack_norms_.empty())
+        for (size_t j = 0; j < order_.size(); ++j) {
+            StackableLayer l;
+            blocks_[(size_t)order_[j]]->stackable(&l);
+            stack_norms_.push_back(to_float32(*rt_, store_, l.norm1));
+            stack_norms_.push_back(to_float32(*rt_, store_, l.norm2));
+        }
+    for (size_t j = 0; j < layers.size(); ++j) {
+        layers[j].norm1 = (const float*)stack_norms_[2 * j].data;
+        layers[j].norm2 = (const float*)stack_norms_[2 * j + 1].data;
+    }
     stack_layers_ = DeviceBuffer(layers.size() * sizeof(StackLayer));
     IMP_CUDA(cudaMemcpy(stack_layers_.data(), layers.data(), layers.size() * sizeof(StackLayer), cudaMemcpyHostToDevice));
-    stack_sync_ = DeviceBuffer((size_t)(2 + STACK_MAX_TOKENS * stack_.hkv + STACK_SS_STRIDE) * 4, true);
+    stack_sync_ = DeviceBuffer((size_t)(2 + STACK_MAX_TOKENS * stack_.hkv) * 4, true);
     IMP_CUDA(cudaStreamSynchronize(rt_->stream));
     stack_on_ = true;
 }

@@ -97,6 +97,7 @@ private:
     // All layers as one launch for steps of a few single tokens, where the model and the device allow it.
     StackableLayer stack_;                       // what its layers share
     DeviceBuffer stack_layers_, stack_sync_;
+    std::vector<Tensor> stack_norms_;            // 32-bit copies of the norms' weights, two a layer
     bool stack_on_ = false;
     std::unique_ptr<Diagnostics> diag_;
 };
