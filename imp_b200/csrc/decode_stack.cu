@@ -67,7 +67,6 @@ constexpr int SHARED_BYTES = (sizeof(Shared) + 127) / 128 * 128;
 extern __shared__ __align__(128) unsigned char stack_smem[];    // Shared | layers | scratch | ring
 
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, Shared& sh, int* status) {
-#pragma unroll 1
     for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) {
         uint32_t done;
         asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
@@ -112,7 +111,7 @@ __device__ __forceinline__ float exp2_fast(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ int share(int n, int cta, int ctas) { return (unsigned)n * (unsigned)cta / (unsigned)ctas; }   // n below 2^22
+__device__ __forceinline__ int share(int n, int cta, int ctas) { return (int)((int64_t)n * cta / ctas); }
 
 // This step's items of attention: item = part of the keys of one (token, kv head).
 struct Item {
@@ -121,14 +120,13 @@ struct Item {
 __device__ __forceinline__ Item item_of(const Shared& sh, int item, int T) {
     Item r;
     r.tok = 0;
-#pragma unroll 1
     while (r.tok + 1 < T && item >= sh.item0[r.tok + 1]) ++r.tok;
     const int i = item - sh.item0[r.tok], n = sh.units[r.tok];
     r.parts = sh.parts[r.tok];
-    r.kvh = (unsigned)i / (unsigned)r.parts;
+    r.kvh = i / r.parts;
     r.part = i - r.kvh * r.parts;
-    r.unit0 = share(n, r.part, r.parts);
-    r.unit1 = share(n, r.part + 1, r.parts);
+    r.unit0 = (int)((int64_t)n * r.part / r.parts);
+    r.unit1 = (int)((int64_t)n * (r.part + 1) / r.parts);
     return r;
 }
 
@@ -176,41 +174,38 @@ struct Producer {
         const int k = chunk * KC, n = min(KC, K - k);
         issue(ring + at.slot * STAGE_BYTES + (lane & 7) * ROW_BYTES, w + (int64_t)row * K + k, lane < 8 && row >= 0 ? (uint32_t)n * 2 : 0u);
     }
-    // The stages of a product.  by_tile (x stays in registers): all of the contraction for a tile of rows, then the next tile; else all tiles
-    // for a part of the contraction, then the next part.  A tile is two stages a part of the contraction: eight rows and eight more, or
-    // (gated) eight gate rows and their up rows; the last tile may want the first only.
-    __device__ __forceinline__ void product(const __nv_bfloat16* w, int r0, int r1, int K, bool by_tile, bool gated) {
-        const int chunks = (K + KC - 1) / KC, per = gated ? ROWS : TILE, tiles = (r1 - r0 + per - 1) / per, l = lane & 7;
-        int tile = 0, chunk = 0;
-#pragma unroll 1
-        for (int i = 0; i < tiles * chunks * 2; ++i) {
-            const int half = i & 1, r = r0 + tile * per + (gated ? 0 : half * ROWS);
-            if (gated || r < r1) {
-                int row = r + l < r1 ? r + l : -1;
-                if (gated && row >= 0) row = row / 8 * 16 + row % 8 + half * 8;   // gate and up rows alternate in runs of 8
-                rows(w, row, K, chunk);
+    // A product whose x stays in registers: all of the contraction for a tile of rows, then the next tile.  A tile is two stages a part
+    // of the contraction: eight rows and eight more, or (gated) eight gate rows and their up rows; the last tile may want the first only.
+    __device__ __forceinline__ void by_tile(const __nv_bfloat16* w, int r0, int r1, int K, bool gated) {
+        const int chunks = (K + KC - 1) / KC, l = lane & 7;
+        for (int r = r0; r < r1; r += gated ? ROWS : TILE)
+            for (int c = 0; c < chunks; ++c) {
+                if (gated) {   // gate and up rows alternate in runs of 8
+                    const int row = r + l < r1 ? (r + l) / 8 * 16 + (r + l) % 8 : -1;
+                    rows(w, row, K, c);
+                    rows(w, row < 0 ? -1 : row + 8, K, c);
+                } else {
+                    rows(w, r + l < r1 ? r + l : -1, K, c);
+                    if (r + ROWS < r1) rows(w, r + ROWS + l < r1 ? r + ROWS + l : -1, K, c);
+                }
             }
-            if (!half) continue;
-            if (by_tile) {
-                if (++chunk == chunks) chunk = 0, ++tile;
-            } else if (++tile == tiles) {
-                tile = 0, ++chunk;
-            }
-        }
+    }
+    // All tiles for a part of the contraction, then the next part.
+    __device__ __forceinline__ void by_chunk(const __nv_bfloat16* w, int r0, int r1, int K) {
+        const int chunks = (K + KC - 1) / KC;
+        for (int c = 0; c < chunks; ++c)
+            for (int r = r0; r < r1; r += ROWS) rows(w, r + (lane & 7) < r1 ? r + (lane & 7) : -1, K, c);
     }
     // Keys and values of this CTA's items.  A lane looks up the page of one run of 16 keys for sixteen blocks of 32 at once.
     __device__ __forceinline__ void keys(const StackLayer& L) {
         const int n_items = sh.item0[a.T];
-#pragma unroll 1
         for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
             const Item it = item_of(sh, item, a.T);
             const int pos = sh.pos[it.tok];
             const int* bt = a.block_table + (int64_t)sh.seq[it.tok] * a.bt_stride;
-#pragma unroll 1
             for (int u0 = it.unit0; u0 < it.unit1; u0 += 16) {
                 const int j_lane = u0 * UNIT + lane * 16;
                 const int page_lane = j_lane <= pos && u0 + (lane >> 1) < it.unit1 ? bt[j_lane / a.page_size] : -1;
-#pragma unroll 1
                 for (int u = u0; u < min(u0 + 16, it.unit1); ++u) {
                     const int run = lane & 1;
                     const int j = u * UNIT + run * 16;
@@ -229,7 +224,6 @@ struct Producer {
     }
     __device__ __forceinline__ void drain() {   // the copies in flight land before the memory is given back
         if (ok || lane != 0) return;
-#pragma unroll 1
         for (int i = 0; i < min(issued, a.n_stages); ++i) {
             if (at.slot == 0) at.phase ^= 1u;
             at.slot = at.slot == 0 ? a.n_stages - 1 : at.slot - 1;
@@ -327,7 +321,6 @@ struct Consumer {
     __device__ __forceinline__ void norm_x(uint32_t (&x)[XS][16], const float* w, float eps) {
         float s = 0.f;
         if (warp < a.T)
-#pragma unroll 1
             for (int i = lane; i < (int)gridDim.x; i += 32) s += __ldcg(a.ss + warp * STACK_SS_STRIDE + i);
 #pragma unroll
         for (int c = 0; c < XS; ++c) {
@@ -362,10 +355,8 @@ struct Consumer {
         norm_x(x, norm_w, eps);
         const int per = gated ? ROWS : TILE, n_tiles = (r1 - r0 + per - 1) / per, chunks = (a.d + KC - 1) / KC;
         const int slot = tid / (TILE * MAX_T), e = tid % (TILE * MAX_T), tok = e % MAX_T, j = e / MAX_T;
-#pragma unroll 1
         for (int b = 0; b < n_tiles; b += BATCH) {
             const int n = min(BATCH, n_tiles - b);
-#pragma unroll 1
             for (int i = 0; i < n; ++i) {
                 float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
                 const bool second = gated || r0 + (b + i) * TILE + ROWS < r1;
@@ -375,7 +366,6 @@ struct Consumer {
                 put_sums(i, c0, c1);
             }
             consumers_sync();
-#pragma unroll 1
             for (int i = slot; i < n; i += SLOTS) {
                 const int r = r0 + (b + i) * per + j;
                 if (j < per && r < r1 && tok < a.T) {
@@ -404,15 +394,15 @@ struct Consumer {
 #pragma unroll
         for (int i = 0; i < TILES; ++i) c[i][0] = c[i][1] = c[i][2] = c[i][3] = 0.f;
 #pragma unroll 1
-        for (int k = 0; k < chunks; ++k) {
+        for (int base = 0; base < chunks; base += BX) {
 #pragma unroll
-            for (int i = 0; i < TILES; ++i)
-                if (i < n_tiles) tile_mma(c[i], c[i], x[0], r0 + i * TILE + ROWS < r1, live(k, K));
+            for (int k = 0; k < BX; ++k) {
+                if (base + k >= chunks) break;
 #pragma unroll
-            for (int b = 0; b + 1 < BX; ++b)
-#pragma unroll
-                for (int i = 0; i < 16; ++i) x[b][i] = x[b + 1][i];
-            if (k + BX < chunks) load_x(x[BX - 1], src, K, k + BX);
+                for (int i = 0; i < TILES; ++i)
+                    if (i < n_tiles) tile_mma(c[i], c[i], x[k], r0 + i * TILE + ROWS < r1, live(base + k, K));
+                if (base + k + BX < chunks) load_x(x[k], src, K, base + k + BX);
+            }
         }
         const float none[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -446,7 +436,6 @@ struct Consumer {
     __device__ __forceinline__ void first_squares(int r0, int r1) {
         const int tok = tid % MAX_T;
         float sq = 0.f;
-#pragma unroll 1
         for (int r = r0 + tid / MAX_T; r < r1 && tok < a.T; r += CT / MAX_T) {
             const float v = __ldcg(a.h + tok * a.d + r);
             sq += v * v;
@@ -458,7 +447,6 @@ struct Consumer {
     __device__ __forceinline__ void attention(const StackLayer& L) {
         forget();
         const int G = a.hq / a.hkv, n_items = sh.item0[a.T], qkv_ld = (a.hq + 2 * a.hkv) * DH;
-#pragma unroll 1
         for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
             const Item it = item_of(sh, item, a.T);
             const int pos = sh.pos[it.tok], n_units = it.unit1 - it.unit0, n_warps = min(CW, n_units);
@@ -474,7 +462,6 @@ struct Consumer {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
             }
-#pragma unroll 1
             for (int u = 0; u < n_units; ++u) {
                 wait_stage();
                 if (u % CW != warp) {    // passed by all the same: a stage is refilled when every warp has seen it
@@ -519,13 +506,10 @@ struct Consumer {
         const int G = a.hq / a.hkv;
         const Item it = item_of(sh, item, a.T);
         __nv_bfloat16* out = a.attn + (int64_t)it.tok * a.hq * DH + (int64_t)it.kvh * G * DH;
-#pragma unroll 1
         for (int e = tid; e < G * DH; e += CT) {
             const int h = e / DH;
             float M = -INFINITY, s = 0.f, L = 0.f;
-#pragma unroll 1
             for (int w = 0; w < n_warps; ++w) M = fmaxf(M, sh.m[w][h]);
-#pragma unroll 1
             for (int w = 0; w < n_warps; ++w) {
                 const float f = exp2f(sh.m[w][h] - M);
                 s += scratch[w * G * DH + e] * f;
@@ -551,11 +535,9 @@ struct Consumer {
         consumers_sync();
         if (!sh.last) return;
         const int first = item - it.part;
-#pragma unroll 1
         for (int e = tid; e < G * DH; e += CT) {
             const int h = e / DH;
             float M = -INFINITY, s = 0.f, L = 0.f;
-#pragma unroll 1
             for (int p0 = 0; p0 < it.parts; p0 += 8) {     // eight parts on their way at a time, added in part order
                 float2 ml[8];
                 float v[8];
@@ -725,8 +707,8 @@ struct Consumer {
 __device__ __forceinline__ void grid_sync(const StackArgs& a, Shared& sh, unsigned target) {
     consumers_sync();
     if (threadIdx.x == 0) {
+        __threadfence();
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.sync) : "memory");
-#pragma unroll 1
         for (uint32_t i = 0;; ++i) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.sync) : "memory");
@@ -737,6 +719,7 @@ __device__ __forceinline__ void grid_sync(const StackArgs& a, Shared& sh, unsign
                 break;
             }
         }
+        __threadfence();
     }
     consumers_sync();
 }
@@ -753,7 +736,6 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     StackLayer* layers = reinterpret_cast<StackLayer*>(stack_smem + SHARED_BYTES);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t full = smem_u32(sh.full), empty = smem_u32(sh.empty);
-#pragma unroll 1
     for (int i = tid; i < a.n_layers * (int)(sizeof(StackLayer) / 8); i += THREADS)
         reinterpret_cast<uint64_t*>(layers)[i] = reinterpret_cast<const uint64_t*>(a.layers)[i];
     if (tid < a.T) {
@@ -762,7 +744,6 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     }
     if (tid == 0) {
         sh.dead = 0;
-#pragma unroll 1
         for (int i = 0; i < a.n_stages; ++i) {
             mbar_init(full + 8 * i, 1);
             mbar_init(empty + 8 * i, CW);
@@ -771,7 +752,6 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     }
     __syncthreads();
     bool good = true;      // the same for everybody
-#pragma unroll 1
     for (int t = 0; t < a.T; ++t) {
         const int p = sh.pos[t], s = sh.seq[t];
         if (s < 0 || s >= a.n_seqs) {
@@ -786,22 +766,18 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     if (tid == 0) {
         // Parts of the keys: the fewest blocks a part (at least MIN_UNITS) with which the items do not outnumber the CTAs.
         int total = 0, longest = 0;
-#pragma unroll 1
         for (int t = 0; t < a.T; ++t) {
             sh.units[t] = sh.pos[t] / UNIT + 1;
             total += sh.units[t];
             longest = max(longest, sh.units[t]);
         }
-        int most = max(MIN_UNITS, (int)(((unsigned)total * a.hkv + gridDim.x - 1) / gridDim.x));
-#pragma unroll 1
+        int most = max(MIN_UNITS, (int)(((int64_t)total * a.hkv + gridDim.x - 1) / gridDim.x));
         for (; most < longest; ++most) {
             int items = 0;
-#pragma unroll 1
             for (int t = 0; t < a.T; ++t) items += (sh.units[t] + most - 1) / most;
             if (items * a.hkv <= (int)gridDim.x) break;
         }
         int items = 0;
-#pragma unroll 1
         for (int t = 0; t < a.T; ++t) {
             sh.item0[t] = items;
             sh.parts[t] = (sh.units[t] + most - 1) / most;
@@ -817,14 +793,13 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     if (warp >= CW) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         Producer p{a, sh, smem_u32(stack_smem + a.ring_at), full, empty, lane, warp - CW};
-#pragma unroll 1
-        for (int i = 0; i < a.n_layers * 4 && p.ok; ++i) {
-            const StackLayer& L = layers[i >> 2];
-            const int which = i & 3;     // q,k,v; output; gate and up; down
-            if (which == 1) p.keys(L);
-            const void* w = which == 0 ? L.w_qkv : which == 1 ? L.w_o : which == 2 ? L.w_gu : L.w_down;
-            p.product((const __nv_bfloat16*)w, which == 0 ? qkv0 : which == 2 ? f0 : d0, which == 0 ? qkv1 : which == 2 ? f1 : d1,
-                      which == 1 ? a.hq * DH : which == 3 ? a.F : a.d, which == 0 || which == 2, which == 2);
+        for (int i = 0; i < a.n_layers && p.ok; ++i) {
+            const StackLayer& L = layers[i];
+            p.by_tile((const __nv_bfloat16*)L.w_qkv, qkv0, qkv1, a.d, false);
+            p.keys(L);
+            p.by_chunk((const __nv_bfloat16*)L.w_o, d0, d1, a.hq * DH);
+            p.by_tile((const __nv_bfloat16*)L.w_gu, f0, f1, a.d, true);
+            p.by_chunk((const __nv_bfloat16*)L.w_down, d0, d1, a.F);
         }
         p.drain();
     } else {
@@ -833,25 +808,24 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
         unsigned arrived = ctas;
         c.first_squares(d0, d1);
         grid_sync(a, sh, arrived);
-#pragma unroll 1
-        for (int i = 0; i < a.n_layers * 2; ++i) {       // one copy of each product's code: what a layer runs must stay in the instruction cache
-            const StackLayer& L = layers[i >> 1];
-            const bool ffn = i & 1;
-            c.normed_product<XS>(ffn ? L.norm2 : L.norm1, ffn ? a.eps2 : a.eps1, ffn ? f0 : qkv0, ffn ? f1 : qkv1, ffn, ffn ? a.hid : a.qkv, ffn ? a.F : qkv);
-            if (!ffn) {
-                ask(L.norm2, a.d, tid);
-            } else if (i + 1 < a.n_layers * 2) {
-                ask(layers[(i >> 1) + 1].norm1, a.d, tid);
-                ask(layers[(i >> 1) + 1].q_norm, DH, tid);
-                ask(layers[(i >> 1) + 1].k_norm, DH, tid);
+        for (int i = 0; i < a.n_layers; ++i) {
+            const StackLayer& L = layers[i];
+            c.normed_product<XS>(L.norm1, a.eps1, qkv0, qkv1, false, a.qkv, qkv);
+            ask(L.norm2, a.d, tid);
+            grid_sync(a, sh, arrived += ctas);
+            c.attention(L);
+            grid_sync(a, sh, arrived += ctas);
+            c.branch_product(a.attn, a.hq * DH, d0, d1);
+            grid_sync(a, sh, arrived += ctas);
+            c.normed_product<XS>(L.norm2, a.eps2, f0, f1, true, a.hid, a.F);
+            if (i + 1 < a.n_layers) {
+                ask(layers[i + 1].norm1, a.d, tid);
+                ask(layers[i + 1].q_norm, DH, tid);
+                ask(layers[i + 1].k_norm, DH, tid);
             }
             grid_sync(a, sh, arrived += ctas);
-            if (!ffn) {
-                c.attention(L);
-                grid_sync(a, sh, arrived += ctas);
-            }
-            c.branch_product(ffn ? a.hid : a.attn, ffn ? a.F : a.hq * DH, d0, d1);
-            if (i + 1 < a.n_layers * 2) grid_sync(a, sh, arrived += ctas);
+            c.branch_product(a.hid, a.F, d0, d1);
+            if (i + 1 < a.n_layers) grid_sync(a, sh, arrived += ctas);
         }
     }
     __syncthreads();
@@ -859,7 +833,6 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     if (tid == 0) {
         __threadfence();
         if (atomicAdd(a.sync + 1, 1u) == gridDim.x - 1) {
-#pragma unroll 1
             for (int i = 0; i < 2 + a.T * a.hkv; ++i) a.sync[i] = 0u;
             __threadfence();
         }
