@@ -3,9 +3,9 @@
 //
 // What bounds it: every weight is read once per step, so the floor is the memory's rate (8B shape: 386 MB a layer, 59 us at
 // 6.54 TB/s).  As seven launches a layer the step ran at 0.57 of that rate with one token: each launch fills and drains its own
-// pipeline, and between two dependent launches the memory idles.  Here one CTA an SM lives through all layers.  Producer warps
-// stream this CTA's share of every matrix (and the cached keys and values it will need) through one ring of shared memory,
-// in the order in which they will be used, and never wait for the other CTAs: what they fetch does not depend on this step's
+// pipeline, and between two dependent launches the memory idles.  Here one CTA an SM lives through all layers.  A producer warp
+// streams this CTA's share of every matrix (and the cached keys and values it will need) through one ring of shared memory,
+// in the order in which they will be used, and never waits for the other CTAs: what it fetches does not depend on this step's
 // activations.  So while the eight consumer warps wait at a grid barrier between two phases, up to 190 KB an SM (28 MB on
 // the device, 4 us of the memory's time) are already on their way.
 //
@@ -24,7 +24,7 @@
 // The warp with the token's own position makes the new key (norm, rotation) and writes key and value to their page.
 //
 // Every wait is bounded: one that runs out reports IMP_WAIT_TIMEOUT and marks the CTA, which then runs through its
-// remaining phases without waiting; the producers stop and wait (bounded) for the copies in flight.
+// remaining phases without waiting; the producer stops and waits (bounded) for its copies in flight.
 #include "tc_common.cuh"
 #include "decode_stack.h"
 
@@ -33,8 +33,7 @@ namespace {
 constexpr int DH = 128;                       // head size
 constexpr int CW = 8;                         // consumer warps
 constexpr int CT = CW * 32;                   // consumer threads
-constexpr int PW = 4;                         // producer warps: a warpgroup
-constexpr int THREADS = CT + PW * 32;
+constexpr int THREADS = CT + 128;             // and a warpgroup of which one warp is the producer
 constexpr int KW = 128;                       // of the contraction a warp and stage
 constexpr int KC = KW * CW;                   // of the contraction in a stage
 constexpr int ROWS = 8;                       // rows of W in a stage
@@ -130,24 +129,16 @@ __device__ __forceinline__ Item item_of(const Shared& sh, int item, int T) {
     return r;
 }
 
-// ------------------------------------------------------------------------------------------------- producers
-// Each walks all stages and fills every fourth: a warp takes over 100 ns for each copy that it asks for, so one alone, at 2 KB a copy, held
-// an SM to 16 GB/s.
+// ------------------------------------------------------------------------------------------------- producer
 struct Producer {
     const StackArgs& a;
     Shared& sh;
     uint32_t ring, full, empty;
-    int lane, which;
+    int lane;
     Ring at;
     int issued = 0;
     bool ok = true;
 
-    __device__ __forceinline__ bool mine() {
-        if (issued % PW == which) return true;
-        at.next(a.n_stages);
-        ++issued;
-        return false;
-    }
     __device__ __forceinline__ bool slot_free() {
         if (!ok) return false;
         bool got = true;
@@ -170,7 +161,7 @@ struct Producer {
     }
     // The lane's row of W (negative: none), part `chunk` of the contraction.
     __device__ __forceinline__ void rows(const __nv_bfloat16* w, int row, int K, int chunk) {
-        if (!mine() || !slot_free()) return;
+        if (!slot_free()) return;
         const int k = chunk * KC, n = min(KC, K - k);
         issue(ring + at.slot * STAGE_BYTES + (lane & 7) * ROW_BYTES, w + (int64_t)row * K + k, lane < 8 && row >= 0 ? (uint32_t)n * 2 : 0u);
     }
@@ -211,7 +202,6 @@ struct Producer {
                     const int j = u * UNIT + run * 16;
                     const int page = __shfl_sync(0xffffffffu, page_lane, (u - u0) * 2 + run);
                     const bool wanted = j <= pos, good = wanted && page >= 0 && page < a.num_pages;
-                    if (!mine()) continue;
                     if (wanted && !good && lane < 2) imp_report(a.status, IMP_BAD_PAGE);
                     if (!slot_free()) return;
                     const int64_t off = (((int64_t)page * a.hkv + it.kvh) * a.page_size + j % a.page_size) * DH;
@@ -792,16 +782,18 @@ __global__ void __launch_bounds__(THREADS, 1) decode_stack_kernel(const __grid_c
     // 384 threads are launched with 168 registers each, 64,512; of these 256 take 224 and 128 keep 56.
     if (warp >= CW) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-        Producer p{a, sh, smem_u32(stack_smem + a.ring_at), full, empty, lane, warp - CW};
-        for (int i = 0; i < a.n_layers && p.ok; ++i) {
-            const StackLayer& L = layers[i];
-            p.by_tile((const __nv_bfloat16*)L.w_qkv, qkv0, qkv1, a.d, false);
-            p.keys(L);
-            p.by_chunk((const __nv_bfloat16*)L.w_o, d0, d1, a.hq * DH);
-            p.by_tile((const __nv_bfloat16*)L.w_gu, f0, f1, a.d, true);
-            p.by_chunk((const __nv_bfloat16*)L.w_down, d0, d1, a.F);
+        if (warp == CW) {
+            Producer p{a, sh, smem_u32(stack_smem + a.ring_at), full, empty, lane};
+            for (int i = 0; i < a.n_layers && p.ok; ++i) {
+                const StackLayer& L = layers[i];
+                p.by_tile((const __nv_bfloat16*)L.w_qkv, qkv0, qkv1, a.d, false);
+                p.keys(L);
+                p.by_chunk((const __nv_bfloat16*)L.w_o, d0, d1, a.hq * DH);
+                p.by_tile((const __nv_bfloat16*)L.w_gu, f0, f1, a.d, true);
+                p.by_chunk((const __nv_bfloat16*)L.w_down, d0, d1, a.F);
+            }
+            p.drain();
         }
-        p.drain();
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
         Consumer c{a, sh, reinterpret_cast<float*>(stack_smem + a.scratch_at), stack_smem + a.ring_at, full, empty, tid, lane, warp, lane >> 2, lane & 3};
