@@ -6,7 +6,6 @@
 #include <stdint.h>
 
 #include "../branch_terms.h"
-#include "../decode_stack.h"
 #include "../qkv_prepare.h"
 
 extern "C" {
@@ -15,12 +14,6 @@ const char* imp_last_error(void);
 const char* imp_status_string(int code);
 int imp_device_arch(void);
 int imp_device_sm_count(void);
-
-// A step of single tokens through all layers in one launch.  `items`: parts of the keys the scratch must hold; `supported`: 1 where the
-// kernel takes these sizes.
-int imp_decode_stack_items(int T, int hkv);
-int imp_decode_stack_supported(int d, int F, int hq, int hkv, int dh, int page_size, int n_layers);
-int imp_decode_stack(const StackArgs* args, void* stream);
 
 int imp_embedding(float* out, const void* table, const int* ids, int n_tokens, int d, int vocab, int table_dtype,
                   float scale, int* status, void* stream);

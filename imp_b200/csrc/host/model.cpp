@@ -483,86 +483,12 @@ void DeviceModel::attach_cache(CacheManager* cache) {
         own += owns ? cache_count_[j] : 1;
     }
     (void)own;
-    build_stack();
     if (embedding_cache_position_ >= 0) {
         embedding_cache_ = LayerCache();
         embedding_cache_.view = cache->layer_view(embedding_cache_position_, rt_->dtype);
         embedding_cache_.view.writes = 1;
         embedding_cache_.group = cache->layer_ref()[(size_t)embedding_cache_position_].group;
     }
-}
-
-// The decode step of a stack of equal pre-norm layers in one launch: see csrc/decode_stack.cu.  With IMP_B200_DECODE_STACK=1.
-void DeviceModel::build_stack() {
-    stack_on_ = false;
-    if (rt_->dtype != BF16 || diag_ || !rt_->time_without.empty() || !rt_->early_weights || keep_embedding_ || order_.empty() ||
-        !env_flag("IMP_B200_DECODE_STACK", false))
-        return;
-    std::vector<StackLayer> layers;
-    for (size_t j = 0; j < order_.size(); ++j) {
-        StackableLayer l;
-        const LayerCache& lc = layer_caches_[(size_t)cache_first_[j]];
-        const ImpCacheView& v = lc.view;
-        if (cache_count_[j] != 1 || !blocks_[(size_t)order_[j]]->stackable(&l)) return;
-        if (!lc.paged() || !v.writes || lc.group != layer_caches_[(size_t)cache_first_[0]].group || v.kv_heads != l.hkv || v.head_dim != l.dh) return;
-        for (const Tensor* w : {&l.w_qkv, &l.w_o, &l.w_gu, &l.w_down})
-            if (w->dtype != BF16 || !contiguous(*w) || (uintptr_t)w->data % 16) return;
-        if (!imp_decode_stack_supported((int)cols(l.w_qkv), (int)cols(l.w_down), l.hq, l.hkv, l.dh, v.page_size, (int)order_.size())) return;
-        if (rows(l.w_o) != cols(l.w_qkv) || rows(l.w_down) != cols(l.w_qkv) || numel(l.norm1) != cols(l.w_qkv) || numel(l.norm2) != cols(l.w_qkv)) return;
-        if (j == 0) stack_ = l;
-        if (!stack_.same_constants(l)) return;
-        StackLayer d{};
-        d.w_qkv = l.w_qkv.data, d.w_o = l.w_o.data, d.w_gu = l.w_gu.data, d.w_down = l.w_down.data;
-        d.q_norm = l.q_norm, d.k_norm = l.k_norm;
-        d.k_pages = v.k_pages, d.v_pages = v.v_pages;
-        layers.push_back(d);
-    }
-    if (stack_norms_.empty())
-        for (size_t j = 0; j < order_.size(); ++j) {
-            StackableLayer l;
-            blocks_[(size_t)order_[j]]->stackable(&l);
-            stack_norms_.push_back(to_float32(*rt_, store_, l.norm1));
-            stack_norms_.push_back(to_float32(*rt_, store_, l.norm2));
-        }
-    for (size_t j = 0; j < layers.size(); ++j) {
-        layers[j].norm1 = (const float*)stack_norms_[2 * j].data;
-        layers[j].norm2 = (const float*)stack_norms_[2 * j + 1].data;
-    }
-    stack_layers_ = DeviceBuffer(layers.size() * sizeof(StackLayer));
-    IMP_CUDA(cudaMemcpy(stack_layers_.data(), layers.data(), layers.size() * sizeof(StackLayer), cudaMemcpyHostToDevice));
-    stack_sync_ = DeviceBuffer((size_t)(2 + STACK_MAX_TOKENS * stack_.hkv) * 4, true);
-    IMP_CUDA(cudaStreamSynchronize(rt_->stream));
-    stack_on_ = true;
-}
-
-bool DeviceModel::forward_stack(Step& st, Tensor h) {
-    const int T = st.T();
-    if (!stack_on_ || !st.decode_only() || T > STACK_MAX_TOKENS || h.dtype != F32 || !contiguous(h)) return false;
-    const StackableLayer& l = stack_;
-    const ImpCacheView& v = layer_caches_[(size_t)cache_first_[0]].view;
-    StackArgs a{};
-    a.layers = (const StackLayer*)stack_layers_.data();
-    a.n_layers = (int)order_.size(), a.T = T, a.d = (int)cols(h), a.F = (int)cols(l.w_down), a.hq = l.hq, a.hkv = l.hkv;
-    a.h = (float*)h.data;
-    a.qkv = rt_->empty(T, (l.hq + 2 * l.hkv) * l.dh).data;
-    a.attn = rt_->empty(T, l.hq * l.dh).data;
-    a.hid = rt_->empty(T, a.F).data;
-    a.ss = (float*)rt_->empty(T, STACK_SS_STRIDE, F32).data;
-    const int64_t items = imp_decode_stack_items(T, l.hkv), group = l.hq / l.hkv;
-    a.part_o = (float*)rt_->empty(items, group * l.dh, F32).data;
-    a.part_ml = (float*)rt_->empty(items, group * 2, F32).data;
-    a.sync = (unsigned*)stack_sync_.data();
-    a.positions = st.view.positions, a.seq_of_token = st.view.seq_of_token, a.block_table = v.block_table;
-    a.bt_stride = v.bt_stride, a.n_seqs = st.B(), a.page_size = v.page_size, a.num_pages = v.num_pages;
-    a.cos_tab = l.rot.cos, a.sin_tab = l.rot.sin, a.max_pos = l.rot.max_pos;
-    a.eps1 = l.eps1, a.eps2 = l.eps2, a.qk_eps = l.qk_eps, a.scale_log2 = l.scale * 1.4426950408889634f;
-    a.act = l.act, a.act_limit = l.act_limit;
-    a.status = rt_->status;
-    const int rc = imp_decode_stack(&a, rt_->stream);
-    if (rc == -2) return false;
-    ++rt_->launches;
-    check_launch(rc, "decode_stack");
-    return true;
 }
 
 Tensor DeviceModel::forward(Step& st) {
@@ -584,8 +510,7 @@ Tensor DeviceModel::forward(Step& st) {
         IMP_CUDA(cudaMemcpyAsync(st.embedding_out.data, h.data, (size_t)numel(h) * elem_size(h.dtype), cudaMemcpyDeviceToDevice, rt_->stream));
     }
     Branch pending;
-    const bool stacked = forward_stack(st, h);
-    for (size_t j = 0; j < order_.size() && !stacked; ++j) {
+    for (size_t j = 0; j < order_.size(); ++j) {
         rt_->arena->next_layer();
         st.layer = order_[j];
         const void* copy_before = st.stream_copy.data;

@@ -76,8 +76,6 @@ public:
 private:
     void build(const std::vector<std::pair<std::string, Tensor>>& placed);
     void finish_build();
-    void build_stack();
-    bool forward_stack(Step& st, Tensor h);
     ModelPlan plan_;
     Runtime* rt_;
     WeightStore store_;
@@ -94,11 +92,6 @@ private:
     std::vector<TilingSpec> tilings_;
     bool graph_safe_ = true, keep_embedding_ = false;
     CacheManager* cache_ = nullptr;
-    // All layers as one launch for steps of a few single tokens, where the model and the device allow it.
-    StackableLayer stack_;                       // what its layers share
-    DeviceBuffer stack_layers_, stack_sync_;
-    std::vector<Tensor> stack_norms_;            // 32-bit copies of the norms' weights, two a layer
-    bool stack_on_ = false;
     std::unique_ptr<Diagnostics> diag_;
 };
 

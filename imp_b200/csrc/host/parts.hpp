@@ -245,25 +245,8 @@ struct FeedForward : Part {
     void call(Step& st, ImpCall& c) override;
 };
 
-// A layer as the one-launch decode step takes it (csrc/decode_stack.cu): rmsnorm, grouped-query attention with rotary positions over
-// the whole head, rmsnorm, gated feed-forward.
-struct StackableLayer {
-    Tensor w_qkv{}, w_o{}, w_gu{}, w_down{}, norm1{}, norm2{};
-    const float *q_norm = nullptr, *k_norm = nullptr;
-    float eps1 = 0, eps2 = 0, qk_eps = 0, scale = 0;
-    int hq = 0, hkv = 0, dh = 0, act = 0;
-    float act_limit = 0;
-    Position::Rotary rot{};
-    bool same_constants(const StackableLayer& o) const {   // what all layers of a launch share
-        return eps1 == o.eps1 && eps2 == o.eps2 && qk_eps == o.qk_eps && scale == o.scale && hq == o.hq && hkv == o.hkv && dh == o.dh && act == o.act &&
-               act_limit == o.act_limit && rot.cos == o.rot.cos && rot.sin == o.rot.sin && rot.max_pos == o.rot.max_pos &&
-               w_qkv.shape[1] == o.w_qkv.shape[1] && w_gu.shape[0] == o.w_gu.shape[0];
-    }
-};
-
 struct Block : Part {
     const char* category() const override { return "block"; }
-    virtual bool stackable(StackableLayer* out) const { (void)out; return false; }   // this block as such a layer, if it is one
     bool defer_pending = false;                          // set by the model: the pending it returns may be unsummed
     virtual bool takes_split_sum() const { return false; }   // the pending it is given may be unsummed
     bool scale_pending = false;                          // set by the model: the pending it returns may carry a col_scale

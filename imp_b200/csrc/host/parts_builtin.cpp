@@ -324,21 +324,6 @@ struct PreNormBlock : Block {
         return {{"mixer_norm", "norm"}, {"mixer", "mixer"}, {"ffn_norm", "norm"}, {"feed_forward", "feed_forward"}};
     }
     bool takes_split_sum() const override { return norm1->takes_split_sum(); }
-    bool stackable(StackableLayer* out) const override {
-        const auto* n1 = dynamic_cast<const RMSNorm*>(norm1);
-        const auto* n2 = dynamic_cast<const RMSNorm*>(norm2);
-        const auto* at = dynamic_cast<const GQAAttention*>(mixer_);
-        const auto* ff = dynamic_cast<const SwiGLU*>(ffn);
-        StackableLayer l;
-        if (!n1 || !n2 || !at || !ff || n1->offset != 0.f || n2->offset != 0.f || at->g.window != 0 || !ff->interleaved || ff->has_bias) return false;
-        if (!at->position || !at->position->rotary(&l.rot) || l.rot.rot_dim != at->g.dh) return false;
-        l.w_qkv = at->w_qkv, l.w_o = at->w_o, l.w_gu = ff->w_gu, l.w_down = ff->w_down, l.norm1 = n1->weight, l.norm2 = n2->weight;
-        if (at->has_norm) l.q_norm = (const float*)at->q_norm_f32.data, l.k_norm = (const float*)at->k_norm_f32.data;
-        l.eps1 = n1->eps, l.eps2 = n2->eps, l.qk_eps = at->norm_eps, l.scale = at->g.scale;
-        l.hq = at->g.hq, l.hkv = at->g.hkv, l.dh = at->g.dh, l.act = ff->act.kind, l.act_limit = ff->act.limit;
-        *out = l;
-        return true;
-    }
     Mixer* mixer() const override { return mixer_; }
     std::vector<Part*> parts() const override { return {norm1, mixer_, norm2, ffn}; }
     bool graph_safe() const override { return norm1->graph_safe() && mixer_->graph_safe() && norm2->graph_safe() && ffn->graph_safe(); }
