@@ -83,6 +83,7 @@ public:
 
 private:
     Tensor forward_decode_graph(Step& st);
+    Tensor capture(Step& st, std::vector<cudaGraphExec_t>* execs);
     void drop_graphs();
     DeviceModel* model_;
     CacheManager* cache_;
@@ -94,7 +95,7 @@ private:
     BatchBuffers buf_;
     Step step_;
     struct Graph {
-        cudaGraphExec_t exec = nullptr;
+        std::vector<cudaGraphExec_t> execs;   // one after the other
         Tensor logits{};
         int64_t launches = 0;
         Arena::Mark mark;    // the workspace's cursors when the capture ended
