@@ -519,7 +519,6 @@ Tensor DeviceModel::forward(Step& st) {
         if (cache_count_[j] == 1 && !lc->view.kind) lc = nullptr;
         pending = blocks_[(size_t)order_[j]]->forward(st, h, pending, lc);
         if (st.stream_copy.data == copy_before) st.stream_copy = Tensor{};   // the block left no copy of its own: the old one is stale
-        if (st.between_layers && j + 1 < order_.size()) st.between_layers();
         if (diag_ && !diag_->dump_dir.empty()) diag_->dump_stream(st, (int)j, h, pending);
     }
     st.layer = -1;

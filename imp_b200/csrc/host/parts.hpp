@@ -112,7 +112,6 @@ struct Step {
     Tensor embedding_out{};                    // a copy of the embedding's output, kept when a block asks for it (Block::wants_embedding)
     Tensor stream_copy{};                      // the stream in the activation type, when the block (or the embedding) that just ran
                                                // left one: its last norm writes it beside the 32-bit stream; else null
-    std::function<void()> between_layers;      // set while a graph is captured: called between two layers, which may go to different graphs
     RowOp* row_op = nullptr;                   // set around one add_norm call by a block that offers its reader's per-row operation
     int context = 0;                           // the sequences' mean length after this step, rounded to a power of two: what
                                                // launch choices may depend on (a decode graph is kept per batch size and context)

@@ -76,7 +76,7 @@ Stepper::~Stepper() { drop_graphs(); }
 
 void Stepper::drop_graphs() {
     for (auto& kv : graphs_)
-        for (auto e : kv.second.execs) cudaGraphExecDestroy(e);
+        if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     graphs_.clear();
     graph_uses_.clear();
 }
@@ -275,58 +275,7 @@ Tensor Stepper::step(const StepEntryView* entries, int n, const int32_t* device_
     return logits;
 }
 
-// Captures a step in up to three graphs, cut between layers.  The device starts a graph when the host has handed over all of it, 0.6 us a
-// launch: as one graph of 200 launches a step's first kernel waited 110 us.  A short first graph is running after 15, and while a graph of
-// n launches runs (3 us each at the least) the host hands over four times as many.  Every further graph costs its own start and the overlap
-// of the two kernels where it was cut.
-constexpr int GRAPH_FIRST = 16, GRAPH_NEXT = 4;   // launches of the first graph, and how many times as many the second has
-Tensor Stepper::capture(Step& st, std::vector<cudaGraphExec_t>* execs) {
-    cudaStream_t s = rt_->stream;
-    int64_t begun = rt_->launches;
-    bool open = false;
-    auto begin = [&] {
-        IMP_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        open = true;
-        begun = rt_->launches;
-    };
-    auto end = [&] {
-        open = false;
-        cudaGraph_t graph = nullptr;
-        IMP_CUDA(cudaStreamEndCapture(s, &graph));
-        cudaGraphExec_t exec = nullptr;
-        const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess) fail(IMP_ERROR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-        execs->push_back(exec);
-    };
-    struct Unset {
-        Step& st;
-        ~Unset() { st.between_layers = nullptr; }
-    } unset{st};
-    try {
-        begin();
-        st.between_layers = [&] {
-            if (execs->size() >= 2 || rt_->launches - begun < GRAPH_FIRST * (execs->empty() ? 1 : GRAPH_NEXT)) return;
-            end();
-            begin();
-        };
-        Tensor logits = model_->forward(st);
-        end();
-        return logits;
-    } catch (...) {
-        if (open) {
-            cudaGraph_t graph = nullptr;
-            cudaStreamEndCapture(s, &graph);
-            if (graph) cudaGraphDestroy(graph);
-        }
-        (void)cudaGetLastError();
-        for (auto e : *execs) cudaGraphExecDestroy(e);
-        execs->clear();
-        throw;
-    }
-}
-
-// Decode-only batches of a given size replay captured CUDA graphs.  The batch arrays live at fixed
+// Decode-only batches of a given size replay one captured CUDA graph.  The batch arrays live at fixed
 // addresses and the workspace hands out the same addresses for the same sequence of requests, so a graph
 // captured for B sequences serves every later step of B sequences; only the arrays' contents change.  The
 // first step of a size runs eagerly (it sizes the workspace and sets kernel attributes), the second is
@@ -345,28 +294,39 @@ Tensor Stepper::forward_decode_graph(Step& st) {
         }
         const uint64_t gen = rt_->arena->generation();
         const int64_t launches_before = rt_->launches;
-        Graph g;
+        cudaGraph_t graph = nullptr;
+        Tensor logits{};
         IMP_CUDA(cudaStreamSynchronize(rt_->stream));
+        IMP_CUDA(cudaStreamBeginCapture(rt_->stream, cudaStreamCaptureModeThreadLocal));
         rt_->arena->freeze(true);
         try {
-            g.logits = capture(st, &g.execs);
+            logits = model_->forward(st);
         } catch (...) {
             rt_->arena->freeze(false);
+            cudaStreamEndCapture(rt_->stream, &graph);
+            if (graph) cudaGraphDestroy(graph);
+            (void)cudaGetLastError();
             graph_uses_[key] = 0;        // try again after an eager step has sized the workspace
             rt_->arena->begin_step(rt_->stream);
             ++eager_steps;
             return model_->forward(st);
         }
         rt_->arena->freeze(false);
+        IMP_CUDA(cudaStreamEndCapture(rt_->stream, &graph));
+        Graph g;
+        g.logits = logits;
         g.mark = rt_->arena->mark();
         g.launches = rt_->launches - launches_before;   // launcher calls the graph stands for
         rt_->launches = launches_before;
+        cudaError_t e = cudaGraphInstantiate(&g.exec, graph, 0);
+        cudaGraphDestroy(graph);
+        if (e != cudaSuccess) fail(IMP_ERROR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
         if (gen != rt_->arena->generation()) fail(IMP_ERROR_INTERNAL, "the workspace moved during graph capture");
         ++graph_captures;
         hit = graphs_.emplace(key, g).first;
     }
     rt_->arena->restore(hit->second.mark);
-    for (auto e : hit->second.execs) IMP_CUDA(cudaGraphLaunch(e, rt_->stream));
+    IMP_CUDA(cudaGraphLaunch(hit->second.exec, rt_->stream));
     rt_->launches += hit->second.launches;
     ++graph_replays;
     return hit->second.logits;

@@ -83,7 +83,6 @@ public:
 
 private:
     Tensor forward_decode_graph(Step& st);
-    Tensor capture(Step& st, std::vector<cudaGraphExec_t>* execs);
     void drop_graphs();
     DeviceModel* model_;
     CacheManager* cache_;
@@ -95,7 +94,7 @@ private:
     BatchBuffers buf_;
     Step step_;
     struct Graph {
-        std::vector<cudaGraphExec_t> execs;   // one after the other
+        cudaGraphExec_t exec = nullptr;
         Tensor logits{};
         int64_t launches = 0;
         Arena::Mark mark;    // the workspace's cursors when the capture ended
