@@ -790,6 +790,35 @@ __device__ __forceinline__ bool dt_wait(uint32_t bar, uint32_t parity, int* stat
     return false;
 }
 
+// The bank conflicts of the stages.  Rows follow one another without padding (a run of 16 comes as one copy), so with DH a multiple of
+// 64 every row starts in the same bank.  Of a key's fragments, the eight lanes of a pass (two keys, four lanes each) asked for 64 bytes of
+// the same banks: odd keys read each pair of 64-byte blocks in the other order, and a pass meets all banks once.  Of the values', they asked for two
+// 16-byte pieces of four rows each: in every second block of 64 dimensions lane g takes the piece g ^ 4 (dim_of_smem), and odd lanes t read that block
+// first: four pieces.  256 -> 160 passes for 16 keys of 128 with the way in.  Which key or dimension meets which register stays, or changes
+// whole columns, so every sum is the same.
+template <bool SWAP> __device__ __forceinline__ void swap_if(uint4& a, uint4& b, bool odd) {
+    if (SWAP) {
+        const uint4 x = odd ? b : a, y = odd ? a : b;
+        a = x, b = y;
+    }
+}
+__device__ __forceinline__ void load_key_frags(uint32_t (&f)[KSTEPS][2], const unsigned char* row, int t, bool odd) {
+    if constexpr (DH % 64 != 0) {
+        load_row_frags(f, reinterpret_cast<const __nv_bfloat16*>(row), t);
+    } else {
+#pragma unroll
+        for (int b = 0; b < DH / 32; b += 2) {
+            uint4 v0 = *reinterpret_cast<const uint4*>(row + b * 64 + (odd ? 64 : 0) + 16 * t), v1 = *reinterpret_cast<const uint4*>(row + b * 64 + (odd ? 0 : 64) + 16 * t);
+            swap_if<true>(v0, v1, odd);
+            f[2 * b][0] = v0.x; f[2 * b][1] = v0.y; f[2 * b + 1][0] = v0.z; f[2 * b + 1][1] = v0.w;
+            f[2 * b + 2][0] = v1.x; f[2 * b + 2][1] = v1.y; f[2 * b + 3][0] = v1.z; f[2 * b + 3][1] = v1.w;
+        }
+    }
+}
+constexpr bool V_PAIRS = DH % 128 == 0;
+// dim_of for what dec_compute_smem accumulated.
+__device__ __forceinline__ int dim_of_smem(int tile, int c) { return dim_of(tile, V_PAIRS && (tile >> 3) % 2 ? c ^ 4 : c); }
+
 // Scores, softmax update and P V for 16 keys whose rows lie at `ksm` / `vsm` (16 rows of DH bfloat16).
 template <int NR>
 __device__ __forceinline__ void dec_compute_smem(DecState<NR>& st, const uint32_t (&qa)[KSTEPS][4], const RowInfo (&rows)[2],
@@ -802,8 +831,8 @@ __device__ __forceinline__ void dec_compute_smem(DecState<NR>& st, const uint32_
     for (int i = 0; i < 2 * NR; ++i) s0[i] = s1[i] = 0.f;
     {
         uint32_t k0[KSTEPS][2], k1[KSTEPS][2];
-        load_row_frags(k0, reinterpret_cast<const __nv_bfloat16*>(ksm + g * RB), t);
-        load_row_frags(k1, reinterpret_cast<const __nv_bfloat16*>(ksm + (g + 8) * RB), t);
+        load_key_frags(k0, ksm + g * RB, t, g & 1);
+        load_key_frags(k1, ksm + (g + 8) * RB, t, g & 1);
 #pragma unroll
         for (int ks = 0; ks < KSTEPS; ++ks) {
             dec_mma<NR>(s0, qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], k0[ks][0], k0[ks][1]);
@@ -846,11 +875,24 @@ __device__ __forceinline__ void dec_compute_smem(DecState<NR>& st, const uint32_
     const uint32_t pa1 = NR == 2 ? pa[0][NR - 1] : 0u, pa3 = NR == 2 ? pa[1][NR - 1] : 0u;
     const unsigned char* vr[4] = {vsm + (2 * t) * RB, vsm + (2 * t + 1) * RB, vsm + (2 * t + 8) * RB, vsm + (2 * t + 9) * RB};
     int tile = 0;
+    uint4 ahead[4];                                  // V_PAIRS: of the pair's second block
 #pragma unroll
     for (int b = 0; b < VBlocks::N64; ++b) {
         uint4 r[4];
+        if (!V_PAIRS || b % 2 == 0) {
+            const bool odd = V_PAIRS && (t & 1);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) r[k] = *reinterpret_cast<const uint4*>(vr[k] + b * 128 + 16 * g);
+            for (int k = 0; k < 4; ++k) {
+                r[k] = *reinterpret_cast<const uint4*>(vr[k] + b * 128 + (odd ? 128 + 16 * (g ^ 4) : 16 * g));
+                if (V_PAIRS) {
+                    ahead[k] = *reinterpret_cast<const uint4*>(vr[k] + b * 128 + (odd ? 16 * g : 128 + 16 * (g ^ 4)));
+                    swap_if<V_PAIRS>(r[k], ahead[k], odd);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) r[k] = ahead[k];
+        }
         const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&r[0]);
         const uint32_t* w1 = reinterpret_cast<const uint32_t*>(&r[1]);
         const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&r[2]);
@@ -1324,16 +1366,16 @@ __global__ void __launch_bounds__((DT_CONSUMERS + 1) * 32) attn_decode_tma_kerne
             __nv_bfloat16* o = out + (int64_t)tok * out_stride + (int64_t)head * DH;
 #pragma unroll
             for (int i = 0; i < NTILES; ++i) {
-                o[dim_of(i, 2 * t4)] = __float2bfloat16_rn(st.o[i][2 * r] * inv);
-                o[dim_of(i, 2 * t4 + 1)] = __float2bfloat16_rn(st.o[i][2 * r + 1] * inv);
+                o[dim_of_smem(i, 2 * t4)] = __float2bfloat16_rn(st.o[i][2 * r] * inv);
+                o[dim_of_smem(i, 2 * t4 + 1)] = __float2bfloat16_rn(st.o[i][2 * r + 1] * inv);
             }
         } else {
             const int64_t slot = ((int64_t)tok * Hq + head) * n_splits + split;
             float* o = part_o + slot * DH;
 #pragma unroll
             for (int i = 0; i < NTILES; ++i) {
-                o[dim_of(i, 2 * t4)] = st.o[i][2 * r];
-                o[dim_of(i, 2 * t4 + 1)] = st.o[i][2 * r + 1];
+                o[dim_of_smem(i, 2 * t4)] = st.o[i][2 * r];
+                o[dim_of_smem(i, 2 * t4 + 1)] = st.o[i][2 * r + 1];
             }
             if (t4 == 0) {
                 part_ml[slot * 2] = st.m[r];
