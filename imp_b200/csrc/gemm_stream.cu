@@ -89,7 +89,8 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
             }
         }
     };
-    // Activation copies: 8*NT rows x 32 chunks, 2*NT per thread; rows past M and columns past K are zeros.
+    // Activation copies: 8*NT rows x 32 chunks, 2*NT per thread, of the M rows there are; columns past K are zeros.  (As zeros in
+    // shared memory the rows past M were a third of all copies at one row.)
     auto issue_a = [&]() {
         if (q_issue < total) {
             const uint32_t sbase = smem_base + (q_issue % STAGES) * STAGE_BYTES + W_BYTES;
@@ -98,8 +99,9 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
                 const int c = tid + i * THREADS;
                 const int row = c >> 5, col = c & 31;
                 const int k = i_stage * GS_STAGE_K + col * 8;
-                const __nv_bfloat16* src = A + (int64_t)min(row, M - 1) * lda + min(k, K - 8);
-                gs_cp_async(sbase + row * GS_ROW_BYTES + col * 16, src, (k + 8 <= K && row < M) ? 16 : 0);
+                if (row >= M) break;
+                const __nv_bfloat16* src = A + (int64_t)row * lda + min(k, K - 8);
+                gs_cp_async(sbase + row * GS_ROW_BYTES + col * 16, src, k + 8 <= K ? 16 : 0);
             }
         }
     };
@@ -145,8 +147,11 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
         const uint4 wb1 = *reinterpret_cast<const uint4*>(wp + (g + 8) * GS_ROW_BYTES + 16);
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-            const uint4 c0 = *reinterpret_cast<const uint4*>(sp + W_BYTES + (8 * nt + g) * GS_ROW_BYTES);
-            const uint4 c1 = *reinterpret_cast<const uint4*>(sp + W_BYTES + (8 * nt + g) * GS_ROW_BYTES + 16);
+            uint4 c0 = make_uint4(0u, 0u, 0u, 0u), c1 = c0;
+            if (8 * nt + g < M) {
+                c0 = *reinterpret_cast<const uint4*>(sp + W_BYTES + (8 * nt + g) * GS_ROW_BYTES);
+                c1 = *reinterpret_cast<const uint4*>(sp + W_BYTES + (8 * nt + g) * GS_ROW_BYTES + 16);
+            }
             gs_mma(acc[nt], wa0.x, wb0.x, wa0.y, wb0.y, c0.x, c0.y);
             gs_mma(acc[nt], wa0.z, wb0.z, wa0.w, wb0.w, c0.z, c0.w);
             gs_mma(acc[nt], wa1.x, wb1.x, wa1.y, wb1.y, c1.x, c1.y);
