@@ -291,7 +291,7 @@ struct GatedDeltaRule : Mixer {
                          "gdr_conv_state");
         // prompts: eight tokens at a time, except in float32, where cutting a prompt into portions must change no bit
         int rc = -2;
-        if (!single && !rt.is_f32() && env_flag("IMP_B200_GDR_BLOCK", false)) {
+        if (!single && !rt.is_f32()) {
             float* scratch = rt.arena->take<float>((size_t)imp_gdr_block_floats((int)T, st.B(), H));
             rc = imp_gdr_block_scan(qn, kn, vc, beta, decay, S, o, scratch, st.view.q_start, st.view.state_slots, st.B(), st.view.max_q_len, G, D, H, Dv,
                                     rt.stream);
