@@ -446,12 +446,18 @@ __global__ void __launch_bounds__(COLS * GS_LANES, SINGLE ? 3 : 1) gdr_scan_kern
 // from block to block where the scan above has one per token.  The 8 x 8 matrices do not depend on the column; gdr_block_kernel
 // makes T = (I + L)^-1 and D (q . k) T per head and block, a warp each.  32-bit arithmetic as above.  Where a prompt is cut decides which
 // tokens share a block, so the last bits depend on it; the 32-bit models, whose results must not, keep the scan above.
-// Bound by the waits inside a block (exchanges and reads of shared memory): 780 instructions a warp in 2,300 cycles, one warp a scheduler.  A thread
-// serves two columns, so that each read of k and q feeds two of them.
+// Bound by the waits inside a block: with sixteen lanes for two columns 780 instructions a warp took 2,300 cycles, one warp a scheduler (306 us for
+// 2,048 tokens of 16 heads, 392 token by token); with 32 lanes there are two warps a scheduler for the same reads of shared memory: 281.1 us.  A
+// lane serves two columns, so that each read of k and q feeds two of them.
 constexpr int GB_TOKENS = 8, GB_D = 128, GB_REC = 160;    // floats of a block's record: T | D (q . k) T | P | D_7j | beta
 constexpr int GB_COLS = 16, GB_CHUNK = 2;                 // columns of a CTA, blocks in a stage of its ring
-constexpr int GB_THREADS = GB_COLS / 2 * 16;
+constexpr int GB_THREADS = GB_COLS / 2 * 32;
 
+__device__ __forceinline__ float gs_sum2(unsigned long long x) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x));
+    return a + b;
+}
 __device__ __forceinline__ int64_t gb_record(int start, int seq, int block) { return start / GB_TOKENS + seq + block; }   // of a sequence's block
 
 __global__ void __launch_bounds__(128) gdr_block_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ beta,
@@ -539,8 +545,8 @@ __global__ void __launch_bounds__(128) gdr_block_kernel(const float* __restrict_
     }
 }
 
-// A CTA: 16 columns of one head of one sequence.  Sixteen lanes share two columns; lane r holds dimensions 4 r ... 4 r + 3 and 64 more of
-// both (16-byte reads of neighbouring lanes are neighbours).  The state's layout in memory is the scan's above.
+// A CTA: 16 columns of one head of one sequence.  A warp has two columns; lane r holds dimensions 4 r ... 4 r + 3 of both (16-byte reads of
+// neighbouring lanes are neighbours).  The state's layout in memory is the scan's above.
 __global__ void __launch_bounds__(GB_THREADS) gdr_block_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc,
                                                                     const float* __restrict__ rec, float* __restrict__ state, float* __restrict__ out,
                                                                     const int* __restrict__ q_start, const int* __restrict__ slots, int G, int H, int Dv) {
@@ -549,19 +555,19 @@ __global__ void __launch_bounds__(GB_THREADS) gdr_block_scan_kernel(const float*
     constexpr int CH = GB_CHUNK * GB_TOKENS;
     __shared__ __align__(16) float k_s[2][CH][GB_D], q_s[2][CH][GB_D];
     __shared__ __align__(16) float rec_s[2][GB_CHUNK][GB_REC], v_s[2][CH][GB_COLS], o_s[CH][GB_COLS];
-    const int tid = threadIdx.x, lane = tid & 31, r = tid & 15, pair = tid >> 4, tok = r & 7, own = r >> 3;
+    const int tid = threadIdx.x, r = tid & 31, pair = tid >> 5, tok = r & 7, own = (r >> 3) & 1;
     const int col0 = blockIdx.x * GB_COLS, h = blockIdx.y, seq = blockIdx.z, hk = h / (H / G);
     const int start = q_start[seq], n = q_start[seq + 1] - start;
     if (n <= 0) return;
     // two neighbouring columns' elements: plane d % 16, place (column % 32) * 8 + d / 16 of the block of 32 columns
     const int blocks = (Dv + GS_COLS - 1) / GS_COLS, col = col0 + 2 * pair;
     float* S = state + (((int64_t)slots[seq] * H + h) * blocks + col / GS_COLS) * 16 * GS_BLOCK + col % GS_COLS * GS_LANES;
-    auto place = [&](int i) { const int d = (i < 4 ? 0 : 64) + 4 * r + i % 4; return d % 16 * GS_BLOCK + d / 16; };
-    unsigned long long s[2][4];
+    auto place = [&](int i) { const int d = 4 * r + i; return d % 16 * GS_BLOCK + d / 16; };
+    unsigned long long s[2][2];
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) s[c][i] = gs_pair(S[place(2 * i) + c * GS_LANES], S[place(2 * i + 1) + c * GS_LANES]);
+        for (int i = 0; i < 2; ++i) s[c][i] = gs_pair(S[place(2 * i) + c * GS_LANES], S[place(2 * i + 1) + c * GS_LANES]);
     const int64_t row = (int64_t)G * GB_D, hv = (int64_t)H * Dv;
     auto load_chunk = [&](int t0, int buf) {
         const int nt = min(CH, n - t0);
@@ -596,23 +602,21 @@ __global__ void __launch_bounds__(GB_THREADS) gdr_block_scan_kernel(const float*
         __syncthreads();
 #pragma unroll 1
         for (int b = 0; b * GB_TOKENS < nt; ++b) {
-            unsigned long long k[GB_TOKENS][4];
+            unsigned long long k[GB_TOKENS][2];
             float a[16], c[16];                          // column 0's eight tokens, column 1's
 #pragma unroll
             for (int j = 0; j < GB_TOKENS; ++j) {
                 const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(&k_s[buf][b * GB_TOKENS + j][4 * r]);
-                const ulonglong2 k1 = *reinterpret_cast<const ulonglong2*>(&k_s[buf][b * GB_TOKENS + j][64 + 4 * r]);
                 const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(&q_s[buf][b * GB_TOKENS + j][4 * r]);
-                const ulonglong2 q1 = *reinterpret_cast<const ulonglong2*>(&q_s[buf][b * GB_TOKENS + j][64 + 4 * r]);
-                k[j][0] = k0.x, k[j][1] = k0.y, k[j][2] = k1.x, k[j][3] = k1.y;
+                k[j][0] = k0.x, k[j][1] = k0.y;
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    a[8 * x + j] = gs_sum4(gs_fma2(s[x][2], k1.x, gs_mul2(s[x][0], k0.x)), gs_fma2(s[x][3], k1.y, gs_mul2(s[x][1], k0.y)));
-                    c[8 * x + j] = gs_sum4(gs_fma2(s[x][2], q1.x, gs_mul2(s[x][0], q0.x)), gs_fma2(s[x][3], q1.y, gs_mul2(s[x][1], q0.y)));
+                    a[8 * x + j] = gs_sum2(gs_fma2(s[x][1], k0.y, gs_mul2(s[x][0], k0.x)));
+                    c[8 * x + j] = gs_sum2(gs_fma2(s[x][1], q0.y, gs_mul2(s[x][0], q0.x)));
                 }
             }
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) {            // over the sixteen lanes; lane r keeps token r % 8 of column r / 8
+            for (int o = 8; o > 0; o >>= 1) {            // over sixteen lanes; lane r keeps token r % 8 of column r / 8 % 2
                 const bool up = r & o;
 #pragma unroll
                 for (int j = 0; j < o; ++j) {
@@ -621,6 +625,8 @@ __global__ void __launch_bounds__(GB_THREADS) gdr_block_scan_kernel(const float*
                     c[j] = kc + __shfl_xor_sync(0xffffffffu, gc, o);
                 }
             }
+            a[0] += __shfl_xor_sync(0xffffffffu, a[0], 16);   // and the other sixteen: both halves go on with the same numbers
+            c[0] += __shfl_xor_sync(0xffffffffu, c[0], 16);
             const float* m = rec_s[buf][b];
             const float p = m[128 + tok];
             const float bv = m[144 + tok] * fmaf(-p, a[0], v_s[buf][b * GB_TOKENS + tok][2 * pair + own]);
@@ -630,25 +636,25 @@ __global__ void __launch_bounds__(GB_THREADS) gdr_block_scan_kernel(const float*
             float u0 = 0.f, u1 = 0.f, o0 = p * c[0], o1 = 0.f;
 #pragma unroll
             for (int i = 0; i < 8; i += 2) {
-                const float x = __shfl_sync(0xffffffffu, bv, (lane & 24) | i), y = __shfl_sync(0xffffffffu, bv, (lane & 24) | (i + 1));
+                const float x = __shfl_sync(0xffffffffu, bv, (r & 24) | i), y = __shfl_sync(0xffffffffu, bv, (r & 24) | (i + 1));
                 u0 = fmaf(tr[i], x, u0), u1 = fmaf(tr[i + 1], y, u1);
                 o0 = fmaf(rr[i], x, o0), o1 = fmaf(rr[i + 1], y, o1);
             }
-            o_s[b * GB_TOKENS + tok][2 * pair + own] = o0 + o1;
+            if (r < 16) o_s[b * GB_TOKENS + tok][2 * pair + own] = o0 + o1;
             const float du = m[136 + tok] * (u0 + u1), last = m[128 + GB_TOKENS - 1];
             const unsigned long long p2 = gs_pair(last, last);
 #pragma unroll
             for (int x = 0; x < 2; ++x)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s[x][i] = gs_mul2(p2, s[x][i]);
+                for (int i = 0; i < 2; ++i) s[x][i] = gs_mul2(p2, s[x][i]);
 #pragma unroll
             for (int j = 0; j < GB_TOKENS; ++j)
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    const float w = __shfl_sync(0xffffffffu, du, (lane & 16) | (8 * x) | j);
+                    const float w = __shfl_sync(0xffffffffu, du, 8 * x + j);
                     const unsigned long long w2 = gs_pair(w, w);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) s[x][i] = gs_fma2(k[j][i], w2, s[x][i]);
+                    for (int i = 0; i < 2; ++i) s[x][i] = gs_fma2(k[j][i], w2, s[x][i]);
                 }
         }
         __syncthreads();
@@ -660,7 +666,7 @@ __global__ void __launch_bounds__(GB_THREADS) gdr_block_scan_kernel(const float*
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 2; ++i) {
             float lo, hi;
             asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(s[c][i]));
             S[place(2 * i) + c * GS_LANES] = lo;
