@@ -6,7 +6,7 @@
 // of a short causal convolution over time per channel (taps - 1 earlier inputs are part of a request's
 // state) followed by silu; q and k are then unit vectors per head and q carries D^(-1/2).
 //
-// Four kernels, all 32-bit arithmetic on 32-bit state whatever the activation type:
+// Token by token there are four kernels, all 32-bit arithmetic on 32-bit state whatever the activation type:
 //   gdr_prepare     one warp per token and head: convolution + silu of its channels, unit q and k; beta and decay
 //   gdr_conv_state  the last taps - 1 inputs of every sequence of the batch go to its state slot
 //   gdr_scan        the recurrence; a CTA owns 32 value columns of one head of one sequence and walks
@@ -16,7 +16,10 @@
 //   gdr_output      per head: o / rms(o) * w * silu(gate)
 // Every column of S evolves independently of the others, which is what the scan kernel's split rests on.
 // A token's result depends on the tokens before it only through S and the convolution's inputs, and the
-// order of every sum is fixed by the sizes alone: cutting a prompt into portions changes no bit.
+// order of every sum of these kernels is fixed by the sizes alone: cutting a prompt into portions changes
+// no bit.  Prompts of 16-bit models take the recurrence eight tokens at a time (gdr_block_kernel and
+// gdr_block_scan_kernel); its sums are ordered by the blocks of a portion, so a cut that is not at a
+// multiple of eight tokens may change the last bits of float32 there.
 #include <algorithm>
 
 #include "common.cuh"
@@ -120,7 +123,8 @@ __global__ void __launch_bounds__(GP_BLOCK) gdr_prepare_kernel(
 // The same for a prompt's rows, heads of up to 128 in whole 32s: a warp makes one head of eight neighbouring tokens.  A token's row is asked for
 // once instead of once a tap, the taps' weights once for eight tokens, and all rows go out together: 11 loads and 4 a lane and channel where
 // single tokens take 64.  A lane has the same channels and adds them in the same order, so the bits are the single tokens'.
-// 2,048 tokens of 8 + 8 + 16 heads of 128: 49 us before.
+// The tokens' sequences are looked up by eight lanes at once: one after the other they were two dependent loads a token.
+// 2,048 tokens of 8 + 8 + 16 heads of 128: 39.7 us; single tokens 49, with the lookups one after the other 51.
 constexpr int GP_RUN = 8, GP_CH = 4;      // tokens of a warp, channels of a lane at most
 template <typename TA, int TAPS>
 __global__ void __launch_bounds__(GP_BLOCK) gdr_prepare_run_kernel(
@@ -146,6 +150,17 @@ __global__ void __launch_bounds__(GP_BLOCK) gdr_prepare_run_kernel(
         }
         return;
     }
+    // lane r looks up token r's sequence, its first token and its slot
+    int l_seq = -1, l_start = 0, l_slot = 0;
+    if (lane < n_run) {
+        l_seq = seq_of_token[t0 + lane];
+        if (l_seq < 0 || l_seq >= n_seqs) {
+            if (unit == 0) imp_report(status, IMP_BAD_SEQUENCE);
+            l_seq = -1;
+        } else {
+            l_start = q_start[l_seq], l_slot = slots[l_seq];
+        }
+    }
     const bool value = unit >= 2 * G;
     const int size = value ? Dv : D, c0 = (value ? 2 * nqk + (unit - 2 * G) * Dv : unit * D) + lane;
     float w[GP_CH][TAPS], x[GP_RUN + TAPS - 1][GP_CH];
@@ -161,13 +176,9 @@ __global__ void __launch_bounds__(GP_BLOCK) gdr_prepare_run_kernel(
     }
 #pragma unroll
     for (int r = 0; r < GP_RUN; ++r) {
-        if (r >= n_run) break;
-        const int t = t0 + r, seq = seq_of_token[t];
-        if (seq < 0 || seq >= n_seqs) {
-            if (lane == 0 && unit == 0) imp_report(status, IMP_BAD_SEQUENCE);
-            continue;
-        }
-        const int n = t - q_start[seq];         // index of the token inside its portion
+        const int t = t0 + r, seq = __shfl_sync(0xffffffffu, l_seq, r), n = t - __shfl_sync(0xffffffffu, l_start, r);   // n: index in its portion
+        const int64_t before = (int64_t)__shfl_sync(0xffffffffu, l_slot, r) * (TAPS - 1) + TAPS - 1;   // row of the state behind the last one
+        if (seq < 0) continue;
         float y[GP_CH], ss = 0.f;
 #pragma unroll
         for (int i = 0; i < GP_CH; ++i) {
@@ -176,7 +187,7 @@ __global__ void __launch_bounds__(GP_BLOCK) gdr_prepare_run_kernel(
             for (int j = 0; j < TAPS; ++j) {
                 const int idx = n - (TAPS - 1) + j;
                 float v = x[r + j][i];
-                if (idx < 0) v = 32 * i < size ? conv_state[((int64_t)slots[seq] * (TAPS - 1) + TAPS - 1 + idx) * C + c0 + 32 * i] : 0.f;
+                if (idx < 0) v = 32 * i < size ? conv_state[(before + idx) * C + c0 + 32 * i] : 0.f;
                 acc = fmaf(w[i][j], v, acc);
             }
             y[i] = 32 * i < size ? silu_f(acc) : 0.f;
