@@ -458,8 +458,8 @@ __global__ void __launch_bounds__(COLS * GS_LANES, SINGLE ? 3 : 1) gdr_scan_kern
 // makes T = (I + L)^-1 and D (q . k) T per head and block, a warp each.  32-bit arithmetic as above.  Where a prompt is cut decides which
 // tokens share a block, so the last bits depend on it; the 32-bit models, whose results must not, keep the scan above.
 // Bound by the waits inside a block: with sixteen lanes for two columns 780 instructions a warp took 2,300 cycles, one warp a scheduler (306 us for
-// 2,048 tokens of 16 heads, 392 token by token); with 32 lanes there are two warps a scheduler for the same reads of shared memory: 281.1 us.  A
-// lane serves two columns, so that each read of k and q feeds two of them.
+// 2,048 tokens of 16 heads, 392 token by token); with 32 lanes there are two warps a scheduler for the same reads of shared memory: 281.1 us.  Eight
+// sequences of 64 tokens and 32 heads, whose CTAs fill the device: 112.8 us (sixteen lanes 92.6, token by token 126.6).  A lane serves two columns, so that each read of k and q feeds two of them.
 constexpr int GB_TOKENS = 8, GB_D = 128, GB_REC = 160;    // floats of a block's record: T | D (q . k) T | P | D_7j | beta
 constexpr int GB_COLS = 16, GB_CHUNK = 2;                 // columns of a CTA, blocks in a stage of its ring
 constexpr int GB_THREADS = GB_COLS / 2 * 32;
