@@ -448,243 +448,6 @@ __global__ void __launch_bounds__(COLS * GS_LANES, SINGLE ? 3 : 1) gdr_scan_kern
     }
 }
 
-// ------------------------------------------------------------------------------- scan, eight tokens at a time
-// The same recurrence for prompts in a 16-bit model (key size 128), eight tokens as one step.  With S the state before the block,
-// P_j = g_0 ... g_j, D_ji = g_(i+1) ... g_j and L_ji = beta_j D_ji (k_j . k_i) for i < j,
-//     b_j = beta_j (v_j - P_j S^T k_j);   u = (I + L)^-1 b;   o_j = P_j S^T q_j + sum_(i <= j) D_ji (q_j . k_i) u_i;
-//     S <- P_7 S + sum_j D_7j k_j u_j^T.
-// So the sums over the key dimension of all eight tokens start from one state: one exchange over the lanes per block is on the way
-// from block to block where the scan above has one per token.  The 8 x 8 matrices do not depend on the column; gdr_block_kernel
-// makes T = (I + L)^-1 and D (q . k) T per head and block, a warp each.  32-bit arithmetic as above.  Where a prompt is cut decides which
-// tokens share a block, so the last bits depend on it; the 32-bit models, whose results must not, keep the scan above.
-// Bound by the waits inside a block: with sixteen lanes for two columns 780 instructions a warp took 2,300 cycles, one warp a scheduler (306 us for
-// 2,048 tokens of 16 heads, 392 token by token); with 32 lanes there are two warps a scheduler for the same reads of shared memory: 281.1 us.  Eight
-// sequences of 64 tokens and 32 heads, whose CTAs fill the device: 112.8 us (sixteen lanes 92.6, token by token 126.6).  A lane serves two columns, so that each read of k and q feeds two of them.
-constexpr int GB_TOKENS = 8, GB_D = 128, GB_REC = 160;    // floats of a block's record: T | D (q . k) T | P | D_7j | beta
-constexpr int GB_COLS = 16, GB_CHUNK = 2;                 // columns of a CTA, blocks in a stage of its ring
-constexpr int GB_THREADS = GB_COLS / 2 * 32;
-
-__device__ __forceinline__ float gs_sum2(unsigned long long x) {
-    float a, b;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x));
-    return a + b;
-}
-__device__ __forceinline__ int64_t gb_record(int start, int seq, int block) { return start / GB_TOKENS + seq + block; }   // of a sequence's block
-
-__global__ void __launch_bounds__(128) gdr_block_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ beta,
-                                                        const float* __restrict__ decay, float* __restrict__ rec, const int* __restrict__ q_start, int G,
-                                                        int H) {
-    pdl_wait();
-    pdl_launch_dependents();
-    __shared__ float mats[4][3][GB_TOKENS][GB_TOKENS];   // L, D (q . k), T
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = blockIdx.y, seq = blockIdx.z, block = blockIdx.x * 4 + warp;
-    const int start = q_start[seq], n = min(GB_TOKENS, q_start[seq + 1] - start - block * GB_TOKENS), t0 = start + block * GB_TOKENS;
-    if (n <= 0) return;
-    const int64_t row = (int64_t)G * GB_D, at = (int64_t)(h / (H / G)) * GB_D + 4 * lane;
-    float4 k[GB_TOKENS], q[GB_TOKENS];
-    float g[GB_TOKENS], be[GB_TOKENS];
-#pragma unroll
-    for (int j = 0; j < GB_TOKENS; ++j) {
-        const bool there = j < n;                        // tokens beyond the sequence change nothing: no key, no step, no decay
-        k[j] = there ? *reinterpret_cast<const float4*>(kn + (t0 + j) * row + at) : make_float4(0.f, 0.f, 0.f, 0.f);
-        q[j] = there ? *reinterpret_cast<const float4*>(qn + (t0 + j) * row + at) : make_float4(0.f, 0.f, 0.f, 0.f);
-        g[j] = there ? decay[(int64_t)(t0 + j) * H + h] : 1.f;
-        be[j] = there ? beta[(int64_t)(t0 + j) * H + h] : 0.f;
-    }
-    // Four trees of 32 sums over the lanes each: lane l ends with element 32 half + l of k . k (tree 0, 1) and q . k (2, 3).
-#pragma unroll
-    for (int tree = 0; tree < 4; ++tree) {
-        float x[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-            const int j = (tree & 1) * 4 + e / 8, i = e % 8;
-            const float4 a = tree < 2 ? k[j] : q[j], b = k[i];
-            x[e] = (tree < 2 ? i < j : i <= j) ? fmaf(a.x, b.x, a.y * b.y) + fmaf(a.z, b.z, a.w * b.w) : 0.f;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const bool up = lane & o;
-#pragma unroll
-            for (int j = 0; j < o; ++j) {
-                const float keep = up ? x[j + o] : x[j], give = up ? x[j] : x[j + o];
-                x[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-            }
-        }
-        const int j = (tree & 1) * 4 + lane / 8, i = lane % 8;
-        float d = 1.f, step = 0.f;
-#pragma unroll
-        for (int l = 0; l < GB_TOKENS; ++l) {
-            if (l > i && l <= j) d *= g[l];
-            if (l == j) step = be[l];
-        }
-        mats[warp][tree < 2 ? 0 : 1][j][i] = tree < 2 ? step * d * x[0] : d * x[0];
-    }
-    __syncwarp();
-    if (lane < GB_TOKENS) {                              // column `lane` of (I + L)^-1
-        float t[GB_TOKENS];
-#pragma unroll
-        for (int j = 0; j < GB_TOKENS; ++j) {
-            float v = j == lane ? 1.f : 0.f;
-#pragma unroll
-            for (int l = 0; l < j; ++l) v = fmaf(-mats[warp][0][j][l], t[l], v);
-            t[j] = v;                                    // zero above the diagonal: t[l] is zero for l < lane
-            mats[warp][2][j][lane] = v;
-        }
-    }
-    __syncwarp();
-    float* out = rec + (gb_record(start, seq, block) * H + h) * GB_REC;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const int j = half * 4 + lane / 8, i = lane % 8;
-        float v = 0.f;
-#pragma unroll
-        for (int l = 0; l < GB_TOKENS; ++l) v = fmaf(mats[warp][1][j][l], mats[warp][2][l][i], v);
-        out[half * 32 + lane] = mats[warp][2][j][i];
-        out[64 + half * 32 + lane] = v;
-    }
-    if (lane < GB_TOKENS) {
-        float p = 1.f, e = 1.f, step = 0.f;
-#pragma unroll
-        for (int l = 0; l < GB_TOKENS; ++l) {
-            if (l <= lane) p *= g[l];
-            else e *= g[l];
-            if (l == lane) step = be[l];
-        }
-        out[128 + lane] = p;
-        out[136 + lane] = e;
-        out[144 + lane] = step;
-    }
-}
-
-// A CTA: 16 columns of one head of one sequence.  A warp has two columns; lane r holds dimensions 4 r ... 4 r + 3 of both (16-byte reads of
-// neighbouring lanes are neighbours).  The state's layout in memory is the scan's above.
-__global__ void __launch_bounds__(GB_THREADS) gdr_block_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vc,
-                                                                    const float* __restrict__ rec, float* __restrict__ state, float* __restrict__ out,
-                                                                    const int* __restrict__ q_start, const int* __restrict__ slots, int G, int H, int Dv) {
-    pdl_wait();
-    pdl_launch_dependents();
-    constexpr int CH = GB_CHUNK * GB_TOKENS;
-    __shared__ __align__(16) float k_s[2][CH][GB_D], q_s[2][CH][GB_D];
-    __shared__ __align__(16) float rec_s[2][GB_CHUNK][GB_REC], v_s[2][CH][GB_COLS], o_s[CH][GB_COLS];
-    const int tid = threadIdx.x, r = tid & 31, pair = tid >> 5, tok = r & 7, own = (r >> 3) & 1;
-    const int col0 = blockIdx.x * GB_COLS, h = blockIdx.y, seq = blockIdx.z, hk = h / (H / G);
-    const int start = q_start[seq], n = q_start[seq + 1] - start;
-    if (n <= 0) return;
-    // two neighbouring columns' elements: plane d % 16, place (column % 32) * 8 + d / 16 of the block of 32 columns
-    const int blocks = (Dv + GS_COLS - 1) / GS_COLS, col = col0 + 2 * pair;
-    float* S = state + (((int64_t)slots[seq] * H + h) * blocks + col / GS_COLS) * 16 * GS_BLOCK + col % GS_COLS * GS_LANES;
-    auto place = [&](int i) { const int d = 4 * r + i; return d % 16 * GS_BLOCK + d / 16; };
-    unsigned long long s[2][2];
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) s[c][i] = gs_pair(S[place(2 * i) + c * GS_LANES], S[place(2 * i + 1) + c * GS_LANES]);
-    const int64_t row = (int64_t)G * GB_D, hv = (int64_t)H * Dv;
-    auto load_chunk = [&](int t0, int buf) {
-        const int nt = min(CH, n - t0);
-        for (int e = tid; e < CH * GB_D / 4; e += GB_THREADS) {
-            const int tt = e / (GB_D / 4), d = e % (GB_D / 4) * 4;
-            const int64_t src = tt < nt ? (start + t0 + tt) * row + hk * GB_D + d : 0;
-            gs_cp_async16(&k_s[buf][tt][d], kn + src, tt < nt);
-            gs_cp_async16(&q_s[buf][tt][d], qn + src, tt < nt);
-        }
-        for (int e = tid; e < GB_CHUNK * GB_REC / 4; e += GB_THREADS) {
-            const int b = e / (GB_REC / 4), d = e % (GB_REC / 4) * 4;
-            const bool there = b * GB_TOKENS < nt && d < 152;
-            gs_cp_async16(&rec_s[buf][b][d], rec + (there ? (gb_record(start, seq, t0 / GB_TOKENS + b) * H + h) * GB_REC + d : 0), there);
-        }
-        for (int e = tid; e < CH * GB_COLS; e += GB_THREADS) {
-            const int tt = e / GB_COLS, c = e % GB_COLS;
-            const bool there = tt < nt && col0 + c < Dv;
-            gs_cp_async4(&v_s[buf][tt][c], vc + (there ? (start + t0 + tt) * hv + (int64_t)h * Dv + col0 + c : 0), there);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    load_chunk(0, 0);
-    int buf = 0;
-    for (int t0 = 0; t0 < n; t0 += CH, buf ^= 1) {
-        const int nt = min(CH, n - t0);
-        if (t0 + CH < n) {
-            load_chunk(t0 + CH, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        }
-        __syncthreads();
-#pragma unroll 1
-        for (int b = 0; b * GB_TOKENS < nt; ++b) {
-            unsigned long long k[GB_TOKENS][2];
-            float a[16], c[16];                          // column 0's eight tokens, column 1's
-#pragma unroll
-            for (int j = 0; j < GB_TOKENS; ++j) {
-                const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(&k_s[buf][b * GB_TOKENS + j][4 * r]);
-                const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(&q_s[buf][b * GB_TOKENS + j][4 * r]);
-                k[j][0] = k0.x, k[j][1] = k0.y;
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    a[8 * x + j] = gs_sum2(gs_fma2(s[x][1], k0.y, gs_mul2(s[x][0], k0.x)));
-                    c[8 * x + j] = gs_sum2(gs_fma2(s[x][1], q0.y, gs_mul2(s[x][0], q0.x)));
-                }
-            }
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) {            // over sixteen lanes; lane r keeps token r % 8 of column r / 8 % 2
-                const bool up = r & o;
-#pragma unroll
-                for (int j = 0; j < o; ++j) {
-                    const float ka = up ? a[j + o] : a[j], ga = up ? a[j] : a[j + o], kc = up ? c[j + o] : c[j], gc = up ? c[j] : c[j + o];
-                    a[j] = ka + __shfl_xor_sync(0xffffffffu, ga, o);
-                    c[j] = kc + __shfl_xor_sync(0xffffffffu, gc, o);
-                }
-            }
-            a[0] += __shfl_xor_sync(0xffffffffu, a[0], 16);   // and the other sixteen: both halves go on with the same numbers
-            c[0] += __shfl_xor_sync(0xffffffffu, c[0], 16);
-            const float* m = rec_s[buf][b];
-            const float p = m[128 + tok];
-            const float bv = m[144 + tok] * fmaf(-p, a[0], v_s[buf][b * GB_TOKENS + tok][2 * pair + own]);
-            const float4 ta = *reinterpret_cast<const float4*>(m + 8 * tok), tb = *reinterpret_cast<const float4*>(m + 8 * tok + 4);
-            const float4 ra = *reinterpret_cast<const float4*>(m + 64 + 8 * tok), rb = *reinterpret_cast<const float4*>(m + 68 + 8 * tok);
-            const float tr[8] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w}, rr[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
-            float u0 = 0.f, u1 = 0.f, o0 = p * c[0], o1 = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; i += 2) {
-                const float x = __shfl_sync(0xffffffffu, bv, (r & 24) | i), y = __shfl_sync(0xffffffffu, bv, (r & 24) | (i + 1));
-                u0 = fmaf(tr[i], x, u0), u1 = fmaf(tr[i + 1], y, u1);
-                o0 = fmaf(rr[i], x, o0), o1 = fmaf(rr[i + 1], y, o1);
-            }
-            if (r < 16) o_s[b * GB_TOKENS + tok][2 * pair + own] = o0 + o1;
-            const float du = m[136 + tok] * (u0 + u1), last = m[128 + GB_TOKENS - 1];
-            const unsigned long long p2 = gs_pair(last, last);
-#pragma unroll
-            for (int x = 0; x < 2; ++x)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) s[x][i] = gs_mul2(p2, s[x][i]);
-#pragma unroll
-            for (int j = 0; j < GB_TOKENS; ++j)
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    const float w = __shfl_sync(0xffffffffu, du, 8 * x + j);
-                    const unsigned long long w2 = gs_pair(w, w);
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) s[x][i] = gs_fma2(k[j][i], w2, s[x][i]);
-                }
-        }
-        __syncthreads();
-        for (int e = tid; e < nt * GB_COLS; e += GB_THREADS) {
-            const int tt = e / GB_COLS, c = e % GB_COLS;
-            if (col0 + c < Dv) out[(start + t0 + tt) * hv + (int64_t)h * Dv + col0 + c] = o_s[tt][c];
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            float lo, hi;
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(s[c][i]));
-            S[place(2 * i) + c * GS_LANES] = lo;
-            S[place(2 * i + 1) + c * GS_LANES] = hi;
-        }
-}
-
 // -------------------------------------------------------------------------------------- output
 // y[t, h, :] = o[t, h, :] / sqrt(mean(o^2) + eps) * w[h * w_head_stride + :] * act(gate[t, h, :]); a warp per (token, head).
 // w may be null (no weight); w_head_stride 0: one weight vector for all heads; act: 0 silu, 1 sigmoid.
@@ -830,24 +593,6 @@ IMP_API int imp_gdr_scan(const float* qn, const float* kn, const float* vc, cons
     return imp_gdr_scan_ex(qn, kn, vc, beta, decay, state, out, q_start, slots, n_seqs, G, D, H, Dv, 0, stream);
 }
 
-
-// The scan eight tokens at a time (see gdr_block_scan_kernel): key size 128, rows that start on 16 bytes; else IMP_ERR_UNSUPPORTED, nothing
-// done.  scratch: imp_gdr_block_floats(n_tokens, n_seqs, H); max_tokens: of one sequence.
-IMP_API int64_t imp_gdr_block_floats(int n_tokens, int n_seqs, int H) { return ((int64_t)n_tokens / GB_TOKENS + n_seqs + 1) * H * GB_REC; }
-IMP_API int imp_gdr_block_scan(const float* qn, const float* kn, const float* vc, const float* beta, const float* decay, float* state, float* out,
-                               float* scratch, const int* q_start, const int* slots, int n_seqs, int max_tokens, int G, int D, int H, int Dv, void* stream) {
-    if (n_seqs == 0) return 0;
-    IMP_CHECK_ARG(qn && kn && vc && beta && decay && state && out && scratch && q_start && slots, "imp_gdr_block_scan: null pointer");
-    IMP_CHECK_ARG(G > 0 && H % G == 0 && Dv > 0 && H <= 65535 && n_seqs <= 65535 && max_tokens > 0, "imp_gdr_block_scan: bad sizes");
-    if (D != GB_D || (uintptr_t)qn % 16 || (uintptr_t)kn % 16 || (uintptr_t)scratch % 16) return IMP_ERR_UNSUPPORTED;
-    cudaStream_t s = (cudaStream_t)stream;
-    const int blocks = (max_tokens + GB_TOKENS - 1) / GB_TOKENS;
-    imp_launch(gdr_block_kernel, dim3((blocks + 3) / 4, H, n_seqs), dim3(128), 0, s, qn, kn, beta, decay, scratch, q_start, G, H);
-    // An ordinary launch: ahead of its turn its CTAs crowd on the SMs that are free first, and 2,048 tokens of 16 heads take 450 us instead of 300.
-    imp_launch_as(false, gdr_block_scan_kernel, dim3((Dv + GS_COLS - 1) / GS_COLS * (GS_COLS / GB_COLS), H, n_seqs), dim3(GB_THREADS), 0, s, qn, kn, vc,
-               (const float*)scratch, state, out, q_start, slots, G, H, Dv);
-    IMP_RETURN_LAUNCH();
-}
 
 // The same read-out with one norm over the whole row: y[t, :] = o[t, :] / sqrt(mean over all n of o^2 + eps) * w * act(gate[t, :]),
 // the heads side by side (n = H * Dv); a CTA per token, sums in 32-bit in an order the row's size fixes.

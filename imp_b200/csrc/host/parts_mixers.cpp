@@ -289,16 +289,7 @@ struct GatedDeltaRule : Mixer {
             check_launch(imp_gdr_conv_state(proj.data, proj.stride0, conv_state, taps, C, st.view.q_start, st.view.state_slots, st.B(), rt.dtype,
                                             rt.stream),
                          "gdr_conv_state");
-        // prompts: eight tokens at a time, except in float32, where cutting a prompt into portions must change no bit
-        int rc = -2;
-        if (!single && !rt.is_f32()) {
-            float* scratch = rt.arena->take<float>((size_t)imp_gdr_block_floats((int)T, st.B(), H));
-            rc = imp_gdr_block_scan(qn, kn, vc, beta, decay, S, o, scratch, st.view.q_start, st.view.state_slots, st.B(), st.view.max_q_len, G, D, H, Dv,
-                                    rt.stream);
-            rt.launches += rc == 0;
-        }
-        if (rc == -2) rc = imp_gdr_scan_ex(qn, kn, vc, beta, decay, S, o, st.view.q_start, st.view.state_slots, st.B(), G, D, H, Dv, single ? 1 : 0, rt.stream);
-        check_launch(rc, "gdr_scan");
+        check_launch(imp_gdr_scan_ex(qn, kn, vc, beta, decay, S, o, st.view.q_start, st.view.state_slots, st.B(), G, D, H, Dv, st.decode_only() ? 1 : 0, rt.stream), "gdr_scan");
         Tensor y = rt.empty(T, (int64_t)H * Dv);
         const Tensor gate = col_slice(proj, C, (int64_t)H * Dv);
         check_launch(imp_gdr_output(y.data, o, gate.data, gate.stride0, (const float*)out_norm.data, eps, (int)T, H, Dv, rt.dtype, rt.stream),

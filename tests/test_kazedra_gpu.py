@@ -259,16 +259,19 @@ RIGHT_CASES = [
     dict(heads=2, kv_heads=2, dim=70, vdim=33, conv=5, d=40),
     dict(heads=4, kv_heads=1, dim=128, vdim=64, conv=1, d=64),
     dict(heads=1, kv_heads=1, dim=8, vdim=100, conv=2, d=24),
+    dict(heads=4, kv_heads=2, dim=128, vdim=128, conv=4, d=64),
 ]
 
 
-def right_setup(dtype, case, slots=4):
+def right_setup(dtype, case, slots=4, eighths=False):
     c = {k: case[k] for k in ("heads", "kv_heads", "dim", "vdim", "conv")}
     params = {"hidden_size": case["d"], "num_heads": c["heads"], "num_kv_heads": c["kv_heads"], "key_dim": c["dim"],
               "value_dim": c["vdim"], "conv_taps": c["conv"], "norm_eps": 2e-5}
     # the state this mixer asks for (S in its scan kernel's layout, and the convolution's last inputs)
     bench = PartBench(NAME[dtype], [mixer_cache_spec("gated_delta_rule", params)], slots=slots, max_tokens=512, max_seq_len=512)
     w = {k: v.to(dtype) for k, v in right_weights(case["d"], c, seed=200).items()}
+    if eighths:      # with inputs of -1, 0 and 1 every product in front of the recurrence is exact, whatever its kernel and order
+        w.update({k: ((8 * w[k].float()).round() / 8).clamp(-2, 2).to(dtype) for k in ("q", "k", "v", "g", "b", "a")})
     part = bench.build("mixer", PartSpec("gated_delta_rule", params), {RIGHT_NAMES[k]: v.to(DEV) for k, v in w.items()})
     return bench, part, c, {"m." + k: v.double() for k, v in w.items()}
 
@@ -323,6 +326,48 @@ def test_delta_rule_portions_change_no_bit():
         bench.commit()
         done += n
     assert torch.equal(torch.cat(outs), whole_out)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case", RIGHT_CASES[2:], ids=lambda c: f"{c['dim']}-{c['conv']}")
+def test_cuts_and_company_change_no_bit_of_the_recurrence(dtype, case):
+    """A request's state after 60 tokens: read at once and alone, or in portions and single tokens beside other requests' portions."""
+    bench, part, _, _ = right_setup(dtype, case, slots=3, eighths=True)
+    g = torch.Generator().manual_seed(5)
+    x, other = (torch.randint(-1, 2, (n, case["d"]), generator=g).to(dtype) for n in (60, 90))
+
+    def step(entries):
+        ctx = bench.prepare([(r, [1] * len(rows), []) for r, rows in entries])
+        view = bench.cache_view(0)
+        run_mixer(bench, part, torch.cat([rows for _, rows in entries]), ctx, view)
+        states = [[t[slot].clone() for t in view.states] for slot in ctx.slots]
+        bench.commit()
+        return states
+
+    want = step([("alone", x)])[0]
+    at = done = 0
+    for n, beside in ((1, 9), (3, 0), (16, 1), (1, 33), (1, 0), (7, 2), (1, 40), (30, 5)):
+        entries = [("cut", x[at:at + n])] + ([("other", other[done:done + beside])] if beside else [])
+        got = step(entries)[0]
+        at, done = at + n, done + beside
+    assert at == len(x) and done == len(other)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case", RIGHT_CASES[2:], ids=lambda c: f"{c['dim']}-{c['conv']}")
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_what_is_not_finite_reaches_no_earlier_token(dtype, case, value):
+    bench, part, _, _ = right_setup(dtype, case)
+    x = rnd(24, case["d"], seed=79).to(dtype)
+    clean = run_mixer(bench, part, x, bench.prepare([("a", [1] * 24, [])]), bench.cache_view(0))
+    bench.commit()
+    x[13] = value
+    out = run_mixer(bench, part, x, bench.prepare([("b", [1] * 24, [])]), bench.cache_view(0))
+    bench.commit()
+    assert torch.isfinite(clean).all() and torch.equal(out[:13], clean[:13])
+    assert not torch.isfinite(out[13]).any()
 
 
 def test_long_decay_and_state_carry():
