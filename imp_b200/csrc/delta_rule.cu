@@ -6,8 +6,9 @@
 // of a short causal convolution over time per channel (taps - 1 earlier inputs are part of a request's
 // state) followed by silu; q and k are then unit vectors per head and q carries D^(-1/2).
 //
-// Token by token there are four kernels, all 32-bit arithmetic on 32-bit state whatever the activation type:
+// Kernels, all 32-bit arithmetic on 32-bit state whatever the activation type:
 //   gdr_prepare     one warp per token and head: convolution + silu of its channels, unit q and k; beta and decay
+//   gdr_prepare_run the same for long prompts, one warp per head and eight neighbouring tokens
 //   gdr_conv_state  the last taps - 1 inputs of every sequence of the batch go to its state slot
 //   gdr_scan        the recurrence; a CTA owns 32 value columns of one head of one sequence and walks
 //                   the sequence's new tokens in order; eight lanes share a column, each holding an
@@ -16,10 +17,8 @@
 //   gdr_output      per head: o / rms(o) * w * silu(gate)
 // Every column of S evolves independently of the others, which is what the scan kernel's split rests on.
 // A token's result depends on the tokens before it only through S and the convolution's inputs, and the
-// order of every sum of these kernels is fixed by the sizes alone: cutting a prompt into portions changes
-// no bit.  Prompts of 16-bit models take the recurrence eight tokens at a time (gdr_block_kernel and
-// gdr_block_scan_kernel); its sums are ordered by the blocks of a portion, so a cut that is not at a
-// multiple of eight tokens may change the last bits of float32 there.
+// order of every sum is fixed by the sizes alone: neither cutting a prompt into portions nor the other
+// requests of a step change a bit.
 #include <algorithm>
 
 #include "common.cuh"
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(GP_BLOCK) gdr_prepare_kernel(
 // once instead of once a tap, the taps' weights once for eight tokens, and all rows go out together: 11 loads and 4 a lane and channel where
 // single tokens take 64.  A lane has the same channels and adds them in the same order, so the bits are the single tokens'.
 // The tokens' sequences are looked up by eight lanes at once: one after the other they were two dependent loads a token.
-// 2,048 tokens of 8 + 8 + 16 heads of 128: 39.7 us; single tokens 49, with the lookups one after the other 51.
+// A warp's eight tokens follow one another, about 9 us from start to end: gdr_prepare_run_pays says from where on that is worth it.
 constexpr int GP_RUN = 8, GP_CH = 4;      // tokens of a warp, channels of a lane at most
 template <typename TA, int TAPS>
 __global__ void __launch_bounds__(GP_BLOCK) gdr_prepare_run_kernel(
@@ -477,12 +476,36 @@ __global__ void gdr_output_kernel(TA* __restrict__ y, const float* __restrict__ 
 }
 
 // ------------------------------------------------------------------------------------ launchers
+// Eight tokens a warp, where that is faster.  592 CTAs are resident (four on each of 148 SMs) and a round of them takes 9 us however few they are, so
+// it takes a round that is three quarters full, or 3.5 million channels (855 tokens of 8 + 8 + 16 heads of 128), from where on the last round no longer
+// counts.  In us, against a warp a token, bfloat16, those heads: 512 tokens (528 CTAs) 10.5 and 12.9, 900 tokens 18.8 and 20.8, 2,048 tokens 46.8 and 51.3; but
+// two tokens 4.2 and 2.9, 64 tokens 8.4 and 4.9, 256 tokens (264 CTAs) 10.2 and 7.6, 640 tokens (660 CTAs) 16.4 and 15.5.
+// In bfloat16 a warp's request is half a 128-byte line and the gain is small: heads below 96 lose (2,929 tokens of heads of 64: 49.7 and 48.5), and so do many
+// short sequences, whose taps come from the states (2,048 tokens in portions of 9: 57.1 and 54.7).  In float32 all of them gain from 3.5 million channels on
+// (2,048 tokens: 34.4 and 55.2; in portions of 9: 43.7 and 57.1).
+static bool gdr_prepare_run_pays(int n_tokens, int n_seqs, int G, int D, int H, int Dv, bool f32) {
+    constexpr int64_t resident = 592;
+    const int64_t run_ctas = ((int64_t)(n_tokens + GP_RUN - 1) / GP_RUN * (2 * G + H + 1) + GP_BLOCK / 32 - 1) / (GP_BLOCK / 32);
+    const bool wide = D >= 96 && Dv >= 96 && n_tokens >= 64 * (int64_t)n_seqs;
+    if (wide && 4 * run_ctas >= 3 * resident * ((run_ctas + resident - 1) / resident)) return true;
+    return n_tokens * ((int64_t)2 * G * D + (int64_t)H * Dv) >= 3500000 && (f32 || wide);
+}
+static bool gdr_prepare_run_applies(int taps, int D, int Dv, int update_state) {
+    return !update_state && taps == 4 && D % 32 == 0 && D <= 32 * GP_CH && Dv % 32 == 0 && Dv <= 32 * GP_CH;
+}
+
+// Tokens a warp of imp_gdr_prepare for such a step: 1 or 8.
+IMP_API int imp_gdr_prepare_tokens(int n_tokens, int n_seqs, int G, int D, int H, int Dv, int taps, int update_state, int act_dtype) {
+    return gdr_prepare_run_applies(taps, D, Dv, update_state) && gdr_prepare_run_pays(n_tokens, n_seqs, G, D, H, Dv, act_dtype == IMP_F32) ? GP_RUN : 1;
+}
+
 // update_state: the step brings one token per sequence (n_tokens == n_seqs) and the kernel also writes the
 // convolution's new state; otherwise imp_gdr_conv_state has to follow.
-IMP_API int imp_gdr_prepare(const void* proj, int64_t ld, const float* conv_w, int taps, float* conv_state,
-                            const int* seq_of_token, const int* q_start, const int* slots, int n_tokens, int n_seqs, int G, int D,
-                            int H, int Dv, const float* a_log, const float* dt_bias, float* qn, float* kn, float* vc, float* beta,
-                            float* decay, int update_state, int act_dtype, int* status, void* stream) {
+// form: tokens a warp, 1 or 8 (IMP_ERR_UNSUPPORTED where 8 does not apply), or 0 for what imp_gdr_prepare_tokens says.
+IMP_API int imp_gdr_prepare_form(const void* proj, int64_t ld, const float* conv_w, int taps, float* conv_state,
+                                 const int* seq_of_token, const int* q_start, const int* slots, int n_tokens, int n_seqs, int G, int D,
+                                 int H, int Dv, const float* a_log, const float* dt_bias, float* qn, float* kn, float* vc, float* beta,
+                                 float* decay, int update_state, int act_dtype, int* status, int form, void* stream) {
     if (n_tokens == 0) return 0;
     IMP_CHECK_ARG(proj && conv_w && conv_state && seq_of_token && q_start && slots && a_log && dt_bias && qn && kn && vc && beta && decay,
                   "imp_gdr_prepare: null pointer");
@@ -491,7 +514,9 @@ IMP_API int imp_gdr_prepare(const void* proj, int64_t ld, const float* conv_w, i
     IMP_CHECK_ARG(!update_state || n_tokens == n_seqs, "imp_gdr_prepare: the state is updated in place only when every sequence brings one token");
     IMP_CHECK_ARG(ld >= (int64_t)2 * G * D + 2 * (int64_t)H * Dv + 2 * H, "imp_gdr_prepare: the projection's rows are too short");
     cudaStream_t s = (cudaStream_t)stream;
-    if (!update_state && taps == 4 && D % 32 == 0 && D <= 32 * GP_CH && Dv % 32 == 0 && Dv <= 32 * GP_CH) {
+    if (form == GP_RUN && !gdr_prepare_run_applies(taps, D, Dv, update_state)) return IMP_ERR_UNSUPPORTED;
+    if (form == 0) form = imp_gdr_prepare_tokens(n_tokens, n_seqs, G, D, H, Dv, taps, update_state, act_dtype);
+    if (form == GP_RUN) {
         const int64_t warps = (int64_t)((n_tokens + GP_RUN - 1) / GP_RUN) * (2 * G + H + 1), run_ctas = (warps + GP_BLOCK / 32 - 1) / (GP_BLOCK / 32);
         IMP_CHECK_ARG(run_ctas <= 0x7fffffff, "imp_gdr_prepare: too many tokens");
 #define GDR_PREPARE_RUN(TA)                                                                                                                        \
@@ -521,6 +546,14 @@ IMP_API int imp_gdr_prepare(const void* proj, int64_t ld, const float* conv_w, i
 #undef GDR_PREPARE_T
 #undef GDR_PREPARE
     IMP_RETURN_LAUNCH();
+}
+
+IMP_API int imp_gdr_prepare(const void* proj, int64_t ld, const float* conv_w, int taps, float* conv_state,
+                            const int* seq_of_token, const int* q_start, const int* slots, int n_tokens, int n_seqs, int G, int D,
+                            int H, int Dv, const float* a_log, const float* dt_bias, float* qn, float* kn, float* vc, float* beta,
+                            float* decay, int update_state, int act_dtype, int* status, void* stream) {
+    return imp_gdr_prepare_form(proj, ld, conv_w, taps, conv_state, seq_of_token, q_start, slots, n_tokens, n_seqs, G, D, H, Dv, a_log, dt_bias, qn, kn, vc, beta,
+                                decay, update_state, act_dtype, status, 0, stream);
 }
 
 IMP_API int imp_gdr_conv_state(const void* proj, int64_t ld, float* conv_state, int taps, int C, const int* q_start, const int* slots,

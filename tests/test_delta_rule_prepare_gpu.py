@@ -30,18 +30,19 @@ def test_runs_give_the_bits_of_single_tokens(lengths, G, D, H, Dv, dtype):
     stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
     sizes = (G * D, G * D, H * Dv, H, H)
 
-    def call(rows, state, seq, starts, slot, update):
+    def call(rows, state, seq, starts, slot, form):        # form: tokens a warp
+        update = int(form == 1)
         out = [torch.full((len(rows), m), float("nan"), device=DEV) for m in sizes]
         seq, starts = torch.tensor(seq, dtype=torch.int32, device=DEV), torch.tensor(starts, dtype=torch.int32, device=DEV)
-        rc = lib.imp_gdr_prepare(ptr(rows), ctypes.c_int64(ld), ptr(w), TAPS, ptr(state), ptr(seq), ptr(starts), ptr(slot), len(rows), len(starts) - 1, G, D, H, Dv,
-                                 ptr(a_log), ptr(dt), *map(ptr, out), update, 0 if dtype == torch.float32 else 1, ptr(status), stream)
+        rc = lib.imp_gdr_prepare_form(ptr(rows), ctypes.c_int64(ld), ptr(w), TAPS, ptr(state), ptr(seq), ptr(starts), ptr(slot), len(rows), len(starts) - 1, G, D, H, Dv,
+                                 ptr(a_log), ptr(dt), *map(ptr, out), update, 0 if dtype == torch.float32 else 1, ptr(status), form, stream)
         assert rc == 0
         torch.cuda.synchronize()
         return out
 
     at = [sum(lengths[:i]) for i in range(n + 1)]
     state = first_state.clone()
-    whole = call(proj, state, [i for i, m in enumerate(lengths) for _ in range(m)], at, slots, 0)
+    whole = call(proj, state, [i for i, m in enumerate(lengths) for _ in range(m)], at, slots, 8)
     assert torch.equal(state, first_state)
     for i in range(n):
         for t in range(at[i], at[i + 1]):

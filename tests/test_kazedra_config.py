@@ -126,3 +126,20 @@ def test_distance_buckets_of_the_plain_implementation():
     assert b[D - 1] <= B - 1 and all(x == B - 1 for x in b[D:])     # from the largest distance on: the last row
     assert K.query_temperature(0, 0.5, 4) == 1.0 and K.query_temperature(2, 0.5, 4) == 1.0
     assert K.query_temperature(3, 0.5, 4) == pytest.approx(1 + 0.5 * 0.6931471805599453)
+
+
+def test_tokens_a_warp_of_the_preparation():
+    """gdr_prepare_run_pays: eight where a round of 592 CTAs is three quarters full or from 3.5 million channels on, in bfloat16 for wide heads
+    and long portions only; never for what the kernel does not take."""
+    from imp_b200 import capi
+    choose = capi.load().imp_gdr_prepare_tokens
+    F32, BF16 = 0, 1
+
+    def tokens(n, seqs=1, G=8, D=128, H=16, Dv=128, taps=4, update=0, dtype=BF16):     # 4,096 channels
+        return choose(n, seqs, G, D, H, Dv, taps, update, dtype)
+
+    assert [tokens(n) for n in (1, 2, 24, 256, 424)] == [1] * 5 and [tokens(n) for n in (425, 448, 512, 568)] == [8] * 4     # 33 units: 444 CTAs from 425 on
+    assert [tokens(n) for n in (576, 640, 840)] == [1] * 3 and [tokens(n) for n in (855, 900, 1160, 2048)] == [8] * 4          # more than one round
+    assert [tokens(2048, s) for s in (32, 33)] == [8, 1] and tokens(2048, 1024, dtype=F32) == 8 and tokens(512, 16) == 1
+    assert tokens(4000, D=64, Dv=64) == 1 and tokens(4000, D=64, Dv=64, dtype=F32) == 8
+    assert [tokens(4000, **kw) for kw in ({"taps": 3}, {"D": 144}, {"Dv": 100}, {"D": 256}, {"seqs": 4000, "update": 1, "dtype": F32})] == [1] * 5

@@ -356,6 +356,23 @@ def test_cuts_and_company_change_no_bit_of_the_recurrence(dtype, case):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+def test_a_long_portion_gives_the_bits_of_short_ones(dtype):
+    """Enough channels for the kernel that prepares eight tokens a warp, and portions that go token by token."""
+    bench, part, _, _ = right_setup(dtype, dict(heads=32, kv_heads=16, dim=128, vdim=128, conv=4, d=64), eighths=True)
+    x, got = torch.randint(-1, 2, (509, 64), generator=torch.Generator().manual_seed(6)).to(dtype), []
+    for r, pieces in (("whole", [509]), ("cut", [3, 1, 200, 190, 115])):
+        at = 0
+        for n in pieces:
+            ctx, view = bench.prepare([(r, [1] * n, [])]), bench.cache_view(0)
+            run_mixer(bench, part, x[at:at + n], ctx, view)
+            bench.commit()
+            at += n
+        got.append([t[ctx.slots[0]].clone() for t in view.states])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("case", RIGHT_CASES[2:], ids=lambda c: f"{c['dim']}-{c['conv']}")
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 def test_what_is_not_finite_reaches_no_earlier_token(dtype, case, value):
