@@ -53,7 +53,8 @@ template <int N> __device__ __forceinline__ void gs_wait_group() {
 // the two matrices in blocks of 8 rows), so accumulator slots c and c+2 of a lane hold gate and up
 // of the same output column and token; the epilogue writes act(gate) * up into C[M, N/2] (gate_act: 0 silu, 1 the tanh
 // form of gelu).
-template <int NT, typename TO, bool SWIGLU, int STAGES, int RG>
+// ALL_ROWS: the rows of x past M are copied as zeros and read like the others; else they are left out, copies and reads (see gs_leave_out).
+template <int NT, typename TO, bool SWIGLU, int STAGES, int RG, bool ALL_ROWS>
 __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __restrict__ C, int64_t ldc,
                                                                     const __nv_bfloat16* __restrict__ A, int64_t lda,
                                                                     const __nv_bfloat16* __restrict__ W, int64_t ldw,
@@ -89,8 +90,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
             }
         }
     };
-    // Activation copies: 8*NT rows x 32 chunks, 2*NT per thread, of the M rows there are; columns past K are zeros.  (As zeros in
-    // shared memory the rows past M were a third of all copies at one row.)
+    // Activation copies: 8*NT rows x 32 chunks, 2*NT per thread; columns past K are zeros, with ALL_ROWS rows past M too.
     auto issue_a = [&]() {
         if (q_issue < total) {
             const uint32_t sbase = smem_base + (q_issue % STAGES) * STAGE_BYTES + W_BYTES;
@@ -99,9 +99,9 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
                 const int c = tid + i * THREADS;
                 const int row = c >> 5, col = c & 31;
                 const int k = i_stage * GS_STAGE_K + col * 8;
-                if (row >= M) break;
-                const __nv_bfloat16* src = A + (int64_t)row * lda + min(k, K - 8);
-                gs_cp_async(sbase + row * GS_ROW_BYTES + col * 16, src, k + 8 <= K ? 16 : 0);
+                if (!ALL_ROWS && row >= M) break;
+                const __nv_bfloat16* src = A + (int64_t)(ALL_ROWS ? min(row, M - 1) : row) * lda + min(k, K - 8);
+                gs_cp_async(sbase + row * GS_ROW_BYTES + col * 16, src, (k + 8 <= K && row < M) ? 16 : 0);
             }
         }
     };
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             uint4 c0 = make_uint4(0u, 0u, 0u, 0u), c1 = c0;
-            if (8 * nt + g < M) {
+            if (ALL_ROWS || 8 * nt + g < M) {
                 c0 = *reinterpret_cast<const uint4*>(sp + W_BYTES + (8 * nt + g) * GS_ROW_BYTES);
                 c1 = *reinterpret_cast<const uint4*>(sp + W_BYTES + (8 * nt + g) * GS_ROW_BYTES + 16);
             }
@@ -215,12 +215,12 @@ __global__ void __launch_bounds__(GS_WARPS * 32 * RG) gemm_stream_kernel(TO* __r
     IMP_TL_END()
 }
 
-template <int NT, typename TO, bool SWIGLU, int STAGES, int RG>
+template <int NT, typename TO, bool SWIGLU, int STAGES, int RG, bool ALL_ROWS = true>
 static cudaError_t launch_stream_st(TO* C, int64_t ldc, const __nv_bfloat16* A, int64_t lda, const __nv_bfloat16* W,
                                     int64_t ldw, int M, int N, int K, cudaStream_t s, GateAct gate_act = GateAct()) {
     static bool attr_set = false;   // once per instantiation (one device per process)
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_stream_kernel<NT, TO, SWIGLU, STAGES, RG>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_stream_kernel<NT, TO, SWIGLU, STAGES, RG, ALL_ROWS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, gs_smem_bytes(NT, STAGES, RG));
         if (e != cudaSuccess) return e;
         attr_set = true;
@@ -229,7 +229,7 @@ static cudaError_t launch_stream_st(TO* C, int64_t ldc, const __nv_bfloat16* A, 
     // One tile per CTA measured faster than two persistent CTAs per SM on every shape of the 8B model
     // (the kernel itself takes any grid size: a CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...).
     const int grid = n_tiles;
-    return imp_launch_product(gemm_stream_kernel<NT, TO, SWIGLU, STAGES, RG>, dim3(grid), dim3(GS_WARPS * 32 * RG), gs_smem_bytes(NT, STAGES, RG), s, C, ldc,
+    return imp_launch_product(gemm_stream_kernel<NT, TO, SWIGLU, STAGES, RG, ALL_ROWS>, dim3(grid), dim3(GS_WARPS * 32 * RG), gs_smem_bytes(NT, STAGES, RG), s, C, ldc,
                       A, lda, W, ldw, M, N, K, gate_act);
 }
 
@@ -246,6 +246,19 @@ static int gs_env_stages() {
     return v;
 }
 
+// Whether the rows of x past M are left out.  Their copies of zeros are a third of a stage's at one row.
+// One row: always.  Its copies stand between the kernel before and the first sum, so a chain of launches gains more than a launch alone: decoding with one
+// sequence, 8B shape 133.9 -> 132.5 ms (2,048 + 32 tokens), 0.6B shape 14.77 -> 14.71 ms, although single launches of short K lose (6,144 x 1,024 4.78 ->
+// 4.92 us, 1,024 x 2,048 4.29 -> 4.37; 4,096 x 12,288 22.4 -> 20.8).
+// More rows, launches alone: 4 of 4,096 x 12,288 24.1 -> 22.9 us and of 4,096 x 4,096 10.1 -> 9.6 in the form with two row groups and six stages, 2 of
+// 4,096 x 12,288 22.9 -> 22.3.  Asking for every row costs more than that at seven and eight rows (8 of 4,096 x 12,288: 23.7 -> 24.0), at three and more in
+// the eight-stage form (4 of 2,048 x 4,096: 7.07 -> 7.27), at two of a short N (1,024 x 4,096: 6.47 -> 6.51), and always with more than eight rows
+// (16 of 4,096 x 12,288: 32.7 -> 34.9).
+static bool gs_leave_out(int M, int N, int K, int row_groups) {
+    if (M == 1) return true;
+    return K >= 4096 && (row_groups == 2 ? M <= 6 : M == 2 && N >= 2048);
+}
+
 template <int NT, typename TO, bool SWIGLU>
 static cudaError_t launch_stream_nt(TO* C, int64_t ldc, const __nv_bfloat16* A, int64_t lda, const __nv_bfloat16* W,
                                     int64_t ldw, int M, int N, int K, cudaStream_t s, GateAct gate_act = GateAct()) {
@@ -260,14 +273,20 @@ static cudaError_t launch_stream_nt(TO* C, int64_t ldc, const __nv_bfloat16* A, 
     const int sms = imp_sm_count();
     if (NT == 1 && M >= 3 && rg_env >= 2 && stages == 0 && (N + 31) / 32 >= sms)
         return launch_stream_st<1, TO, SWIGLU, 4, 2>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
-    if (NT == 1 && M >= 3 && rg_env == 3 && stages == 0 && (N + 31) / 32 >= (sms * 96 + 147) / 148 && (N + 31) / 32 < sms)
+    if (NT == 1 && M >= 3 && rg_env == 3 && stages == 0 && (N + 31) / 32 >= (sms * 96 + 147) / 148 && (N + 31) / 32 < sms) {
+        if (gs_leave_out(M, N, K, 2)) return launch_stream_st<1, TO, SWIGLU, 6, 2, false>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
         return launch_stream_st<1, TO, SWIGLU, 6, 2>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
+    }
     if (stages == 0) stages = (NT == 1 && (N + 15) / 16 <= 2 * sms) ? 8 : 5;
     switch (stages) {
         case 4: return launch_stream_st<NT, TO, SWIGLU, 4, 1>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
         case 6: return launch_stream_st<NT, TO, SWIGLU, 6, 1>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
-        case 8: return launch_stream_st<NT, TO, SWIGLU, 8, 1>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
-        default: return launch_stream_st<NT, TO, SWIGLU, 5, 1>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
+        case 8:
+            if (NT == 1 && gs_leave_out(M, N, K, 1)) return launch_stream_st<NT, TO, SWIGLU, 8, 1, NT != 1>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
+            return launch_stream_st<NT, TO, SWIGLU, 8, 1>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
+        default:
+            if (NT == 1 && M == 1) return launch_stream_st<NT, TO, SWIGLU, 5, 1, NT != 1>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
+            return launch_stream_st<NT, TO, SWIGLU, 5, 1>(C, ldc, A, lda, W, ldw, M, N, K, s, gate_act);
     }
 }
 

@@ -288,6 +288,18 @@ def test_gemm_bf16_stream(K, M, N, K_, odtype):
     assert torch.equal(out2, out)
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 6, 7])
+@pytest.mark.parametrize("N,K_", [(4096, 4096), (4100, 4104), (2048, 4096), (2047, 4096), (4096, 4088)])   # both sides of each line of the rule
+def test_gemm_bf16_stream_without_the_rows_that_are_not_there(K, M, N, K_):
+    """The bits of a row do not depend on how many rows come with it; with eight all of them are copied and read."""
+    a, w = rnd(8, K_, dtype=torch.bfloat16, seed=12).to(DEV), rnd(N, K_, dtype=torch.bfloat16, seed=13).to(DEV)
+    every = K.gemm_bf16_stream(torch.empty(8, N, dtype=torch.float32, device=DEV), a, w)
+    some = K.gemm_bf16_stream(torch.full((M, N), float("nan"), device=DEV), a[:M], w)
+    assert torch.equal(some, every[:M])
+    want = a.double().cpu() @ w.double().cpu().T
+    close(every, want, torch.float32, scale=float(want.abs().max()) * 4)
+
+
 @pytest.mark.parametrize("M", [1, 3, 8, 11, 16, 40])
 @pytest.mark.parametrize("F,K_", [(8, 64), (200, 96), (3072, 1024), (24, 100)])
 def test_linear_swiglu_fused(K, M, F, K_):
