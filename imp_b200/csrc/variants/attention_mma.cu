@@ -795,7 +795,8 @@ __device__ __forceinline__ bool dt_wait(uint32_t bar, uint32_t parity, int* stat
 // the same banks: odd keys read each pair of 64-byte blocks in the other order, and a pass meets all banks once.  Of the values', they asked for two
 // 16-byte pieces of four rows each: in every second block of 64 dimensions lane g takes the piece g ^ 4 (dim_of_smem), and odd lanes t read that block
 // first: four pieces.  256 -> 160 passes for 16 keys of 128 with the way in.  Which key or dimension meets which register stays, or changes
-// whole columns, so every sum is the same.
+// whole columns, so every sum is the same.  64 sequences of 1,024 keys, 32 query heads on 8: heads of 128 48.9 -> 48.2 us, of 192 (keys alone) 86.0 -> 83.4, of
+// 256 107.8 -> 102.7.  Heads of 64 read their keys as they lie: one pair of blocks, two passes saved, and the exchange cost more (26.1 -> 26.4).
 template <bool SWAP> __device__ __forceinline__ void swap_if(uint4& a, uint4& b, bool odd) {
     if (SWAP) {
         const uint4 x = odd ? b : a, y = odd ? a : b;
@@ -803,7 +804,7 @@ template <bool SWAP> __device__ __forceinline__ void swap_if(uint4& a, uint4& b,
     }
 }
 __device__ __forceinline__ void load_key_frags(uint32_t (&f)[KSTEPS][2], const unsigned char* row, int t, bool odd) {
-    if constexpr (DH % 64 != 0) {
+    if constexpr (DH % 64 != 0 || DH == 64) {
         load_row_frags(f, reinterpret_cast<const __nv_bfloat16*>(row), t);
     } else {
 #pragma unroll
