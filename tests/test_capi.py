@@ -133,6 +133,26 @@ def ints(values):
     return (c_int32 * max(len(values), 1))(*values)
 
 
+def test_a_step_s_entries_as_the_library_reads_them():
+    """Engine._marshal packs the entries by offset: read back through the structure, they are what went in."""
+    import numpy as np
+    from imp_b200 import Engine, StepEntry
+    engine = Engine.__new__(Engine)
+    engine._ids, engine._next_replay_id = {}, -(1 << 40)
+    given = [("a", [5], [0]), (("b", 1), list(range(40)), [39, 0]), ("c", np.arange(3, dtype=np.int64), []), ("a2", (7, 2 ** 31 - 1), (1,)), ("d", [], [])]
+    arr, keep, wanted = engine._marshal([StepEntry(*g) for g in given])
+    assert wanted == 4 and len(arr) == len(given)
+    for i, (rid, tokens, want) in enumerate(given):
+        e = arr[i]
+        assert e.id == engine._ids[rid] == -(1 << 40) + i
+        assert [e.tokens[j] for j in range(e.n_tokens)] == [int(t) for t in tokens] and [e.want[j] for j in range(e.n_want)] == list(want)
+    arr, keep, wanted = engine._marshal([])
+    assert len(arr) == 1 and wanted == 0 and not arr[0].n_tokens
+    with pytest.raises((TypeError, ValueError)):
+        engine._marshal([StepEntry("e", ["x"], [])])
+    assert "e" not in engine._ids
+
+
 @pytest.mark.gpu
 def test_generate_prefill_decode_and_replay_through_raw_calls(lib, context):
     from plain.qwen3_plain import PlainModel
